@@ -117,6 +117,9 @@ def fused_cross_entropy_loss_and_logsumexp_penalty(pred_embeddings, pred_lm_head
     x = pred_embeddings.reshape(-1, pred_embeddings.shape[-1])
     t = target_ids.reshape(-1)
     if CE.kernel_ok(x, pred_lm_head):
+        V = pred_lm_head.shape[0]
+        if V % 8 != 0:  # out of range: no target logit, as in the blockwise form below, and nothing for the kernel to report
+            t = torch.where(t >= V, -1, t)
         loss, _ = CE.fused_linear_cross_entropy(x, pred_lm_head, t, soft_cap=logit_soft_cap, z_weight=logsumexp_weight)
         return loss.view(lead)
     block = block_size or pred_lm_head.shape[0]
@@ -146,6 +149,8 @@ def maybe_fused_next_token_loss(pred_embeddings: torch.Tensor, pred_lm_head: tor
         logits = (pred_embeddings.to(dtype) @ pred_lm_head.to(dtype).t()) if dtype is not None else pred_embeddings @ pred_lm_head.t()
         loss, _ = cross_entropy_and_logsumexp_penalty(logits, target, logsumexp_weight=logsumexp_weight, logit_soft_cap=logit_soft_cap)
     else:
+        if block_size is None and pred_lm_head.shape[0] % 8 != 0:
+            target = target.clamp(0, pred_lm_head.shape[0] - 1)  # as in the materialised form above
         loss = fused_cross_entropy_loss_and_logsumexp_penalty(pred_embeddings, pred_lm_head, target, block_size=block_size,
                                                               logsumexp_weight=logsumexp_weight, dtype=dtype,
                                                               logit_soft_cap=logit_soft_cap)

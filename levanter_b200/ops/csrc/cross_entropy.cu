@@ -127,8 +127,51 @@ __global__ void __launch_bounds__(kBlock) ce_grad_kernel(const float* __restrict
   }
 }
 
+// (max, sum) of a row's column tiles -> log-sum-exp and loss.  32 rows x 8 shares of the tiles per block, lanes along the rows.
+__global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restrict__ part, int tiles, const int* __restrict__ targets,
+                                                         const float* __restrict__ target_logit, float* __restrict__ lse_out,
+                                                         float* __restrict__ loss_out, int rows, int vocab, float z_weight, int* status) {
+  __shared__ float2 share[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
+  float m = -INFINITY, s = 0.f;
+  if (row < rows) {
+    for (int t = w; t < tiles; t += 8) {
+      const float2 v = part[static_cast<size_t>(t) * rows + row];
+      const float nm = fmaxf(m, v.x);
+      s = (m == -INFINITY ? s : s * __expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * __expf(v.x - nm));
+      m = nm;
+    }
+  }
+  share[w][lane] = make_float2(m, s);
+  __syncthreads();
+  if (w > 0 || row >= rows) return;
+  for (int i = 1; i < 8; ++i) {
+    const float2 v = share[i][lane];
+    const float nm = fmaxf(m, v.x);
+    s = (m == -INFINITY ? s : s * __expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * __expf(v.x - nm));
+    m = nm;
+  }
+  const float lse = m + logf(s);
+  const int t = targets[row];
+  if (t >= vocab) record_status(status, kBoundsCheck, 500, t);
+  // targets outside the vocabulary (padding, ignored ids) contribute no target logit; their loss weight is expected to be zero
+  lse_out[row] = lse;
+  loss_out[row] = lse - (t >= 0 && t < vocab ? target_logit[row] : 0.f) + z_weight * lse * lse;
+}
+
 }  // namespace ce
 }  // namespace lvb
+
+// part: float2[tiles, rows] and target_logit of lvb_head_ce_stats -> lse, loss = lse - target logit + z_weight * lse^2 (float[rows]).
+extern "C" int lvb_ce_combine(const void* part, int tiles, const int* targets, const float* target_logit, float* lse, float* loss, int rows,
+                              int vocab, float z_weight, int* status, void* stream) {
+  using namespace lvb;
+  if (rows <= 0 || tiles <= 0) return kErrBadArg;
+  ce::ce_combine_kernel<<<(rows + 31) / 32, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const float2*>(part), tiles, targets, target_logit, lse, loss, rows, vocab, z_weight, status);
+  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+}
 
 // logits: fp32 [rows, vocab] with row stride ld (multiple of 4); targets: int32 [rows].
 extern "C" int lvb_ce_stats(const float* logits, long long ld, const int* targets, float* lse, float* tgt, int rows,

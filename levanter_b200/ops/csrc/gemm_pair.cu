@@ -76,11 +76,27 @@ struct Params {
   int cj_u0, cj_u1;
   const uint8_t* cj_src[kMaxPeers];
   uint8_t* cj_dst;
+  // ---- operands that wrap (kPlain): K block kb >= k_wrap > 0 reads B's block kb - k_wrap again and A's with its x coordinate
+  // moved by a_wrap_x.  A matrix held as two bf16 parts (high and low, side by side) is then multiplied in one accumulation.
+  int k_wrap = 0;
+  int a_wrap_x = 0;
+  // ---- cross-entropy epilogues (kCeStats, kCeGrad): C is never stored, it is the logits
+  const int* ce_targets = nullptr;
+  float2* ce_part = nullptr;        // kCeStats: (max, sum of exponentials) of every (column tile, row)
+  float* ce_target_logit = nullptr; // kCeStats: the row's logit at its target
+  const float* ce_lse = nullptr;    // kCeGrad
+  const float* ce_g_loss = nullptr;
+  const float* ce_g_logz = nullptr; // may be null
+  float ce_cap = 0.f;               // tanh soft cap of the logits, 0: none
+  int ce_cols = 0;                  // kCeGrad: columns of C to write; those from N on get zeros
+  long long ce_low = 0;             // kCeGrad: offset of the low parts (0: C holds one bf16 number per logit)
 };
 
 constexpr int kPlain = 0;
 constexpr int kScatter = 1;
 constexpr int kCopyJob = 2;
+constexpr int kCeStats = 3;
+constexpr int kCeGrad = 4;
 constexpr int kCopyUnit = 16384;                  // bytes per bulk copy of a copy job
 constexpr int kCopyExtra = 256 + 2 * kCopyUnit;  // extra dynamic shared memory of the copy-job kernel
 constexpr int kCopyThreads = kNumThreads + 32;
@@ -174,6 +190,94 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
   nb = r / gm;
 }
 
+// Cross-entropy on the accumulators of a tile: a lane owns a row and sees it 32 columns at a time, so that the logits are consumed
+// where they are made.  A separate pass over fp32 logits costs 8 bytes of traffic per logit in the forward pass (write, read) and 12
+// in the backward one; here it is 8 bytes per row and 256 columns, and the 2 (one bf16 part) or 4 bytes (two) of the gradient.  8192 rows x
+// 50257 x 768: 600 us forward (1.05 PFLOP/s), 975 us for both parts of the gradient, where the exponentials of the four epilogue warps and
+// the stores weigh as much as the products; at 32000 x 4096 the products bound it, and the separate passes over logits (415 us) are gone.
+struct CeRow {
+  float m = -INFINITY, s = 0.f;  // running maximum and scaled sum of exponentials
+  float lse = 0.f, gl = 0.f, gp = 0.f;
+  int target = -1;
+
+  template <int MODE>
+  __device__ __forceinline__ void begin(const Params& p, int row) {
+    target = __ldg(p.ce_targets + row);
+    if constexpr (MODE == kCeGrad) {
+      lse = __ldg(p.ce_lse + row);
+      gl = __ldg(p.ce_g_loss + row);
+      gp = gl + (p.ce_g_logz != nullptr ? __ldg(p.ce_g_logz + row) : 0.f);
+    }
+  }
+  __device__ __forceinline__ void stats(const Params& p, int row, int col0, const uint32_t (&r)[32]) {
+    const int live = p.N - col0;  // columns of this piece that exist (<= 0: none)
+    if (live <= 0) return;
+    float v[32];
+    float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      v[j] = __uint_as_float(r[j]);
+      if (p.ce_cap > 0.f) v[j] = p.ce_cap * tanhf(v[j] / p.ce_cap);
+      if (j >= live) v[j] = -INFINITY;
+      top[j & 3] = fmaxf(top[j & 3], v[j]);
+    }
+    const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
+    if (mx > m) {
+      s = m == -INFINITY ? 0.f : s * __expf(m - mx);
+      m = mx;
+    }
+    if (m != -INFINITY) {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum[j & 3] += __expf(v[j] - m);
+      s += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    } else {  // nothing but -inf so far, or NaN, which has to show
+#pragma unroll
+      for (int j = 0; j < 32; ++j) s += v[j] != v[j] ? v[j] : 0.f;
+    }
+    const int at = target - col0;
+    if (at >= 0 && at < 32 && at < live) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j == at) p.ce_target_logit[row] = v[j];
+    }
+  }
+  // d(cap)/d(raw) * ((g_loss + g_logz) * probability - g_loss * [column == target])
+  __device__ __forceinline__ void grad(const Params& p, int row, int col0, const uint32_t (&r)[32]) {
+    if (col0 >= p.ce_cols) return;
+    const int at = target - col0;
+    uint32_t hi[16], lo[16];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      float g[2];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float a = __uint_as_float(r[j + e]), slope = 1.f;
+        if (p.ce_cap > 0.f) {
+          const float th = tanhf(a / p.ce_cap);
+          a = p.ce_cap * th;
+          slope = 1.f - th * th;
+        }
+        float x = gp * __expf(a - lse);
+        if (j + e == at) x -= gl;
+        g[e] = col0 + j + e < p.N ? x * slope : 0.f;
+      }
+      const __nv_bfloat162 h = __floats2bfloat162_rn(g[0], g[1]);
+      hi[j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+      const float2 back = __bfloat1622float2(h);
+      lo[j >> 1] = pack_bf16x2(g[0] - back.x, g[1] - back.y);
+    }
+    // rows are multiples of 64 columns long and 16-byte aligned; a piece lies inside or outside them as a whole
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(out)[q] = make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
+    if (p.ce_low > 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(out + p.ce_low)[q] = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
+    }
+  }
+};
+
 template <int BN, bool A_MN, bool B_MN, int MODE>
 __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& p) {
   using L = Smem<BN>;
@@ -252,12 +356,18 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
           uint8_t* sa = smem + stage * L::kStageBytes;
           uint8_t* sb = sa + L::kABytes;
           if (cta == 0) mbar_expect_tx(&full_bar[stage], 2 * L::kStageBytes);  // both CTAs' loads of this stage
-          const int k0 = kb * BK;
+          int k0 = kb * BK, ax = 0;
+          if constexpr (MODE == kPlain) {
+            if (p.k_wrap > 0 && kb >= p.k_wrap) {
+              k0 -= p.k_wrap * BK;
+              ax = p.a_wrap_x;
+            }
+          }
           if constexpr (!A_MN) {
-            tma_load_2d_pair(sa, &tmA, &full_bar[stage], k0, m0);
+            tma_load_2d_pair(sa, &tmA, &full_bar[stage], k0 + ax, m0);
           } else {
 #pragma unroll
-            for (int c = 0; c < BMC / 64; ++c) tma_load_2d_pair(sa + c * (64 * BK * 2), &tmA, &full_bar[stage], m0 + 64 * c, k0);
+            for (int c = 0; c < BMC / 64; ++c) tma_load_2d_pair(sa + c * (64 * BK * 2), &tmA, &full_bar[stage], m0 + ax + 64 * c, k0);
           }
           if constexpr (!B_MN) {
             tma_load_2d_pair(sb, &tmB, &full_bar[stage], k0, n0);
@@ -335,12 +445,23 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
         c_dest = c_live ? row0w / p.c_rows_per_rank : 0;
         c_dst_row0 = reinterpret_cast<float*>(p.c_peer[c_dest]) + static_cast<size_t>(row0w - c_dest * p.c_rows_per_rank) * p.ldc;
       }
+      CeRow ce;
+      if constexpr (MODE == kCeStats || MODE == kCeGrad) {
+        if (row < p.M) ce.begin<MODE>(p, row);
+      }
 #pragma unroll 1
       for (int c = 0; c < BN; c += 32) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c, r);
         tmem_ld_wait();
         const int col0 = n0 + c;
+        if constexpr (MODE == kCeStats || MODE == kCeGrad) {
+          if (row < p.M) {
+            if constexpr (MODE == kCeStats) ce.stats(p, row, col0, r);
+            else ce.grad(p, row, col0, r);
+          }
+          continue;
+        }
         if constexpr (MODE == kScatter) {
           // Peer stores: turn the row-per-lane fragment into row-contiguous 128-byte segments through shared memory, so a
           // store instruction covers 4 rows x 128 B instead of 32 rows x 16 B (NVLink moves short writes poorly).
@@ -472,6 +593,9 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
             }
           }
         }
+      }
+      if constexpr (MODE == kCeStats) {
+        if (row < p.M) p.ce_part[static_cast<size_t>(nb) * p.M + row] = make_float2(ce.m, ce.s);
       }
       // all TMEM reads of this warp are complete (tmem_ld_wait above)
       tc_fence_before();
@@ -616,6 +740,12 @@ gemm_pair_copy_job_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   gemm_pair_body<BN, A_MN, B_MN, kCopyJob>(tmA, tmB, p);
 }
 
+template <int MODE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kNumThreads, 1)
+gemm_pair_ce_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Params p) {
+  gemm_pair_body<256, false, false, MODE>(tmA, tmB, p);
+}
+
 template <typename Kern>
 int max_resident_pairs(Kern kern, int threads, int smem) {
   // as many pairs as can be resident at once (a GPC with an odd number of free SMs cannot host a pair on the last one)
@@ -692,12 +822,39 @@ int launch_copy_job(const void* A, const void* B, Params p, int lda, int ldb, cu
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }
 
+template <int MODE>
+int launch_ce(const void* A, const void* B, Params p, int lda, int ldb, cudaStream_t stream) {
+  using L = Smem<256>;
+  CUtensorMap tmA, tmB;
+  int rc = make_maps<256, false, false>(&tmA, &tmB, A, B, p, lda, ldb);
+  if (rc != kErrOk) return rc;
+  p.tiles_m = (p.M + BMP - 1) / BMP;
+  p.tiles_n = (p.N + 255) / 256;
+  auto kern = gemm_pair_ce_kernel<MODE>;
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal) != cudaSuccess) return kErrCuda;
+    max_pairs = max_resident_pairs(kern, kNumThreads, L::kTotal);
+  }
+  const int tiles = p.tiles_m * p.tiles_n;
+  kern<<<2 * (tiles < max_pairs ? tiles : max_pairs), kNumThreads, L::kTotal, stream>>>(tmA, tmB, p);
+  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+}
+
 template <int BN, bool A_MN, bool B_MN>
-int launch(const void* A, const void* B, Params p, int lda, int ldb, cudaStream_t stream, int max_ctas) {
-  using L = Smem<BN>;
+int launch_maps(const CUtensorMap& tmA, const CUtensorMap& tmB, Params p, cudaStream_t stream, int max_ctas);
+
+template <int BN, bool A_MN, bool B_MN>
+int launch(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream, int max_ctas) {
   CUtensorMap tmA, tmB;
   int rc = make_maps<BN, A_MN, B_MN>(&tmA, &tmB, A, B, p, lda, ldb);
   if (rc != kErrOk) return rc;
+  return launch_maps<BN, A_MN, B_MN>(tmA, tmB, p, stream, max_ctas);
+}
+
+template <int BN, bool A_MN, bool B_MN>
+int launch_maps(const CUtensorMap& tmA, const CUtensorMap& tmB, Params p, cudaStream_t stream, int max_ctas) {
+  using L = Smem<BN>;
   p.tiles_m = (p.M + BMP - 1) / BMP;
   p.tiles_n = (p.N + BN - 1) / BN;
   auto kern = gemm_pair_kernel<BN, A_MN, B_MN>;
@@ -755,6 +912,86 @@ extern "C" int lvb_gemm_bf16_pair(const void* A, const void* B, void* C, int M, 
   if (!a_mn && b_mn) return launch<256, false, true>(A, B, p, lda, ldb, s, max_ctas);
   if (a_mn && b_mn) return launch<256, true, true>(A, B, p, lda, ldb, s, max_ctas);
   return launch<256, true, false>(A, B, p, lda, ldb, s, max_ctas);
+}
+
+// Logits x[T, E] * w[V, E]^T consumed where they are made (V > 128, E and the row strides multiples of 8).
+// part: float2[ceil(V / 256), T] = (max, sum of exponentials) of every column tile's part of a row; target_logit: float[T], written for
+// targets in [0, V) only.
+extern "C" int lvb_head_ce_stats(const void* x, const void* w, const int* targets, void* part, float* target_logit, int T, int V, int E,
+                                 int ldx, int ldw, float soft_cap, int* status, void* stream) {
+  using namespace lvb;
+  using namespace lvb::gemm2;
+  if (T <= 0 || V <= 128 || E <= 0 || (ldx & 7) || (ldw & 7)) return kErrBadArg;
+  Params p{};
+  p.splits = 1;
+  p.M = T; p.N = V; p.K = E;
+  p.alpha = 1.f;
+  p.status = status;
+  p.ce_targets = targets;
+  p.ce_part = reinterpret_cast<float2*>(part);
+  p.ce_target_logit = target_logit;
+  p.ce_cap = soft_cap;
+  return launch_ce<kCeStats>(x, w, p, ldx, ldw, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// The gradient of the logits, bf16 [T, ldd] with columns [V, cols) zero (cols a multiple of 64, at least V); with low > 0 what the
+// rounding lost is stored as a second bf16 number `low` columns further on.
+extern "C" int lvb_head_ce_grad(const void* x, const void* w, const int* targets, const float* lse, const float* g_loss, const float* g_logz,
+                                void* dlogits, long long ldd, int cols, long long low, int T, int V, int E, int ldx, int ldw, float soft_cap,
+                                int* status, void* stream) {
+  using namespace lvb;
+  using namespace lvb::gemm2;
+  if (T <= 0 || V <= 128 || E <= 0 || (ldx & 7) || (ldw & 7) || (ldd & 7) || (low & 7) || (cols & 63) || cols < V || ldd > 0x7fffffff ||
+      ldd < low + cols || (low > 0 && low < cols))
+    return kErrBadArg;
+  Params p{};
+  p.splits = 1;
+  p.M = T; p.N = V; p.K = E;
+  p.alpha = 1.f;
+  p.status = status;
+  p.C = dlogits;
+  p.ldc = static_cast<int>(ldd);
+  p.ce_targets = targets;
+  p.ce_lse = lse;
+  p.ce_g_loss = g_loss;
+  p.ce_g_logz = g_logz;
+  p.ce_cap = soft_cap;
+  p.ce_cols = cols;
+  p.ce_low = low;
+  return launch_ce<kCeGrad>(x, w, p, ldx, ldw, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// Products with the gradient d [T, ldd] that lvb_head_ce_grad made (low > 0: high and low parts, both multiplied in one accumulation):
+//   a_mn = 0: C[T, E] = d * w[V, E]      (K = V, split over CTA pairs where T x E has few tiles; workspace as lvb_gemm_bf16_pair_splitk)
+//   a_mn = 1: C[V, E] = d^T * x[T, E]    (K = T)
+extern "C" int lvb_head_ce_product(const void* d, const void* b, void* C, int T, int V, int E, long long ldd, int cols, long long low, int ldb,
+                                   int ldc, int a_mn, int flags, int splits, void* workspace, int* status, void* stream) {
+  using namespace lvb;
+  using namespace lvb::gemm2;
+  if (T <= 0 || V <= 0 || E <= 0 || (ldb & 7) || (ldd & 7) || ldd > 0x7fffffff || splits < 1 || splits > 8) return kErrBadArg;
+  Params p{};
+  p.C = C;
+  p.ldc = ldc;
+  p.flags = flags;
+  p.alpha = 1.f;
+  p.status = status;
+  p.M = a_mn ? V : T;
+  p.N = E;
+  const int depth = a_mn ? T : cols;  // of one part
+  const int blocks = (depth + BK - 1) / BK;
+  p.K = low > 0 ? 2 * blocks * BK : depth;
+  p.k_wrap = low > 0 ? blocks : 0;
+  p.a_wrap_x = static_cast<int>(low);
+  p.splits = a_mn ? 1 : splits;
+  p.ws = reinterpret_cast<float*>(workspace);
+  const int wide = low > 0 ? static_cast<int>(low) + cols : cols;  // columns of d
+  CUtensorMap tmA, tmB;
+  int rc = a_mn ? make_tmap_2d_bf16(&tmA, d, T, wide, static_cast<int>(ldd), BK, 64) : make_tmap_2d_bf16(&tmA, d, T, wide, static_cast<int>(ldd), BMC, BK);
+  if (rc != kErrOk) return rc;
+  rc = make_tmap_2d_bf16(&tmB, b, a_mn ? T : V, E, ldb, BK, 64);
+  if (rc != kErrOk) return rc;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return a_mn ? launch_maps<256, true, true>(tmA, tmB, p, s, 0) : launch_maps<256, false, true>(tmA, tmB, p, s, 0);
 }
 
 // lvb_gemm_bf16_pair for K-major operands with K split over `splits` CTA pairs per tile (0: chosen by the launcher so that about
