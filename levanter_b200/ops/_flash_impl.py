@@ -16,7 +16,7 @@ _FORCE_ONE_TILE = False  # tests flip this to exercise the one-tile forward kern
 def _fwd():
     if "f" not in _f:
         c = lib
-        _f["f"] = lib.fn("lvb_flash_attn_fwd", [c.c_void_p] * 8 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p])
+        _f["f"] = lib.fn("lvb_flash_attn_fwd", [c.c_void_p] * 7 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p])
     return _f["f"]
 
 
@@ -30,7 +30,7 @@ def _fwd2():
 def _bwd():
     if "b" not in _f:
         c = lib
-        _f["b"] = lib.fn("lvb_flash_attn_bwd", [c.c_void_p] * 12 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
+        _f["b"] = lib.fn("lvb_flash_attn_bwd", [c.c_void_p] * 13 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
                          launches=2)
     return _f["b"]
 
@@ -39,7 +39,7 @@ def _fwd_hd():
     """Head size 64 or 128, causal or not (one query tile per CTA)."""
     if "fh" not in _f:
         c = lib
-        _f["fh"] = lib.fn("lvb_flash_attn_fwd_hd", [c.c_void_p] * 9 + [c.c_int] * 7 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p])
+        _f["fh"] = lib.fn("lvb_flash_attn_fwd_hd", [c.c_void_p] * 8 + [c.c_int] * 7 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p])
     return _f["fh"]
 
 
@@ -54,7 +54,7 @@ def _fwd2_hd():
 def _bwd_hd():
     if "bh" not in _f:
         c = lib
-        _f["bh"] = lib.fn("lvb_flash_attn_bwd_hd", [c.c_void_p] * 12 + [c.c_int] * 7 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
+        _f["bh"] = lib.fn("lvb_flash_attn_bwd_hd", [c.c_void_p] * 13 + [c.c_int] * 7 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
                           launches=2)
     return _f["bh"]
 
@@ -62,9 +62,22 @@ def _bwd_hd():
 def _bwd2():
     if "b2" not in _f:
         c = lib
-        _f["b2"] = lib.fn("lvb_flash_attn_bwd2", [c.c_void_p] * 12 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
+        _f["b2"] = lib.fn("lvb_flash_attn_bwd2", [c.c_void_p] * 13 + [c.c_int] * 4 + [c.c_float, c.c_float, c.c_int, c.c_void_p, c.c_void_p],
                           launches=2)
     return _f["b2"]
+
+
+def _segment_ranges(q_seg, k_seg):
+    """(lowest, highest) segment id per 128 rows of ``q_seg [B, S]`` and then of ``k_seg [B, Sk]``, by which the kernels leave blocks out."""
+    if q_seg is None:
+        return None
+    if "r" not in _f:
+        c = lib
+        _f["r"] = lib.fn("lvb_segment_ranges", [c.c_void_p] * 2 + [c.c_int] * 3 + [c.c_void_p] * 2)
+    (B, S), Sk = q_seg.shape, k_seg.shape[1]
+    out = torch.empty(B * (S + Sk) // 128, 2, dtype=torch.int32, device=q_seg.device)
+    lib.check_rc(_f["r"](q_seg.data_ptr(), k_seg.data_ptr(), B, S, Sk, out.data_ptr(), lib.stream_ptr()), "lvb_segment_ranges")
+    return out
 
 
 # The backward pass runs on the software-pipelined kernel (``csrc/flash_attn_bwd2.cu``); ``LEVANTER_B200_FLASH_BWD=serial`` selects
@@ -103,7 +116,7 @@ def replaying_outputs(store: list):
 
 class _FlashFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, q, k, v, q_seg, k_seg, scale, soft_cap, window, kblock_lo=None, causal=True, sink=None):
+    def forward(ctx, q, k, v, q_seg, k_seg, scale, soft_cap, window, causal=True, sink=None):
         B, S, Hq, D = q.shape
         Sk = k.shape[1]  # differs from S only for cross attention (no causal part)
         general = D != 128 or not causal  # the kernels templated on the head size; the pipelined backward is causal, 128 only
@@ -111,6 +124,7 @@ class _FlashFn(torch.autograd.Function):
             sink = sink.detach().float().contiguous()
         Hkv = k.shape[2]
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+        ranges = _segment_ranges(q_seg, k_seg)
         if _replay:
             o, lse2 = _replay.pop(0)
             if o.shape != q.shape:
@@ -119,25 +133,26 @@ class _FlashFn(torch.autograd.Function):
             o = torch.empty_like(q)
             lse2 = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
             # two query tiles per CTA when the sequence allows it; the one-tile kernel covers the remaining lengths
+            two = S % 256 == 0 and not _FORCE_ONE_TILE
+            skip = (lib.ptr(ranges),) if two else ()
             if general or sink is not None:
-                rc = (_fwd2_hd() if (S % 256 == 0 and not _FORCE_ONE_TILE) else _fwd_hd())(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg),
-                               lib.ptr(kblock_lo) if causal else 0, lib.ptr(sink), B, S, Sk, Hq, Hkv, D, int(bool(causal)), float(scale),
-                               float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
+                rc = (_fwd2_hd() if two else _fwd_hd())(
+                    q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), *skip, lib.ptr(sink), B, S, Sk,
+                    Hq, Hkv, D, int(bool(causal)), float(scale), float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
             else:
-                fwd = _fwd2() if (S % 256 == 0 and not _FORCE_ONE_TILE) else _fwd()
-                rc = fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg),
-                         lib.ptr(kblock_lo), B, S, Hq, Hkv, float(scale), float(soft_cap or 0.0), int(window or 0),
-                         lib.status_buffer().data_ptr(), lib.stream_ptr())
+                rc = (_fwd2() if two else _fwd())(
+                    q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), *skip, B, S, Hq, Hkv,
+                    float(scale), float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
             lib.check_rc(rc, "lvb_flash_attn_fwd")
             if _keep is not None:
                 _keep.append((o, lse2))
-        ctx.save_for_backward(q, k, v, o, lse2, q_seg, k_seg, sink)
+        ctx.save_for_backward(q, k, v, o, lse2, q_seg, k_seg, sink, ranges)
         ctx.args = (scale, soft_cap, window, causal, general)
         return o
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, o, lse2, q_seg, k_seg, sink = ctx.saved_tensors
+        q, k, v, o, lse2, q_seg, k_seg, sink, ranges = ctx.saved_tensors
         scale, soft_cap, window, causal, general = ctx.args
         B, S, Hq, D = q.shape
         Hkv = k.shape[2]
@@ -150,19 +165,19 @@ class _FlashFn(torch.autograd.Function):
         delta = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
         if general:
             rc = _bwd_hd()(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse2.data_ptr(), delta.data_ptr(),
-                           dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), B, S, k.shape[1], Hq, Hkv, D, int(bool(causal)),
+                           dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), lib.ptr(ranges), B, S, k.shape[1], Hq, Hkv, D, int(bool(causal)),
                            float(scale), float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
         else:
             rc = (_bwd2() if BWD_PIPELINED else _bwd())(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), lse2.data_ptr(), delta.data_ptr(),
-                        dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), B, S, Hq, Hkv, float(scale),
+                        dq32.data_ptr(), dk.data_ptr(), dv.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg), lib.ptr(ranges), B, S, Hq, Hkv, float(scale),
                         float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
         lib.check_rc(rc, "lvb_flash_attn_bwd")
         dsink = None
-        if sink is not None and ctx.needs_input_grad[10]:
+        if sink is not None and ctx.needs_input_grad[9]:
             # the sink column's probability is 2^(sink log2 e - lse2); its value row is zero, so its logit's gradient is
             # -p_sink * delta summed over batch and queries (delta = rowsum(dO * O), left in the scratch by the kernel)
             dsink = -(torch.exp2(sink.view(1, Hq, 1) * 1.4426950408889634 - lse2) * delta).sum(dim=(0, 2))
-        return dq32.to(torch.bfloat16), dk, dv, None, None, None, None, None, None, None, dsink
+        return dq32.to(torch.bfloat16), dk, dv, None, None, None, None, None, None, dsink
 
 
 PAD_SEGMENT = -2  # segment id of the rows added to bring a sequence to a multiple of 256: they see only one another
@@ -204,13 +219,5 @@ def flash_attention_cuda(q, k, v, mask, *, logits_soft_cap: Optional[float] = No
         k_seg = torch.nn.functional.pad(k_seg, (0, pad_k), value=PAD_SEGMENT)
         q = torch.nn.functional.pad(q, (0, 0, 0, 0, 0, pad))
         k, v = (torch.nn.functional.pad(t, (0, 0, 0, 0, 0, pad_k)) for t in (k, v))
-    kblock_lo = None
-    if q_seg is not None and causal and not pad and getattr(mask, "segments_sorted", False) and not torch.is_grad_enabled():
-        # packed sequences: per block of 128 queries, the first block of 128 keys of the first query's sequence (padding ids < 0
-        # sort last); the forward kernels start their key loop there instead of at the beginning of the packed batch
-        big = torch.iinfo(torch.int32).max
-        ks = torch.where(k_seg < 0, torch.full_like(k_seg, big), k_seg)
-        qs = torch.where(q_seg < 0, torch.full_like(q_seg, big), q_seg)[:, ::128].contiguous()
-        kblock_lo = (torch.searchsorted(ks, qs) // 128).to(torch.int32).contiguous()
-    o = _FlashFn.apply(q, k, v, q_seg, k_seg, scale, logits_soft_cap, window, kblock_lo, causal, sink)
+    o = _FlashFn.apply(q, k, v, q_seg, k_seg, scale, logits_soft_cap, window, causal, sink)
     return o[:, :S] if pad else o

@@ -31,7 +31,6 @@ struct FwdParams {
   float* lse2;          // [B, Hq, S]
   const int* q_seg;     // [B, S] or null
   const int* k_seg;     // [B, S] or null
-  const int* kblock_lo; // optional [B, S / 128]: first block of 128 keys that a query of this 128-row block can attend to
   const float* sink;    // optional [Hq]: a learned logit per head that takes part in the softmax denominator only
   int B, S, Hq, Hkv;    // S: query positions per sequence
   int Sk;               // key positions per sequence (= S unless the mask has no causal part)
@@ -103,11 +102,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   if (p.window > 0) {
     const int first_key = q0 - p.window + 1;
     jlo = first_key > 0 ? first_key / BN : 0;
-  }
-  if (p.kblock_lo != nullptr) {
-    // packed sequences (segment ids ascending): key blocks before the first query's sequence hold nothing these rows can see
-    const int lo = p.kblock_lo[b * nqb + qb];
-    jlo = max(jlo, min(lo, jhi));
   }
   const int nblocks = jhi - jlo + 1;
 
@@ -438,21 +432,20 @@ int launch_fwd(const void* q, const void* k, const void* v, FwdParams p, cudaStr
 // S must be a multiple of 128.  q_seg/k_seg: int32 [B, S] or null.  window: 0 = none.  soft_cap: 0 = none.  sink: fp32 [Hq] or
 // null (a learned logit per head added to the softmax denominator).  Sk: keys per sequence, a multiple of 128 (k / v are
 // [B, Sk, Hkv, D], k_seg [B, Sk]); equal to S when causal.  causal: 0 lets
-// every query see every key of its segment (encoders); window must be 0 and kblock_lo null then.
+// every query see every key of its segment (encoders); window must be 0 then.
 extern "C" int lvb_flash_attn_fwd_hd(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
-                                     const int* k_seg, const int* kblock_lo, const float* sink, int B, int S, int Sk, int Hq, int Hkv,
+                                     const int* k_seg, const float* sink, int B, int S, int Sk, int Hq, int Hkv,
                                      int head_dim, int causal, float scale, float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fa;
   if (B <= 0 || S <= 0 || (S % BM) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
-  if (!causal && (window != 0 || kblock_lo != nullptr)) return kErrBadArg;
+  if (!causal && window != 0) return kErrBadArg;
   if (Sk <= 0 || (Sk % BN) != 0 || (causal && Sk != S)) return kErrBadArg;
   FwdParams p;
   p.O = reinterpret_cast<__nv_bfloat16*>(o);
   p.lse2 = lse2;
   p.q_seg = q_seg;
   p.k_seg = k_seg;
-  p.kblock_lo = kblock_lo;
   p.sink = sink;
   p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale;
@@ -468,7 +461,7 @@ extern "C" int lvb_flash_attn_fwd_hd(const void* q, const void* k, const void* v
 
 // Causal, head_dim 128 (the original entry point).
 extern "C" int lvb_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
-                                  const int* k_seg, const int* kblock_lo, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
+                                  const int* k_seg, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
                                   int window, int* status, void* stream) {
-  return lvb_flash_attn_fwd_hd(q, k, v, o, lse2, q_seg, k_seg, kblock_lo, nullptr, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window, status, stream);
+  return lvb_flash_attn_fwd_hd(q, k, v, o, lse2, q_seg, k_seg, nullptr, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window, status, stream);
 }

@@ -1,5 +1,6 @@
 // Flash attention backward for sm_100a (head_dim 64 or 128, bf16): see the block comment below.
 #include "common.cuh"
+#include "flash_segments.cuh"
 
 namespace lvb {
 namespace fa {
@@ -42,6 +43,7 @@ struct BwdParams {
   const float* delta;          // [B, Hq, S]
   const int* q_seg;
   const int* k_seg;
+  const uint2* ranges;         // with segment ids: (lowest, highest) id per 128 rows, of the queries, then of the keys
   int B, S, Hq, Hkv;           // S: query positions per sequence
   int Sk;                      // key positions per sequence (= S unless the mask has no causal part)
   float scale, soft_cap;
@@ -93,14 +95,23 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const int hkv = blockIdx.y % p.Hkv;
   const int G = p.Hq / p.Hkv;
   const int k0 = jb * BN;
-  const int ilo = causal ? jb : 0;
+  int ilo = causal ? jb : 0;
   int ihi = nqb - 1;
   if (p.window > 0) {
     const int last_q = k0 + BN - 1 + p.window - 1;
     ihi = min(ihi, last_q / BM);
   }
-  const int nq = ihi - ilo + 1;
-  const int iters = nq * G;
+  volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last query block that can see one of the keys
+  if constexpr (kSeg) {
+    if (warp == 2) {
+      const uint2 own = __ldg(p.ranges + p.B * nqb + b * (p.Sk / BN) + jb);
+      const int2 m = seg::meeting_blocks(p.ranges + b * nqb, own, ilo, ihi, lane);
+      if (lane == 0) {  // at least one, so that dK and dV are written
+        bounds[0] = m.x <= m.y ? m.x : ilo;
+        bounds[1] = m.x <= m.y ? m.y : ilo;
+      }
+    }
+  }
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -125,6 +136,12 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if constexpr (kSeg) {
+    ilo = bounds[0];
+    ihi = bounds[1];
+  }
+  const int nq = ihi - ilo + 1;
+  const int iters = nq * G;
   const uint32_t tmem_S = tmem_base;          // also receives dQ
   const uint32_t tmem_dP = tmem_base + 128;
   const uint32_t tmem_dV = tmem_base + 256;
@@ -234,11 +251,23 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const float dlt = p.delta[stat_idx];
       const float neg_lse = (lse == -INFINITY) ? -INFINITY : -lse;
       const int my_seg = kSeg ? p.q_seg[b * p.S + qi] : 0;
+      int ids[2] = {0, 0};
+      if constexpr (kSeg) {
+        ids[0] = __ldg(kseg_g + cbase + lane);
+        ids[1] = __ldg(kseg_g + cbase + 32 + lane);
+      }
       ok = mbar_wait(sdp_full, ph, abort_flag, p.status, 1100, t);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const bool need_mask = (causal && i == jb) || kSeg || (p.window > 0 && k0 <= i * BM + BM - 1 - p.window);
+      uint32_t visible[2] = {0xffffffffu, 0xffffffffu};  // a bit per key of this warp's columns
+      bool need_mask = (causal && i == jb) || (p.window > 0 && k0 <= i * BM + BM - 1 - p.window);
+      if constexpr (kSeg) need_mask = !seg::same_segment<2>(my_seg, ids, visible) || need_mask;
+      if (need_mask) {
+        const int kc = k0 + cbase;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) visible[u] &= seg::bit_range((p.window > 0 ? qi - p.window + 1 : 0) - kc - 32 * u, causal ? qi - kc - 32 * u : 64);
+      }
 #pragma unroll 1
       for (int c = cbase; c < cbase + 64; c += 32) {
         uint32_t sv[32], dv[32];
@@ -246,6 +275,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         tmem_ld_32x32(tmem_dP + lane_addr + c, dv);
         tmem_ld_wait();
         float pe[32], de[32];
+        const uint32_t bits = c == cbase ? visible[0] : visible[1];
 #pragma unroll
         for (int u = 0; u < 32; ++u) {
           float x, dcap = p.scale;
@@ -257,13 +287,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             x = fmaf(__uint_as_float(sv[u]), scale_log2, neg_lse);
           }
           float pv = exp2f(x);
-          if (need_mask) {
-            const int kj = k0 + c + u;
-            bool valid = !causal || kj <= qi;
-            if (p.window > 0) valid = valid && (qi - kj < p.window);
-            if (kSeg) valid = valid && (kseg_g[c + u] == my_seg);
-            pv = valid ? pv : 0.f;
-          }
+          if (need_mask) pv = (bits & (1u << u)) ? pv : 0.f;
           pe[u] = pv;
           de[u] = pv * (__uint_as_float(dv[u]) - dlt) * dcap;
         }
@@ -422,14 +446,15 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
 }  // namespace lvb
 
 // Backward of lvb_flash_attn_fwd_hd.  dq32: fp32 [B,S,Hq,D], must be zero on entry.  delta: fp32 [B,Hq,S] scratch.  D = head_dim
-// is 64 or 128; causal and Sk (keys per sequence: k / v / dk / dv are [B, Sk, Hkv, D]) as in the forward.
+// is 64 or 128; causal and Sk (keys per sequence: k / v / dk / dv are [B, Sk, Hkv, D]) as in the forward.  ranges: of
+// lvb_segment_ranges, with segment ids.
 extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                      const float* lse2, float* delta, float* dq32, void* dk, void* dv, const int* q_seg,
-                                     const int* k_seg, int B, int S, int Sk, int Hq, int Hkv, int head_dim, int causal, float scale,
+                                     const int* k_seg, const void* ranges, int B, int S, int Sk, int Hq, int Hkv, int head_dim, int causal, float scale,
                                      float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fa;
-  if (B <= 0 || S <= 0 || (S % BM) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
+  if (B <= 0 || S <= 0 || (S % BM) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
   if (!causal && window != 0) return kErrBadArg;
   if (Sk <= 0 || (Sk % BN) != 0 || (causal && Sk != S)) return kErrBadArg;
   BwdParams p;
@@ -440,6 +465,7 @@ extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v
   p.delta = delta;
   p.q_seg = q_seg;
   p.k_seg = k_seg;
+  p.ranges = reinterpret_cast<const uint2*>(ranges);
   p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.soft_cap = soft_cap; p.window = window;
   p.causal = causal ? 1 : 0;
@@ -453,8 +479,8 @@ extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v
 // Causal, head_dim 128 (the original entry point).
 extern "C" int lvb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
                                   const float* lse2, float* delta, float* dq32, void* dk, void* dv, const int* q_seg,
-                                  const int* k_seg, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
+                                  const int* k_seg, const void* ranges, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
                                   int window, int* status, void* stream) {
-  return lvb_flash_attn_bwd_hd(q, k, v, o, d_o, lse2, delta, dq32, dk, dv, q_seg, k_seg, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window,
+  return lvb_flash_attn_bwd_hd(q, k, v, o, d_o, lse2, delta, dq32, dk, dv, q_seg, k_seg, ranges, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window,
                                status, stream);
 }

@@ -25,6 +25,7 @@
 // this file.  Semantics of the reference's fused attention (src/levanter/layers/attention.py:533-544,
 // src/levanter/models/flash_attention.py:143-385).
 #include "common.cuh"
+#include "flash_segments.cuh"
 
 namespace lvb {
 namespace fab2 {
@@ -47,6 +48,7 @@ struct Params {
   const float* delta;  // [B, Hq, S]
   const int* q_seg;
   const int* k_seg;
+  const uint2* ranges;  // with segment ids: (lowest, highest) id per 128 rows, of the queries, then of the keys
   int B, S, Hq, Hkv;
   float scale, soft_cap;
   int window;
@@ -58,8 +60,8 @@ struct Smem {
   static constexpr int kV = kK + kKVTile;
   static constexpr int kQ = kV + kKVTile;          // two buffers of {Q tile, dO tile}
   static constexpr int kP = kQ + 2 * 2 * kQTile;   // two buffers of {P^T tile, dS^T tile}
-  static constexpr int kStat = kP + 2 * 2 * kPTile;  // per warpgroup: lse2[64], delta[64], q_seg[64]
-  static constexpr int kBars = kStat + 2 * 3 * 64 * 4;
+  static constexpr int kStat = kP + 2 * 2 * kPTile;  // per warpgroup: lse2[64], delta[64]
+  static constexpr int kBars = kStat + 2 * 2 * 64 * 4;
   static constexpr int kNumBars = 13;
   static constexpr int kTotal = kBars + kNumBars * 8 + 16 + 1024;
 };
@@ -122,14 +124,23 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int hkv = blockIdx.y % p.Hkv;
   const int G = p.Hq / p.Hkv;
   const int k0 = jb * BKEYS;
-  const int ilo = k0 / BQ;  // first block of 64 queries that can see a key of this block
+  int ilo = k0 / BQ;  // first block of 64 queries that can see a key of this block
   int ihi = nqb - 1;
   if (p.window > 0) {
     const int last_q = k0 + BKEYS - 1 + p.window - 1;
     ihi = min(ihi, last_q / BQ);
   }
-  const int nq = ihi - ilo + 1;
-  const int iters = nq * G;
+  volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last block of 128 queries that can see one
+  if constexpr (kSeg) {
+    if (warp == 2) {
+      const uint2 own = __ldg(p.ranges + p.B * (p.S / BKEYS) + b * (p.S / BKEYS) + jb);
+      const int2 m = seg::meeting_blocks(p.ranges + b * (p.S / BKEYS), own, ilo * BQ / BKEYS, ihi * BQ / BKEYS, lane);
+      if (lane == 0) {  // at least one, so that dK and dV are written
+        bounds[0] = m.x <= m.y ? m.x : jb;
+        bounds[1] = m.x <= m.y ? m.y : jb;
+      }
+    }
+  }
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -158,6 +169,12 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if constexpr (kSeg) {
+    ilo = max(ilo, bounds[0] * (BKEYS / BQ));
+    ihi = min(ihi, bounds[1] * (BKEYS / BQ) + BKEYS / BQ - 1);
+  }
+  const int nq = ihi - ilo + 1;
+  const int iters = nq * G;
   // pair w: S^T at columns [128 w, 128 w + 64) (later dQ^T), dP^T at [128 w + 64, 128 w + 128)
   const uint32_t tmem_dV = tmem_base + 256;
   const uint32_t tmem_dK = tmem_base + 384;
@@ -262,24 +279,26 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const float scale_log2 = p.scale * 1.4426950408889634f;
     const int kj = k0 + r;
     const int my_kseg = kSeg ? p.k_seg[b * p.S + kj] : 0;
-    float* s_lse = reinterpret_cast<float*>(smem + Smem::kStat + wg * (3 * 64 * 4));
+    float* s_lse = reinterpret_cast<float*>(smem + Smem::kStat + wg * (2 * 64 * 4));
     float* s_dlt = s_lse + 64;
-    int* s_qseg = reinterpret_cast<int*>(s_dlt + 64);
     uint8_t* sPT = smem + Smem::kP + wg * (2 * kPTile);
     uint8_t* sDST = sPT + kPTile;
     const uint32_t tmem_ST = tmem_base + wg * 128, tmem_dPT = tmem_ST + 64;
     bool ok = true;
-    // The per-query statistics of a step (64 x {-lse, delta, segment id}) are fetched one step of this warpgroup ahead into a
+    // The per-query statistics of a step (64 x {-lse, delta}, and the segment ids, two per lane) are fetched one step of this warpgroup ahead into a
     // register per thread, so the global-memory latency is not paid between the two barriers that open a step.
     float pre_stat = 0.f;
-    int pre_seg = 0;
+    int ids[2] = {0, 0};
     auto fetch_stats = [&](int tt) {
       if (tt >= iters) return;
       const int hh = hkv * G + tt / nq;
       const int qq = (ilo + (tt % nq)) * BQ;
       const size_t stat = (static_cast<size_t>(b) * p.Hq + hh) * p.S + qq;
       pre_stat = (wtid < 64) ? p.lse2[stat + wtid] : p.delta[stat + wtid - 64];
-      if (kSeg && wtid < 64) pre_seg = p.q_seg[b * p.S + qq + wtid];
+      if constexpr (kSeg) {
+        ids[0] = __ldg(p.q_seg + b * p.S + qq + lane);
+        ids[1] = __ldg(p.q_seg + b * p.S + qq + 32 + lane);
+      }
     };
     fetch_stats(wg);
     for (int t = wg; t < iters; t += 2) {
@@ -290,6 +309,13 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int q0 = i * BQ;
       // Every warp of the warpgroup passes the three named barriers of a step whatever happened to its waits (a wait that
       // ran out clears `ok` and the work is skipped), or the others would wait for it for ever.
+      uint32_t visible[2] = {0xffffffffu, 0xffffffffu};  // a bit per query
+      bool need_mask = (q0 < k0 + BKEYS) || (p.window > 0 && k0 <= q0 + BQ - 1 - p.window);
+      if constexpr (kSeg) need_mask = !seg::same_segment<2>(my_kseg, ids, visible) || need_mask;
+      if (need_mask) {  // a key is seen by the queries kj .. kj + window - 1 (of its segment)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) visible[u] &= seg::bit_range(kj - q0 - 32 * u, p.window > 0 ? kj + p.window - 1 - q0 - 32 * u : BQ);
+      }
       wg_bar_sync(wg);  // the previous step no longer reads the statistics, and its dQ tile has been handed to the TMA unit
       if (ok) {
         if (wtid < 64) {
@@ -297,7 +323,6 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         } else {
           s_dlt[wtid - 64] = pre_stat;
         }
-        if (kSeg && wtid < 64) s_qseg[wtid] = pre_seg;
         fetch_stats(t + 2);
         // the bulk reduction of the previous step must have read its tile before this step's P^T / dS^T overwrite it
         if (wtid == 0) bulk_wait_read<0>();
@@ -309,7 +334,6 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       if (ok) {
         tc_fence_after();
-        const bool need_mask = (q0 < k0 + BKEYS) || kSeg || (p.window > 0 && k0 <= q0 + BQ - 1 - p.window);
 #pragma unroll 1
         for (int c = 0; c < BQ; c += 32) {
           uint32_t sv[32], dv[32];
@@ -317,6 +341,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tmem_ld_32x32(tmem_dPT + lane_addr + c, dv);
           tmem_ld_wait();
           float pe[32], de[32];
+          const uint32_t bits = c == 0 ? visible[0] : visible[1];
 #pragma unroll
           for (int u = 0; u < 32; ++u) {
             float x, dcap = p.scale;
@@ -329,13 +354,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
               x = fmaf(__uint_as_float(sv[u]), scale_log2, neg_lse);
             }
             float pv = exp2f(x);
-            if (need_mask) {
-              const int qi = q0 + c + u;
-              bool valid = kj <= qi;
-              if (p.window > 0) valid = valid && (qi - kj < p.window);
-              if (kSeg) valid = valid && (s_qseg[c + u] == my_kseg);
-              pv = valid ? pv : 0.f;
-            }
+            if (need_mask) pv = (bits & (1u << u)) ? pv : 0.f;
             pe[u] = pv;
             de[u] = pv * (__uint_as_float(dv[u]) - s_dlt[c + u]) * dcap;
           }
@@ -437,14 +456,14 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }  // namespace fab2
 }  // namespace lvb
 
-// Backward of lvb_flash_attn_fwd, pipelined form (same arguments as lvb_flash_attn_bwd).  dq32: fp32 [B,S,Hq,128], must be
+// Backward of lvb_flash_attn_fwd, pipelined form (arguments of lvb_flash_attn_bwd, whose ranges come from lvb_segment_ranges).  dq32: fp32 [B,S,Hq,128], must be
 // zero on entry.  delta: fp32 [B,Hq,S] scratch.
 extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse2,
-                                   float* delta, float* dq32, void* dk, void* dv, const int* q_seg, const int* k_seg, int B, int S,
+                                   float* delta, float* dq32, void* dk, void* dv, const int* q_seg, const int* k_seg, const void* ranges, int B, int S,
                                    int Hq, int Hkv, float scale, float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fab2;
-  if (B <= 0 || S <= 0 || (S % BKEYS) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
+  if (B <= 0 || S <= 0 || (S % BKEYS) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   {
     const long long rows = static_cast<long long>(B) * S * Hq;
@@ -485,6 +504,7 @@ extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, 
   p.delta = delta;
   p.q_seg = q_seg;
   p.k_seg = k_seg;
+  p.ranges = reinterpret_cast<const uint2*>(ranges);
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.soft_cap = soft_cap; p.window = window;
   p.status = status;

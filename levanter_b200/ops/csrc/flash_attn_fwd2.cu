@@ -24,6 +24,7 @@
 // epilogue forms a1 - weight * a2, its norm over the values and the gate straight from the two accumulators.  The warps of a tile
 // take alternate groups of 32 columns of the result.
 #include "common.cuh"
+#include "flash_segments.cuh"
 
 namespace lvb {
 namespace fa2 {
@@ -41,13 +42,13 @@ struct Params {
   float* lse2;
   const int* q_seg;
   const int* k_seg;
-  const int* kblock_lo;  // optional [B, S / 128]: first block of 128 keys that a query of this 128-row block can attend to
+  const uint2* ranges;   // with segment ids: (lowest, highest) id per 128 rows, [B, S / 128] of the queries, then [B, Sk / 128] of the keys
   const float* sink;     // optional [Hq]: a learned logit per head that takes part in the softmax denominator only
   int B, S, Hq, Hkv;  // S: query positions per sequence
   int Sk;             // key positions per sequence (= S unless the mask has no causal part: cross attention)
   float scale, soft_cap;
   int window;
-  int causal;  // 0: every key is visible (subject to segment ids); window must be 0 and kblock_lo null then
+  int causal;  // 0: every key is visible (subject to segment ids); window must be 0 then
   int* status;
   // ---- kPacked
   const int* pos;            // [S]: position of each packed row in its sequence
@@ -73,7 +74,7 @@ struct SmemT {
   static constexpr int kV = kK + kKStages * kQKTile;
   static constexpr int kBars = kV + kVStages * kVTile;
   static constexpr int kNumBars = 1 + 2 * kKStages + 2 * kStages + 2 + 2 + 2;
-  static constexpr int kTotal = kBars + kNumBars * 8 + 16 + 1024;
+  static constexpr int kTotal = kBars + kNumBars * 8 + 16 + 1024;  // + TMEM address, abort flag, two bounds
 };
 
 template <bool kValue>
@@ -151,14 +152,20 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int first_key = q0 - p.window + 1;
     jlo = first_key > 0 ? first_key / BT : 0;
   }
-  if (p.kblock_lo != nullptr) {
-    // packed sequences (segment ids ascending): key blocks before the first query's sequence hold nothing these rows can see
-    const int lo = p.kblock_lo[b * (p.S / BT) + jdiagA];
-    jlo = max(jlo, min(lo, jdiagA));
-  }
   if constexpr (kPacked) jlo = row_lower_bound(p, q0) / BT;  // bounds do not decrease along the packed rows
-  const int nB = (causal ? jdiagB : p.Sk / BT - 1) - jlo + 1;  // blocks processed by tile B
-  const int nA = causal && !kMaps ? nB - 1 : nB;              // causal: tile A stops one block earlier (its diagonal)
+  int jend = causal ? jdiagB : p.Sk / BT - 1;
+  volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last key block that these rows can see
+  if constexpr (kSeg) {
+    if (warp == 2) {
+      const uint2* own = p.ranges + b * (p.S / BT) + 2 * cb;
+      const uint2 ra = __ldg(own), rb = __ldg(own + 1);
+      const int2 m = seg::meeting_blocks(p.ranges + p.B * (p.S / BT) + b * (p.Sk / BT), make_uint2(min(ra.x, rb.x), max(ra.y, rb.y)), jlo, jend, lane);
+      if (lane == 0) {  // at least one block (and the diagonal ones), so that rows that see nothing are written too
+        bounds[0] = min(m.x, causal ? jdiagA : jend);
+        bounds[1] = max(m.y, jlo);
+      }
+    }
+  }
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -189,6 +196,12 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if constexpr (kSeg) {
+    jlo = bounds[0];
+    if (!causal) jend = max(bounds[1], jlo);
+  }
+  const int nB = jend - jlo + 1;                  // blocks processed by tile B
+  const int nA = causal && !kMaps ? nB - 1 : nB;  // causal: tile A stops one block earlier (its diagonal)
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -342,38 +355,39 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int it = 0; it < nT && ok; ++it) {
       const int j = jlo + it;
       const int k0 = j * BT;
+      int ids[4] = {0, 0, 0, 0};
+      if constexpr (kSeg) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ids[i] = __ldg(kseg_row + k0 + 32 * i + lane);
+      }
       ok = mbar_wait(&s_full[tile], it & 1, abort_flag, p.status, 1400 + tile, it);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const bool need_mask = (j == jdiag) || kSeg || (kPacked && k0 < tile_lo) || (!kPacked && p.window > 0 && k0 <= q0 + tile * BT + BT - 1 - p.window);
-
-      // what the row sees of the block: columns col_lo .. col_lo + col_span (with segment ids: those of its segment)
+      bool need_mask = (j == jdiag) || (kPacked && k0 < tile_lo) || (!kPacked && p.window > 0 && k0 <= q0 + tile * BT + BT - 1 - p.window);
+      // what the row sees of the block: columns col_lo .. col_lo + col_span (with segment ids: those of its segment, a bit per column)
       const int col_lo = (kPacked ? row_lo : p.window > 0 ? qi - p.window + 1 : 0) - k0;
       const unsigned col_span = causal ? static_cast<unsigned>(qi - k0 - col_lo) : 0x7fffffffu;
-      uint32_t same[4] = {0u, 0u, 0u, 0u};  // kSeg: a bit per column, set in pass 1
+      uint32_t visible[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+      if constexpr (kSeg) {
+        need_mask = !seg::same_segment<4>(my_seg, ids, visible) || need_mask;
+        if (need_mask) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) visible[i] &= seg::bit_range(col_lo - 32 * i, (causal ? qi - k0 : BT) - 32 * i);
+        }
+      }
       auto mask = [&](uint32_t (&v)[2][32], int c) {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const uint32_t bits = c == 0 ? same[i] : same[2 + i];
+          uint32_t bits = c == 0 ? visible[i] : visible[2 + i];
+          asm volatile("" : "+r"(bits));  // or the tests of all columns are made ahead and held in registers
 #pragma unroll
           for (int t = 0; t < 32; ++t) {
-            bool valid = static_cast<unsigned>(c + 32 * i + t - col_lo) <= col_span;
-            if (kSeg) valid = valid && ((bits >> t) & 1u);
-            if (!valid) v[i][t] = __float_as_uint(-INFINITY);
+            const bool seen = kSeg ? (bits & (1u << t)) != 0u : static_cast<unsigned>(c + 32 * i + t - col_lo) <= col_span;
+            if (!seen) v[i][t] = __float_as_uint(-INFINITY);
           }
         }
       };
-      if constexpr (kSeg) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll 2
-          for (int t = 0; t < 32; t += 4) {
-            const int4 seg = __ldg(reinterpret_cast<const int4*>(kseg_row + k0 + 32 * i + t));
-            same[i] |= (seg.x == my_seg ? 1u << t : 0u) | (seg.y == my_seg ? 2u << t : 0u) | (seg.z == my_seg ? 4u << t : 0u) |
-                       (seg.w == my_seg ? 8u << t : 0u);
-          }
-      }
 
       // ---- pass 1: row maximum (raw logits; the scale is positive and the soft-cap monotonic).  Rolled loops over 64 columns: unrolled
       // further, the code no longer fits the instruction cache
@@ -644,24 +658,55 @@ int launch_hd(const void* q, const void* k, const void* v, const Params& p, cuda
 }  // namespace fa2
 }  // namespace lvb
 
+namespace lvb {
+namespace seg {
+// ranges[i] = (lowest, highest) of the ids of block i; blocks [0, nq) are q_seg's, the following ones k_seg's
+__global__ void block_ranges_kernel(const int* __restrict__ q_seg, const int* __restrict__ k_seg, uint2* __restrict__ ranges, int nq, int n) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= n) return;
+  const int* src = i < nq ? q_seg + static_cast<long long>(i) * kBlock : k_seg + static_cast<long long>(i - nq) * kBlock;
+  uint32_t lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+  for (int t = 0; t < kBlock / 32; ++t) {
+    const uint32_t v = static_cast<uint32_t>(__ldg(src + 32 * t + lane));
+    lo = min(lo, v);
+    hi = max(hi, v);
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if (lane == 0) ranges[i] = make_uint2(lo, hi);
+}
+}  // namespace seg
+}  // namespace lvb
+
+// ranges[0 .. B (S + Sk) / 128): (lowest, highest) segment id, as unsigned numbers, per 128 rows of q_seg [B, S] and then of k_seg [B, Sk]
+// (S and Sk multiples of 128).
+extern "C" int lvb_segment_ranges(const int* q_seg, const int* k_seg, int B, int S, int Sk, void* ranges, void* stream) {
+  using namespace lvb;
+  if (B <= 0 || S <= 0 || Sk <= 0 || (S % seg::kBlock) != 0 || (Sk % seg::kBlock) != 0 || q_seg == nullptr || k_seg == nullptr) return kErrBadArg;
+  const int nq = B * (S / seg::kBlock), n = nq + B * (Sk / seg::kBlock);
+  seg::block_ranges_kernel<<<(n + 3) / 4, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(q_seg, k_seg, reinterpret_cast<uint2*>(ranges), nq, n);
+  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+}
+
 // Same contract as lvb_flash_attn_fwd_hd (head_dim 64 or 128, causal or not, optional sink logits [Hq]), but S must be a
 // multiple of 256: two query tiles per CTA.  Sk: keys per sequence, a multiple of 128 (k / v are [B, Sk, Hkv, D], k_seg [B, Sk]);
-// Sk must equal S when causal.
+// Sk must equal S when causal.  ranges: what lvb_segment_ranges makes of the segment ids.
 extern "C" int lvb_flash_attn_fwd2_hd(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
-                                      const int* k_seg, const int* kblock_lo, const float* sink, int B, int S, int Sk, int Hq, int Hkv,
+                                      const int* k_seg, const void* ranges, const float* sink, int B, int S, int Sk, int Hq, int Hkv,
                                       int head_dim, int causal, float scale, float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fa2;
   if (B <= 0 || S <= 0 || (S % (2 * BT)) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
-  if (!causal && (window != 0 || kblock_lo != nullptr)) return kErrBadArg;
+  if ((!causal && window != 0) || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
   if (Sk <= 0 || (Sk % BT) != 0 || (causal && Sk != S)) return kErrBadArg;
-  if (reinterpret_cast<uintptr_t>(k_seg) & 15) return kErrBadArg;
   Params p;
   p.O = reinterpret_cast<__nv_bfloat16*>(o);
   p.lse2 = lse2;
   p.q_seg = q_seg;
   p.k_seg = k_seg;
-  p.kblock_lo = kblock_lo;
+  p.ranges = reinterpret_cast<const uint2*>(ranges);
   p.sink = sink;
   p.B = B; p.S = S; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.soft_cap = soft_cap; p.window = window;
@@ -677,9 +722,9 @@ extern "C" int lvb_flash_attn_fwd2_hd(const void* q, const void* k, const void* 
 
 // Causal, head_dim 128 (the original entry point).
 extern "C" int lvb_flash_attn_fwd2(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
-                                   const int* k_seg, const int* kblock_lo, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
+                                   const int* k_seg, const void* ranges, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
                                    int window, int* status, void* stream) {
-  return lvb_flash_attn_fwd2_hd(q, k, v, o, lse2, q_seg, k_seg, kblock_lo, nullptr, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window, status, stream);
+  return lvb_flash_attn_fwd2_hd(q, k, v, o, lse2, q_seg, k_seg, ranges, nullptr, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window, status, stream);
 }
 
 // Causal attention over T packed rows (T a multiple of 256) of sequences that each start at position 0:
@@ -703,7 +748,7 @@ extern "C" int lvb_flash_attn_fwd_packed(const void* q, const void* k, const voi
   if ((reinterpret_cast<uintptr_t>(o) & 15) || (weight != nullptr && sink != nullptr)) return kErrBadArg;
   Params p;
   p.O = reinterpret_cast<__nv_bfloat16*>(o);
-  p.lse2 = nullptr; p.q_seg = nullptr; p.k_seg = nullptr; p.kblock_lo = nullptr; p.sink = sink;
+  p.lse2 = nullptr; p.q_seg = nullptr; p.k_seg = nullptr; p.ranges = nullptr; p.sink = sink;
   p.B = 1; p.S = T; p.Sk = T; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.soft_cap = soft_cap; p.window = window; p.causal = 1; p.status = status;
   p.pos = pos; p.chunk = chunk; p.dk = dk; p.dv = dv;

@@ -247,3 +247,24 @@ def test_cross_attention_with_different_query_and_key_lengths(D, Sq, Sk, Hq, Hkv
     assert KFA.supported(q, k, v, None, None, True, None)
     assert not KFA.supported(q, k, v, AttentionMask.causal(), None, True, None)
     assert not KFA.supported(q[:, :1], k, v, None, None, True, None)
+
+
+@pytest.mark.parametrize("D,causal,window", [(128, True, None), (64, True, None), (128, False, None), (64, False, None), (128, True, 150), (64, True, 150)])
+@pytest.mark.parametrize("layout", ["packed", "scattered", "single", "foreign_first"])
+def test_blocks_of_other_segments_are_left_out(layout, D, causal, window):
+    """Segments in any order: blocks without a common id are skipped in both passes, blocks of one id need no mask, and mixed blocks (many ids
+    in one warp among them) are masked column by column."""
+    S = 896
+    at = torch.arange(S, device="cuda")
+    if layout == "packed":  # edges inside, at and one off the tiles of 32, 64, 128 and 256
+        seg = sum((at >= e).int() for e in (1, 31, 64, 128, 255, 257, 512, 515, 700))
+    elif layout == "scattered":  # each id in several places, 40 ids within one block
+        seg = (at // 128 * 7) % 3 + torch.where((at >= 256) & (at < 384), at % 40, torch.zeros_like(at))
+    elif layout == "single":
+        seg = torch.full_like(at, 5)
+    else:  # ids that decrease, and a negative one first
+        seg = torch.where(at < 200, torch.full_like(at, -3), 9 - at // 300)
+    seg = torch.stack((seg.int(), seg.roll(77).int()))
+    mask = (AttentionMask.causal(sliding_window=window) if causal else AttentionMask(is_causal=False)).with_segment_ids(seg)
+    _run(2, S, 4, 2, mask, D=D, seed=3)
+    _run(2, S, 2, 2, mask, D=D, seed=4, soft_cap=15.0)
