@@ -25,7 +25,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..layers.normalization import LayerNormConfigBase, RmsNormConfig
 from ..nn import Embedding, Linear
-from ..ops.delta_rule import chunk_state_scan
+from ..ops.delta_rule import chunk_state_scan, gated_delta_rule, gated_delta_rule_supported, gated_out_norm
 from ..ops.dwconv import causal_dwconv
 from ..utils.activation import ActivationFunctionEnum
 from ..utils.flop_utils import lm_flops_per_token
@@ -57,7 +57,13 @@ def delta_rule_chunked_scan(q, k, v, g, beta, chunk_size: int = 64, initial_stat
     B, H, L, dk = q.shape
     dv = v.shape[-1]
     dtype = v.dtype
-    q, k, v, g, beta = (t.float() for t in (q, k, v, g, beta))
+    if not q.dtype == k.dtype == v.dtype == torch.bfloat16:
+        q, k, v = q.float(), k.float(), v.float()
+    g, beta = g.float(), beta.float()
+    if gated_delta_rule_supported(q, k, v, chunk_size):
+        out, S = gated_delta_rule(*(t.transpose(1, 2) for t in (q, k, v, g, beta)), initial_state, scale=dk ** -0.5)
+        return out.reshape(B, H, -1, dv)[:, :, :L].to(dtype), S
+    q, k, v = q.float(), k.float(), v.float()
     pad = (-L) % chunk_size
     if pad:
         q, k, v = (F.pad(t, (0, 0, 0, pad)) for t in (q, k, v))
@@ -175,13 +181,17 @@ class GatedDeltaNetLayer(nn.Module):
         q = self._conv(self.q_conv1d, self.q_proj(x)).view(B, L, Hk, dk)
         k = self._conv(self.k_conv1d, self.k_proj(x)).view(B, L, Hk, dk)
         v = self._conv(self.v_conv1d, self.v_proj(x)).view(B, L, H, dv)
-        q = F.normalize(q.float(), dim=-1)
-        k = F.normalize(k.float(), dim=-1)
-        if Hk != H:
-            q = q.repeat_interleave(H // Hk, dim=2)
-            k = k.repeat_interleave(H // Hk, dim=2)
         beta = torch.sigmoid(self.b_proj(x).float())  # [B, L, H]
         g = -self.A_log.float().exp() * F.softplus(self.a_proj(x).float() + self.dt_bias.float())
+        if Hk == H and dv <= 512 and gated_delta_rule_supported(q, k, v, c.chunk_size):
+            o, _ = gated_delta_rule(q, k, v, g, beta, scale=dk ** -0.5, normalize=True)
+            y = gated_out_norm(o, self.g_proj(x).view(B, L, H, dv), self.o_norm_weight, c.layer_norm_epsilon)
+            return self.o_proj(y.view(B, L, H * dv).to(x.dtype))
+        q = F.normalize(q.float(), dim=-1)
+        k = F.normalize(k.float(), dim=-1)
+        if Hk != H:  # the gradients of a group's heads are added in fp32 before the norm
+            q = q.repeat_interleave(H // Hk, dim=2)
+            k = k.repeat_interleave(H // Hk, dim=2)
         o, _ = delta_rule_chunked_scan(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2).float(), g.transpose(1, 2),
                                        beta.transpose(1, 2), chunk_size=c.chunk_size)
         o = o.transpose(1, 2)  # [B, L, H, dv]

@@ -381,12 +381,12 @@ def main(argv=None):
         shape = {"batch": a.batch, "seq": a.seq, "hidden": a.hidden, "heads": a.heads}
         ms, mn = _time(step, a.iters, a.warmup, flush)
         _report("gated_deltanet_layer_fwd_bwd", shape, ms, mn)
-        kernels = (G.chunk_state_scan, G.causal_dwconv)
-        G.chunk_state_scan, G.causal_dwconv = chunk_state_scan_reference, causal_dwconv_reference
+        kernels = (G.chunk_state_scan, G.causal_dwconv, G.gated_delta_rule_supported)
+        G.chunk_state_scan, G.causal_dwconv, G.gated_delta_rule_supported = chunk_state_scan_reference, causal_dwconv_reference, lambda *a: False
         try:
             ms, mn = _time(step, max(a.iters // 4, 2), 2, flush)
         finally:
-            G.chunk_state_scan, G.causal_dwconv = kernels
+            G.chunk_state_scan, G.causal_dwconv, G.gated_delta_rule_supported = kernels
         return _report("gated_deltanet_layer_fwd_bwd_framework_ops", shape, ms, mn)
 
     if a.kernel == "sampler":

@@ -30,7 +30,7 @@ SERVING_SOURCES = ("attention_any", "depth_stream", "elementwise", "flash_attn_f
 
 # Kernels whose results are 32-bit throughout (norms of an fp32 stream, router scores, rotary angles, recurrences, fp32 attention): no
 # fast-math exponentials, divisions or square roots.
-ACCURATE_SOURCES = ("attention_any", "depth_stream", "gated_scan", "linear_attention", "linear_attention_umma", "moe_experts", "qkv_prep",
+ACCURATE_SOURCES = ("attention_any", "delta_chunks", "depth_stream", "gated_scan", "linear_attention", "linear_attention_umma", "moe_experts", "qkv_prep",
                     "residual_stream")
 
 NVCC_FLAGS = [

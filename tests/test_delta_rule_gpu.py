@@ -94,3 +94,74 @@ def test_chunked_scan_on_kernels_matches_recurrence():
     torch.testing.assert_close(s, s_ref, atol=2e-2, rtol=2e-2)
     for x, y in zip(grads, g_ref):
         assert (x - y).abs().max().item() <= 2e-2 * (y.abs().max().item() + 1e-6)
+
+
+def _rule64(q, k, v, g, beta, S, scale, normalize):
+    """The recurrence token by token in 64 bits: ``q, k, v [B, L, H, d]``."""
+    q, k, v, g, beta, S = (t.double().cpu() for t in (q, k, v, g, beta, S))
+    if normalize:
+        q, k = (torch.nn.functional.normalize(t, dim=-1) for t in (q, k))
+    out = []
+    for t in range(q.shape[1]):
+        S = S * g[:, t].exp()[..., None, None]
+        S = S + torch.einsum("bhk,bhv->bhkv", k[:, t], (v[:, t] - torch.einsum("bhk,bhkv->bhv", k[:, t], S)) * beta[:, t, :, None])
+        out.append(torch.einsum("bhk,bhkv->bhv", q[:, t] * scale, S))
+    return torch.stack(out, dim=1), S
+
+
+@pytest.mark.parametrize("B,L,H,dk,dv,dtype,normalize", [
+    (1, 1, 1, 64, 64, torch.float32, False), (2, 63, 2, 128, 128, torch.bfloat16, True), (1, 64, 3, 128, 64, torch.float32, True),
+    (1, 65, 2, 64, 192, torch.bfloat16, True), (1, 200, 2, 128, 256, torch.float32, False)])
+@pytest.mark.parametrize("strided", [False, True])
+def test_gated_delta_rule_matches_the_recurrence_in_64_bits(B, L, H, dk, dv, dtype, normalize, strided):
+    """With fp32 products in the loop everything is fp32: sums of a few hundred terms over states that decay, 2e-4 as for the loop alone.  bf16
+    inputs are exact in fp32; their gradients are rounded once (2^-9)."""
+    from levanter_b200.ops import lib
+    from levanter_b200.ops.delta_rule import gated_delta_rule
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+
+    def rows(d):  # a row of all heads inside a wider one, or heads before positions
+        x = make(B, L, H, d).to(dtype)
+        return x if not strided else x.transpose(1, 2).contiguous().transpose(1, 2) if d == dv else torch.cat((x, x), dim=-1)[..., :d]
+
+    q, k, v = rows(dk), rows(dk), rows(dv)
+    if not normalize:
+        q, k = q * 0.1, (k.float() * dk ** -0.5).to(dtype)
+    g, beta, S0 = -make(B, L, H).abs() * 0.1, make(B, L, H).sigmoid(), make(B, H, dk, dv) * 0.3
+    go, gs = make(B, L, H, dv), make(B, H, dk, dv)
+    args = [t.detach().requires_grad_() for t in (q, k, v, g, beta, S0)]
+    out, S = gated_delta_rule(*args, scale=dk ** -0.5, normalize=normalize, exact=True)
+    o = out.reshape(B, H, -1, dv)[:, :, :L].transpose(1, 2)
+    ((o * go).sum() + (S * gs).sum()).backward()
+    lib.check_status()
+    ref = [t.detach().requires_grad_() for t in (q, k, v, g, beta, S0)]
+    o64, S64 = _rule64(*ref, dk ** -0.5, normalize)
+    ((o64 * go.double().cpu()).sum() + (S64 * gs.double().cpu()).sum()).backward()
+    tol = 2e-4
+    for what, x, y in [("out", o, o64), ("state", S, S64)] + [(f"d{n}", a.grad, r.grad) for n, a, r in zip("q k v g beta S0".split(), args, ref)]:
+        x, y = x.detach().double().cpu(), y.detach().double().cpu()
+        limit = tol + (2 ** -8 if dtype == torch.bfloat16 and what in ("dq", "dk", "dv") else 0.0)
+        assert (x - y).norm() <= limit * y.norm() + 1e-9, f"{what}: {(x - y).norm() / y.norm()}"
+
+
+@pytest.mark.parametrize("dv,dtype", [(64, torch.float32), (128, torch.bfloat16), (512, torch.bfloat16)])
+def test_gated_out_norm_matches_64_bits(dv, dtype):
+    from levanter_b200.ops.delta_rule import gated_out_norm
+
+    B, L, H, eps = 2, 70, 3, 1e-6
+    o = torch.randn(B, H, 2, 64, dv, device="cuda", requires_grad=True)
+    gate = torch.randn(B, L, H, dv, device="cuda").to(dtype).requires_grad_()
+    w = torch.rand(dv, device="cuda").add(0.5).to(dtype).requires_grad_()
+    dy = torch.randn(B, L, H, dv, device="cuda").to(dtype)
+    y = gated_out_norm(o, gate, w, eps)
+    y.backward(dy)
+    o64, g64, w64 = (t.detach().double().requires_grad_() for t in (o, gate, w))
+    x = o64.reshape(B, H, -1, dv)[:, :, :L].transpose(1, 2)
+    y64 = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w64 * torch.nn.functional.silu(g64)
+    y64.backward(dy.double())
+    for a, b in ((y, y64), (o.grad, o64.grad), (gate.grad, g64.grad), (w.grad, w64.grad)):
+        tol = 2 ** -8 if a.dtype == torch.bfloat16 else 1e-5
+        assert (a.double() - b).norm() <= tol * b.norm()
+    assert not o.grad.reshape(B, H, -1, dv)[:, :, L:].any()
