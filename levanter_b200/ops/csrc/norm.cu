@@ -12,7 +12,9 @@
 namespace lvb {
 namespace norm {
 
-constexpr int kMaxVecPerThread = 8;  // backward keeps dw partials in registers: dim <= TX*8*8
+constexpr int kMaxThreads = 512;
+constexpr int kFewRows = 1024;  // up to here a block per row beats a warp per row: fewer warps than the SMs' schedulers hold twice
+constexpr int kMaxVecPerThread = 4;  // backward keeps dw partials in registers: dim <= 512 * 4 * 8
 
 struct Vec8 {
   float v[8];
@@ -71,17 +73,19 @@ __device__ __forceinline__ Vec8 loadw8(const void* w, int wf32, int col, float o
   return o;
 }
 
-// Sum over the TX threads of a row.  TX is a power of two; rows never straddle
-// warps when TX <= 32, otherwise TX is a multiple of 32 and shared memory joins the warps.
+// Sum over the TX threads of a row.  TX is a power of two up to 32 (rows never straddle warps then) or a multiple of 32, where shared memory joins
+// the warps behind one barrier: a caller that comes here again takes the other half of the scratch (2 * reduce_floats).
+__host__ __device__ inline int reduce_floats(int TX, int TY) { return TX > 32 ? TY * (TX >> 5) * 2 : 0; }
+
 template <int N>
 __device__ __forceinline__ void row_reduce(float (&val)[N], float* scratch, int TX) {
   const int tx = threadIdx.x;
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    float v = val[i];
-    for (int o = min(TX, 32) >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    val[i] = v;
-  }
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < TX) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) val[i] += __shfl_xor_sync(0xffffffffu, val[i], o);
+    }
   if (TX > 32) {
     const int nw = TX >> 5;
     float* s = scratch + threadIdx.y * (nw * N);
@@ -91,12 +95,12 @@ __device__ __forceinline__ void row_reduce(float (&val)[N], float* scratch, int 
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      float v = 0.f;
-      for (int w = 0; w < nw; ++w) v += s[w * N + i];
+    for (int i = 0; i < N; ++i) {  // at most 16 warps
+      float v = (tx & 15) < nw ? s[(tx & 15) * N + i] : 0.f;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
       val[i] = v;
     }
-    __syncthreads();
   }
 }
 
@@ -161,6 +165,65 @@ __global__ void norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_
     }
     store8(y + base + i * 8, o);
   }
+}
+
+// Forward with one 16-byte vector per thread (dim <= 4096): the row, the residual and the weights are all on their way before anything waits,
+// and a row over up to 16 warps costs one barrier.  For few rows, where a warp per row leaves the chip idle and its chain of loads, sums and
+// stores is the whole time (8 to 256 rows of 4096: 9.4 to 11 us there, 2.4 to 2.9 here), and for every dim that the warp form below does not have
+// (8192 x 768: 8.9 us, 15.3 in passes over memory).
+template <bool LN>
+__global__ void __launch_bounds__(kMaxThreads)
+norm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual, const void* __restrict__ w,
+                    const void* __restrict__ b, int wf32, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
+                    float* __restrict__ rstd_out, float* __restrict__ mean_out, int rows, int dim, float eps, float w_offset) {
+  extern __shared__ float scratch[];
+  const int col = threadIdx.x * 8;
+  const int row = blockIdx.x * blockDim.y + threadIdx.y;
+  const bool active = row < rows && col < dim;  // the others take part in the sums
+  const size_t at = static_cast<size_t>(row) * dim + col;
+  Vec8 a{}, ww{}, bb{};
+  if (active) {
+    const uint4 v = *reinterpret_cast<const uint4*>(x + at);
+    uint4 r{};
+    if (residual != nullptr) r = *reinterpret_cast<const uint4*>(residual + at);
+    ww = loadw8(w, wf32, col, w_offset);
+    if (b != nullptr) bb = loadw8(b, wf32, col, 0.f);
+    a = unpack8(v);
+    if (residual != nullptr) {
+      const Vec8 rr = unpack8(r);
+      uint4 h;
+      h.x = pack_bf16x2(a.v[0] + rr.v[0], a.v[1] + rr.v[1]);
+      h.y = pack_bf16x2(a.v[2] + rr.v[2], a.v[3] + rr.v[3]);
+      h.z = pack_bf16x2(a.v[4] + rr.v[4], a.v[5] + rr.v[5]);
+      h.w = pack_bf16x2(a.v[6] + rr.v[6], a.v[7] + rr.v[7]);
+      if (h_out != nullptr) {
+        *reinterpret_cast<uint4*>(h_out + at) = h;
+        a = unpack8(h);  // normalise exactly what later layers will read
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a.v[j] += rr.v[j];
+      }
+    }
+  }
+  float acc[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    acc[0] += a.v[j];
+    acc[1] += a.v[j] * a.v[j];
+  }
+  row_reduce<2>(acc, scratch, blockDim.x);
+  if (!active) return;
+  const float mean = LN ? acc[0] / dim : 0.f;
+  const float var = LN ? fmaxf(acc[1] / dim - mean * mean, 0.f) : acc[1] / dim;
+  const float rstd = rsqrtf(var + eps);
+  if (threadIdx.x == 0) {
+    if (rstd_out != nullptr) rstd_out[row] = rstd;
+    if (LN && mean_out != nullptr) mean_out[row] = mean;
+  }
+  Vec8 o;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) o.v[j] = (a.v[j] - mean) * rstd * ww.v[j] + bb.v[j];
+  store8(y + at, o);
 }
 
 // Forward with one warp per row and the row held in registers (packed bf16: VPL 16-byte vectors per lane): every load of the
@@ -242,139 +305,197 @@ norm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
   }
 }
 
-// Backward.  Each block walks rows blockIdx.x*TY + ty, += gridDim.x*TY and keeps its
-// share of dw (and db) in registers; partials go to dw_part[gridDim.x*TY, dim] and are
-// summed by norm_bwd_reduce_kernel, so the result is deterministic.
+// Backward.  Each block walks rows blockIdx.x * TY + ty, += gridDim.x * TY, with the next rows on their way into a ring of shared memory (every
+// thread copies and reads its own vectors, so the ring needs no barrier), and keeps its share of dw (and db) in registers; a block's shares are
+// added in shared memory and go to part[block][dim], which norm_bwd_reduce_kernel sums in a fixed order.  What bounds it is the instructions
+// per element (444 per vector of eight while weights were read and widened twice a row and offsets made anew; about 250 now), then memory:
+// 8192 x 4096 with a residual's gradient 94 -> 69 us (3.9 TB/s), 8192 x 768 with a mean 26 -> 16, 96000 x 128 28 -> 18.  The sum of the shares was
+// 47 us for 7104 shares of 128 (four blocks, one share per thread row) and is 5.6; for 888 of 768, 14 -> 5.9 for both dw and db.
 //   dx = rstd * (g - mean(g) - xhat * mean(g * xhat))        (LN)
 //   dx = rstd * (g - xhat * mean(g * xhat))                   (RMS)      with g = dy * w
 // If dres_in is given it is added to dx (gradient arriving through the residual stream).
-template <bool LN, int VPT>
-__global__ void norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                                const void* __restrict__ w, int wf32, const float* __restrict__ rstd_in,
-                                const float* __restrict__ mean_in, const __nv_bfloat16* __restrict__ dres_in,
-                                __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part,
-                                float* __restrict__ db_part, int rows, int dim, float w_offset) {
-  extern __shared__ float scratch[];
-  const int TX = blockDim.x;
+template <int VPT>
+__host__ __device__ constexpr int ring_rows() { return VPT == 1 ? 4 : VPT == 2 ? 3 : 2; }
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+template <bool LN, bool DB, int VPT>
+__global__ void __launch_bounds__(kMaxThreads, VPT == 1 ? 2 : 1)
+norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const void* __restrict__ w, int wf32,
+                const float* __restrict__ rstd_in, const float* __restrict__ mean_in, const __nv_bfloat16* __restrict__ dres_in,
+                __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, float* __restrict__ db_part, int rows, int dim, float w_offset) {
+  extern __shared__ __align__(16) float scratch[];
+  constexpr int kRing = ring_rows<VPT>();
+  const int TX = blockDim.x, TY = blockDim.y, threads = TX * TY;
   const int nvec = dim >> 3;
-  float dw_acc[VPT][8];
-  float db_acc[VPT][8];
+  const int half = reduce_floats(TX, TY);
+  float* sum = scratch + (2 * half + 3) / 4 * 4;  // [TY][TX][8] in the end, over the ring
+  uint4* ring = reinterpret_cast<uint4*>(sum) + threadIdx.y * TX + threadIdx.x;  // [kRing][2 or 3][VPT][threads]
+  const int kinds = dres_in != nullptr ? 3 : 2;
+  float dw_acc[VPT][8], db_acc[DB ? VPT : 1][8];
 #pragma unroll
   for (int s = 0; s < VPT; ++s)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { dw_acc[s][j] = 0.f; db_acc[s][j] = 0.f; }
-  const int row_stride = gridDim.x * blockDim.y;
-  const int first = blockIdx.x * blockDim.y + threadIdx.y;
+    for (int j = 0; j < 8; ++j) {
+      dw_acc[s][j] = 0.f;
+      if (DB) db_acc[DB ? s : 0][j] = 0.f;
+    }
+  const int row_stride = gridDim.x * TY;
+  const int first = blockIdx.x * TY + threadIdx.y;
   const int iters = (rows + row_stride - 1) / row_stride;
+  Vec8 ww[VPT];
+#pragma unroll
+  for (int s = 0; s < VPT; ++s)
+    if (threadIdx.x + s * TX < nvec) ww[s] = loadw8(w, wf32, (threadIdx.x + s * TX) * 8, w_offset);
+    else ww[s] = Vec8{};
+  // offsets of this thread's first vector in the row that is fetched and in the row that is worked on
+  const long long step = static_cast<long long>(row_stride) * dim;
+  long long at_in = static_cast<long long>(first) * dim + threadIdx.x * 8, at_out = at_in;
+  int row_in = first, slot_in = 0, slot = 0;
+  const int slot_size = kinds * VPT * threads;
+  auto fetch = [&]() {  // one group of copies per row, empty ones past the end
+    if (row_in < rows) {
+      uint4* dst = ring + slot_in * slot_size;
+#pragma unroll
+      for (int s = 0; s < VPT; ++s)
+        if (threadIdx.x + s * TX < nvec) {
+          cp_async16(dst + s * threads, dy + at_in + s * TX * 8);
+          cp_async16(dst + (VPT + s) * threads, x + at_in + s * TX * 8);
+          if (dres_in != nullptr) cp_async16(dst + (2 * VPT + s) * threads, dres_in + at_in + s * TX * 8);
+        }
+    }
+    row_in += row_stride;
+    at_in += step;
+    slot_in = slot_in + 1 == kRing ? 0 : slot_in + 1;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float rstd = first < rows ? __ldg(rstd_in + first) : 0.f, mean = LN && first < rows ? __ldg(mean_in + first) : 0.f;
+#pragma unroll
+  for (int it = 0; it < kRing - 1; ++it) fetch();
   for (int it = 0; it < iters; ++it) {
     const int row = first + it * row_stride;
+    const float my_rstd = rstd, my_mean = mean;
+    const int next = row + row_stride;
+    rstd = next < rows ? __ldg(rstd_in + next) : 0.f;
+    mean = LN && next < rows ? __ldg(mean_in + next) : 0.f;
+    fetch();  // into the place of the previous row
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory");
+    const uint4* src = ring + slot * slot_size;
+    slot = slot + 1 == kRing ? 0 : slot + 1;
     const bool active = row < rows;
-    const size_t base = static_cast<size_t>(active ? row : 0) * dim;
-    const float rstd = active ? rstd_in[row] : 0.f;
-    const float mean = (LN && active) ? mean_in[row] : 0.f;
+    float gw[VPT][8], xh[VPT][8];
     float acc[2] = {0.f, 0.f};
-    if (active) {
 #pragma unroll
-      for (int s = 0; s < VPT; ++s) {
-        const int i = threadIdx.x + s * TX;
-        if (i < nvec) {
-          Vec8 g = load8(dy + base + i * 8);
-          Vec8 a = load8(x + base + i * 8);
-          Vec8 ww = loadw8(w, wf32, i * 8, w_offset);
+    for (int s = 0; s < VPT; ++s) {
+      if (active && threadIdx.x + s * TX < nvec) {
+        const Vec8 g = unpack8(src[s * threads]), a = unpack8(src[(VPT + s) * threads]);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xh = (a.v[j] - mean) * rstd;
-            const float gw = g.v[j] * ww.v[j];
-            acc[0] += gw;
-            acc[1] += gw * xh;
-            dw_acc[s][j] += g.v[j] * xh;
-            db_acc[s][j] += g.v[j];
-          }
+        for (int j = 0; j < 8; ++j) {
+          xh[s][j] = (LN ? a.v[j] - my_mean : a.v[j]) * my_rstd;
+          gw[s][j] = g.v[j] * ww[s].v[j];
+          if (LN) acc[0] += gw[s][j];
+          acc[1] += gw[s][j] * xh[s][j];
+          dw_acc[s][j] += g.v[j] * xh[s][j];
+          if (DB) db_acc[DB ? s : 0][j] += g.v[j];
         }
       }
     }
-    row_reduce<2>(acc, scratch, TX);
-    const float m1 = LN ? acc[0] / dim : 0.f;
-    const float m2 = acc[1] / dim;
+    if (LN) {
+      row_reduce<2>(acc, scratch + (it & 1) * half, TX);
+    } else {
+      float one[1] = {acc[1]};
+      row_reduce<1>(one, scratch + (it & 1) * half, TX);
+      acc[1] = one[0];
+    }
+    const float m1 = LN ? acc[0] / dim * my_rstd : 0.f;
+    const float m2 = acc[1] / dim * my_rstd;
     if (active) {
 #pragma unroll
       for (int s = 0; s < VPT; ++s) {
-        const int i = threadIdx.x + s * TX;
-        if (i < nvec) {
-          Vec8 g = load8(dy + base + i * 8);
-          Vec8 a = load8(x + base + i * 8);
-          Vec8 ww = loadw8(w, wf32, i * 8, w_offset);
+        if (threadIdx.x + s * TX < nvec) {
           Vec8 o;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float xh = (a.v[j] - mean) * rstd;
-            o.v[j] = rstd * (g.v[j] * ww.v[j] - m1 - xh * m2);
-          }
+          for (int j = 0; j < 8; ++j) o.v[j] = my_rstd * gw[s][j] - (LN ? m1 + xh[s][j] * m2 : xh[s][j] * m2);
           if (dres_in != nullptr) {
-            Vec8 r = load8(dres_in + base + i * 8);
+            const Vec8 r = unpack8(src[(2 * VPT + s) * threads]);
 #pragma unroll
             for (int j = 0; j < 8; ++j) o.v[j] += r.v[j];
           }
-          store8(dx + base + i * 8, o);
+          store8(dx + at_out + s * TX * 8, o);
         }
       }
     }
+    at_out += step;
   }
-  const int prow = blockIdx.x * blockDim.y + threadIdx.y;
 #pragma unroll
-  for (int s = 0; s < VPT; ++s) {
-    const int i = threadIdx.x + s * TX;
-    if (i < nvec) {
-      if (dw_part != nullptr) {
-        float* p = dw_part + static_cast<size_t>(prow) * dim + i * 8;
+  for (int which = 0; which < (DB ? 2 : 1); ++which) {
+    float* part = which == 0 ? dw_part : db_part;
+    if (part == nullptr) continue;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) p[j] = dw_acc[s][j];
+    for (int s = 0; s < VPT; ++s) {
+      float v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = which == 0 ? dw_acc[s][j] : db_acc[DB ? s : 0][j];
+      if (TY > 1) {
+        __syncthreads();
+        float4* mine = reinterpret_cast<float4*>(sum + (threadIdx.y * TX + threadIdx.x) * 8);
+        mine[0] = make_float4(v[0], v[1], v[2], v[3]);
+        mine[1] = make_float4(v[4], v[5], v[6], v[7]);
+        __syncthreads();
+        if (threadIdx.y == 0)
+          for (int t = 1; t < TY; ++t)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] += sum[(t * TX + threadIdx.x) * 8 + j];
       }
-      if (db_part != nullptr) {
-        float* p = db_part + static_cast<size_t>(prow) * dim + i * 8;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) p[j] = db_acc[s][j];
+      const int i = threadIdx.x + s * TX;
+      if (threadIdx.y == 0 && i < nvec) {
+        float4* p = reinterpret_cast<float4*>(part + static_cast<size_t>(blockIdx.x) * dim + i * 8);
+        p[0] = make_float4(v[0], v[1], v[2], v[3]);
+        p[1] = make_float4(v[4], v[5], v[6], v[7]);
       }
     }
   }
 }
 
-// out[c] (+)= sum over the partial rows.  A block owns 32 columns; its 8 thread rows each sum every 8th partial row (four
-// independent accumulators, so the loads overlap) and are then added in a fixed order: deterministic, and a few hundred
-// partial rows cost tens of loads per thread instead of one dependent chain of all of them.
-__global__ void __launch_bounds__(256)
-norm_bwd_reduce_kernel(const float* __restrict__ part, float* __restrict__ out, int nparts, int dim, int accumulate) {
-  __shared__ float sm[8][33];
+// out[c] = sum over the blocks' shares, for dw and (blockIdx.y = 1) db.  A block owns 32 columns; its 32 thread rows each sum every 32nd
+// share, four loads at a time, and are added in a fixed order.
+__global__ void __launch_bounds__(1024)
+norm_bwd_reduce_kernel(const float* __restrict__ part_w, const float* __restrict__ part_b, void* __restrict__ out_w, void* __restrict__ out_b, int out_bf16,
+                       int nparts, int dim) {
+  __shared__ float sm[32][33];
+  const float* part = blockIdx.y == 0 ? part_w : part_b;
+  void* out = blockIdx.y == 0 ? out_w : out_b;
+  if (out == nullptr) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+  float a[4] = {0.f, 0.f, 0.f, 0.f};
   if (c < dim) {
     int r = ty;
-    for (; r + 24 < nparts; r += 32) {
-      a0 += part[static_cast<size_t>(r) * dim + c];
-      a1 += part[static_cast<size_t>(r + 8) * dim + c];
-      a2 += part[static_cast<size_t>(r + 16) * dim + c];
-      a3 += part[static_cast<size_t>(r + 24) * dim + c];
-    }
-    for (; r < nparts; r += 8) a0 += part[static_cast<size_t>(r) * dim + c];
-  }
-  sm[ty][tx] = (a0 + a1) + (a2 + a3);
-  __syncthreads();
-  if (ty == 0 && c < dim) {
-    float s = 0.f;
+    for (; r + 96 < nparts; r += 128)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += sm[j][tx];
-    out[c] = accumulate ? out[c] + s : s;
+      for (int j = 0; j < 4; ++j) a[j] += part[static_cast<size_t>(r + 32 * j) * dim + c];
+    for (; r < nparts; r += 32) a[0] += part[static_cast<size_t>(r) * dim + c];
+  }
+  sm[ty][tx] = (a[0] + a[1]) + (a[2] + a[3]);
+  __syncthreads();
+  const float v = warp_sum(sm[tx][ty]);  // warp ty: the column ty of this block
+  const int col = blockIdx.x * 32 + ty;
+  if (tx == 0 && col < dim) {
+    if (out_bf16) reinterpret_cast<__nv_bfloat16*>(out)[col] = __float2bfloat16(v);
+    else reinterpret_cast<float*>(out)[col] = v;
   }
 }
 
+// TX threads per row: one vector each where 512 threads allow it, whole warps (or a power of two below one); TY rows per block of about 256
 inline void pick_block(int dim, int& TX, int& TY) {
   const int nvec = dim >> 3;
   TX = 8;
-  while (TX < nvec && TX < 256) TX <<= 1;  // one vector per thread when possible
-  if (nvec >= 512) TX = 256;
-  TY = 256 / TX;
-  if (TY < 1) TY = 1;
+  while (TX < nvec && TX < 32) TX <<= 1;
+  if (nvec > 32) TX = (nvec + 31) / 32 * 32;
+  if (TX > kMaxThreads) TX = kMaxThreads;
+  TY = TX >= 256 ? 1 : 256 / TX;
 }
 
 }  // namespace norm
@@ -392,7 +513,7 @@ extern "C" int lvb_norm_fwd(const void* x, const void* residual, const void* w, 
   pick_block(dim, TX, TY);
   dim3 block(TX, TY);
   dim3 grid((rows + TY - 1) / TY);
-  size_t smem = sizeof(float) * TY * (TX > 32 ? (TX / 32) * 2 : 0);
+  size_t smem = sizeof(float) * 2 * reduce_floats(TX, TY);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   auto X = reinterpret_cast<const __nv_bfloat16*>(x);
   auto R = reinterpret_cast<const __nv_bfloat16*>(residual);
@@ -400,7 +521,15 @@ extern "C" int lvb_norm_fwd(const void* x, const void* residual, const void* w, 
   auto H = reinterpret_cast<__nv_bfloat16*>(h_out);
   {
     const int vpl = dim / 256;
-    if (dim % 256 == 0 && (vpl == 1 || vpl == 2 || vpl == 4 || vpl == 8 || vpl == 16)) {
+    const bool by_warp = dim % 256 == 0 && (vpl == 1 || vpl == 2 || vpl == 4 || vpl == 8 || vpl == 16);
+    if ((dim >> 3) <= TX && (!by_warp || rows <= kFewRows)) {
+      if (layer_norm)
+        norm_fwd_row_kernel<true><<<grid, block, smem, s>>>(X, R, w, b, w_is_f32, Y, H, rstd_out, mean_out, rows, dim, eps, w_offset);
+      else
+        norm_fwd_row_kernel<false><<<grid, block, smem, s>>>(X, R, w, b, w_is_f32, Y, H, rstd_out, mean_out, rows, dim, eps, w_offset);
+      return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+    }
+    if (by_warp) {
       const dim3 wgrid((rows + 3) / 4);
 #define LVB_NORM_WARP(LNV, V)                                                                                                  \
   if (R != nullptr)                                                                                                            \
@@ -428,22 +557,28 @@ extern "C" int lvb_norm_fwd(const void* x, const void* residual, const void* w, 
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }
 
-// Backward of lvb_norm_fwd.  x is the normalised input (x + residual if a residual was added).
-// scratch: fp32 [2 * nparts * dim] where nparts = lvb_norm_bwd_parts(rows, dim); dw/db are fp32 [dim]
-// (either may be null).  accumulate != 0 adds into dw/db.
+namespace lvb {
+namespace norm {
+inline int vpt_room(int vpt) { return vpt <= 1 ? 1 : vpt <= 2 ? 2 : 4; }
+}  // namespace norm
+}  // namespace lvb
+
+// Backward of lvb_norm_fwd.  x is the normalised input (x + residual if a residual was added).  scratch: fp32 [2 * nparts * dim], 16-byte
+// aligned, where nparts = lvb_norm_bwd_parts(rows, dim); dw / db are [dim], bf16 with out_bf16 and fp32 otherwise (either may be null).
 extern "C" int lvb_norm_bwd_parts(int rows, int dim) {
   using namespace lvb::norm;
   int TX, TY;
   pick_block(dim, TX, TY);
-  int blocks = (rows + TY - 1) / TY;
-  int cap = lvb::num_sms() * 3;  // three CTAs of 256 threads fit an SM at this kernel's register count; two left its warps 25 % active
-  if (blocks > cap) blocks = cap;
-  return blocks * TY;
+  // as many blocks as an SM's registers hold (64 per thread; one block of wide rows), and two rows per thread row, so that few rows do not make
+  // as many shares
+  const int blocks = (rows + 2 * TY - 1) / (2 * TY);
+  const int cap = lvb::num_sms() * ((dim >> 3) > kMaxThreads ? 1 : 1024 / (TX * TY));
+  return blocks < cap ? blocks : cap;
 }
 
 extern "C" int lvb_norm_bwd(const void* dy, const void* x, const void* w, int w_is_f32, const float* rstd,
-                            const float* mean, const void* dres_in, void* dx, float* dw, float* db, float* scratch,
-                            int rows, int dim, float w_offset, int layer_norm, int accumulate, void* stream) {
+                            const float* mean, const void* dres_in, void* dx, void* dw, void* db, int out_bf16, float* scratch,
+                            int rows, int dim, float w_offset, int layer_norm, void* stream) {
   using namespace lvb;
   using namespace lvb::norm;
   if (rows <= 0 || dim <= 0 || (dim & 7)) return kErrBadArg;
@@ -452,8 +587,7 @@ extern "C" int lvb_norm_bwd(const void* dy, const void* x, const void* w, int w_
   if ((dim >> 3) > TX * kMaxVecPerThread) return kErrTooLarge;
   const int nparts = lvb_norm_bwd_parts(rows, dim);
   dim3 block(TX, TY);
-  dim3 grid(nparts / TY);
-  size_t smem = sizeof(float) * TY * (TX > 32 ? (TX / 32) * 2 : 0);
+  const int base = sizeof(float) * ((2 * reduce_floats(TX, TY) + 3) / 4 * 4);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   float* dw_part = dw != nullptr ? scratch : nullptr;
   float* db_part = db != nullptr ? scratch + static_cast<size_t>(nparts) * dim : nullptr;
@@ -462,17 +596,21 @@ extern "C" int lvb_norm_bwd(const void* dy, const void* x, const void* w, int w_
   auto DR = reinterpret_cast<const __nv_bfloat16*>(dres_in);
   auto DX = reinterpret_cast<__nv_bfloat16*>(dx);
   const int vpt = ((dim >> 3) + TX - 1) / TX;
-#define LVB_NORM_BWD(LN, V) \
-  norm_bwd_kernel<LN, V><<<grid, block, smem, s>>>(DY, X, w, w_is_f32, rstd, mean, DR, DX, dw_part, db_part, rows, dim, w_offset)
-  if (layer_norm) {
-    if (vpt <= 1) LVB_NORM_BWD(true, 1); else if (vpt <= 2) LVB_NORM_BWD(true, 2);
-    else if (vpt <= 4) LVB_NORM_BWD(true, 4); else LVB_NORM_BWD(true, 8);
-  } else {
-    if (vpt <= 1) LVB_NORM_BWD(false, 1); else if (vpt <= 2) LVB_NORM_BWD(false, 2);
-    else if (vpt <= 4) LVB_NORM_BWD(false, 4); else LVB_NORM_BWD(false, 8);
-  }
+  auto go = [&](auto kern, int ring) {
+    const int smem = base + ring * (dres_in != nullptr ? 3 : 2) * vpt_room(vpt) * TX * TY * 16;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kErrCuda;
+    kern<<<nparts, block, smem, s>>>(DY, X, w, w_is_f32, rstd, mean, DR, DX, dw_part, db_part, rows, dim, w_offset);
+    return kErrOk;
+  };
+  int rc;
+#define LVB_NORM_BWD(LN, DB)                                                      \
+  if (vpt <= 1) rc = go(norm_bwd_kernel<LN, DB, 1>, ring_rows<1>());              \
+  else if (vpt <= 2) rc = go(norm_bwd_kernel<LN, DB, 2>, ring_rows<2>());         \
+  else rc = go(norm_bwd_kernel<LN, DB, 4>, ring_rows<4>())
+  if (layer_norm) { LVB_NORM_BWD(true, true); } else if (db != nullptr) { LVB_NORM_BWD(false, true); } else { LVB_NORM_BWD(false, false); }
 #undef LVB_NORM_BWD
-  if (dw != nullptr) norm_bwd_reduce_kernel<<<(dim + 31) / 32, 256, 0, s>>>(dw_part, dw, nparts, dim, accumulate);
-  if (db != nullptr) norm_bwd_reduce_kernel<<<(dim + 31) / 32, 256, 0, s>>>(db_part, db, nparts, dim, accumulate);
+  if (rc != kErrOk) return rc;
+  if (dw != nullptr || db != nullptr)
+    norm_bwd_reduce_kernel<<<dim3((dim + 31) / 32, db != nullptr ? 2 : 1), 1024, 0, s>>>(dw_part, db_part, dw, db, out_bf16, nparts, dim);
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }

@@ -26,7 +26,7 @@ def _fwd():
 
 def _bwd():
     c = lib
-    return _fn("lvb_norm_bwd", [c.c_void_p] * 3 + [c.c_int] + [c.c_void_p] * 7 + [c.c_int, c.c_int, c.c_float, c.c_int, c.c_int, c.c_void_p])
+    return _fn("lvb_norm_bwd", [c.c_void_p] * 3 + [c.c_int] + [c.c_void_p] * 6 + [c.c_int, c.c_void_p, c.c_int, c.c_int, c.c_float, c.c_int, c.c_void_p])
 
 
 def _parts():
@@ -115,17 +115,14 @@ class _NormFn(torch.autograd.Function):
         need_db = ctx.has_bias and ctx.needs_input_grad[3]
         nparts = _parts()(rows, dim)
         scratch = torch.empty(2 * nparts * dim, dtype=torch.float32, device=xin.device) if (need_dw or need_db) else None
-        dw = torch.empty(dim, dtype=torch.float32, device=xin.device) if need_dw else None
-        db = torch.empty(dim, dtype=torch.float32, device=xin.device) if need_db else None
+        out = torch.float32 if weight is None else weight.dtype
+        dw = torch.empty(dim, dtype=out, device=xin.device) if need_dw else None
+        db = torch.empty(dim, dtype=out, device=xin.device) if need_db else None
         rc = _bwd()(dy2.data_ptr(), xin.data_ptr(), lib.ptr(weight), ctx.wf32, rstd.data_ptr(), lib.ptr(mean), lib.ptr(dres),
-                    dx.data_ptr(), lib.ptr(dw), lib.ptr(db), lib.ptr(scratch), rows, dim, float(ctx.w_offset),
-                    int(ctx.layer_norm), 0, lib.stream_ptr())
+                    dx.data_ptr(), lib.ptr(dw), lib.ptr(db), int(out == torch.bfloat16), lib.ptr(scratch), rows, dim, float(ctx.w_offset),
+                    int(ctx.layer_norm), lib.stream_ptr())
         lib.check_rc(rc, "lvb_norm_bwd")
         dxv = dx.view(ctx.shape)
-        if dw is not None and weight.dtype != torch.float32:
-            dw = dw.to(weight.dtype)
-        if db is not None and weight is not None and weight.dtype != torch.float32:
-            db = db.to(weight.dtype)
         return dxv, (dxv if ctx.has_res else None), dw, db, None, None, None
 
 

@@ -154,3 +154,27 @@ def test_adamw_and_sumsq():
     _close(p, pr, 1e-5)
     _close(pb, pr, 1e-2)
     _close(m, mr, 1e-5)
+
+
+@pytest.mark.parametrize("rows,dim", [(1, 4096), (8, 2048), (1024, 512), (1025, 512), (999, 768), (5, 776), (3, 8), (40000, 128), (2, 12288), (700, 2056)])
+@pytest.mark.parametrize("ln,residual,wdtype", [(True, False, torch.bfloat16), (False, True, torch.float32), (False, False, torch.bfloat16), (True, True, torch.float32)])
+def test_norm_block_shapes(rows, dim, ln, residual, wdtype):
+    """Widths around a warp, a block and several vectors per thread; few rows and many; a bias with and without a mean.  Sums in fp32 over bf16
+    inputs: the results' bf16 rounding is 2^-9, and a bf16 weight's gradient is rounded once."""
+    torch.manual_seed(rows + dim)
+    x = torch.randn(rows, dim, device="cuda").bfloat16().requires_grad_()
+    r = torch.randn(rows, dim, device="cuda").bfloat16().requires_grad_() if residual else None
+    w = (1 + 0.1 * torch.randn(dim, device="cuda")).to(wdtype).requires_grad_()
+    b = (0.1 * torch.randn(dim, device="cuda")).to(wdtype).requires_grad_()
+    y, h = norm.fused_norm(x, w, b, 1e-5, layer_norm=ln, residual=r)
+    gy, gh = torch.randn_like(y), torch.randn_like(y)
+    torch.autograd.backward([y] + ([h] if residual else []), [gy] + ([gh] if residual else []))
+    x64 = (h if residual else x).detach().double().requires_grad_()
+    w64, b64 = (t.detach().double().requires_grad_() for t in (w, b))
+    c = x64 - x64.mean(-1, keepdim=True) if ln else x64
+    y64 = c * torch.rsqrt(c.pow(2).mean(-1, keepdim=True) + 1e-5) * w64 + b64
+    torch.autograd.backward([y64] + ([x64 * 1] if residual else []), [gy.double()] + ([gh.double()] if residual else []))
+    for got, want in ((y, y64), (x.grad, x64.grad), (w.grad, w64.grad), (b.grad, b64.grad)):
+        assert (got.double() - want).norm() <= 2 ** -8 * want.norm() + 1e-6
+    if residual:
+        assert torch.equal(r.grad, x.grad)
