@@ -8,7 +8,7 @@
 // rows of a kv head are adjacent 2*D-element runs.
 //
 // paged_attention is bandwidth bound (every step re-reads the context once), so the work is cut for parallelism, not for
-// tensor cores: one CTA per (query token, kv head, partition of 256 keys).  A CTA scores its keys against the G query heads
+// tensor cores: one CTA per (query token, kv head, partition of 64 to 1024 keys).  A CTA scores its keys against the G query heads
 // that share the kv head (one key per thread, 16-byte loads), soft-maxes within the partition in shared memory,
 // accumulates P.V with eight output dimensions per thread, and writes an un-normalised partial (o, max, sum).  A second small
 // kernel merges the partitions of each (token, head).  Nothing here synchronises with the host: sequence boundaries,
@@ -20,7 +20,8 @@
 namespace lvb {
 namespace paged {
 
-constexpr int kPart = 256;     // keys per partition
+constexpr int kPart = 256;     // keys per partition of the scalar kernels; the tensor-core kernel's come from part_keys
+constexpr int kMaxParts = 256;
 constexpr int kThreads = 128;  // 4 warps
 constexpr int kMaxG = 16;      // query heads per kv head
 
@@ -75,6 +76,8 @@ struct Params {
   float* part_o;                  // [T, H, parts, D]
   float* part_ml;                 // [T, H, parts, 2]
   int T, H, KV, S, pages_per_seq, page_size, num_pages, parts;
+  int part;                       // keys per partition
+  bool by_mma;                    // by the tensor-core kernel, which writes the result where one partition holds all of a token's keys
   float scale, soft_cap;
   // ---- general form (lvb_paged_attention_general); the plain entry point sets dk = dv = D, chunk = 0, no gate
   int dk, dv;                 // query/key and value sizes; a cache slot holds, per KV head, dk key and dv value elements
@@ -89,6 +92,7 @@ struct Params {
   int maps;
   const float* weight;
   float diff_scale, eps;
+  int* status;
 };
 
 // First visible key of a query whose context (its position + 1) is ctx.
@@ -118,6 +122,28 @@ __device__ __forceinline__ bool locate(const Params& p, int t, int& seq, int& ct
   const int kl = p.kv_lens[seq];
   if (kl <= 0 || kl > p.pages_per_seq * p.page_size) return false;
   ctx = kl - (q1 - q0) + (t - q0) + 1;  // absolute position of the token + 1
+  return ctx > 0;
+}
+
+// The same by a whole block of kThreadsB threads: one round of independent loads instead of a search whose every step waits for the last one (some
+// ten memory latencies, longer than a partition of 256 keys takes to stream).
+template <int kThreadsB>
+__device__ __forceinline__ bool locate_block(const Params& p, int t, int& seq, int& ctx) {
+  __shared__ int s_before[kThreadsB / 32];
+  const int n = min(p.num_seqs[0], p.S);
+  int before = 0;  // sequences that end at or before the token
+  for (int i = threadIdx.x; i < p.S; i += kThreadsB) before += i < n && p.cu_q_lens[i + 1] <= t;
+  before = __reduce_add_sync(0xffffffffu, before);
+  if ((threadIdx.x & 31) == 0) s_before[threadIdx.x >> 5] = before;
+  __syncthreads();
+  seq = 0;
+#pragma unroll
+  for (int w = 0; w < kThreadsB / 32; ++w) seq += s_before[w];
+  if (seq >= n) return false;
+  const int q0 = p.cu_q_lens[seq], q1 = p.cu_q_lens[seq + 1];
+  const int kl = p.kv_lens[seq];
+  if (kl <= 0 || kl > p.pages_per_seq * p.page_size) return false;
+  ctx = kl - (q1 - q0) + (t - q0) + 1;
   return ctx > 0;
 }
 
@@ -467,19 +493,22 @@ __global__ void __launch_bounds__(kThreads) paged_attention_staged_kernel(Params
 // and the loops stop at the next multiple of 16.  The query heads that share a KV head are the M rows
 // of warp-level MMAs (m16n8k16, bf16, fp32 accumulation; rows beyond G are zero), so one pass over a key's K and V rows
 // serves all of them at a sixteenth of the instruction count of the scalar kernels, which were bound by instruction issue
-// and shared-memory reads, not by the cache traffic.  Each of the four warps owns 64 keys of the partition and is its own
+// and shared-memory reads, not by the cache traffic.  Each of the four warps owns a quarter of the partition's keys and is its own
 // pipeline: it copies stages of 16 keys (K and V rows are adjacent in the cache: 512 bytes per key, padded to 528 in
-// shared memory so that ldmatrix reads are conflict-free) with cp.async, double-buffered, and needs no CTA-wide barrier
+// shared memory so that ldmatrix reads are conflict-free) with one bulk copy per key (kExact; cp.async otherwise), double-buffered, and needs no CTA-wide barrier
 // inside the loop.  Scores S = Q K^T come from ldmatrix'd K rows, the online softmax runs on the accumulator fragments,
 // P is re-packed in registers as the A operand of O += P V (V rows through ldmatrix.trans), and the four warps' (max, sum,
-// O) are merged through shared memory at the end.
+// O) are merged through shared memory at the end.  kSplitP: the probabilities enter O += P V as two bf16 parts, for a size whose scalar kernel
+// kept them in fp32 (heads of 64: 24 us there for one sequence of 300 tokens, 5.5 here).
 constexpr int kMmaStageKeys = 16;
-constexpr int kMmaWarpKeys = kPart / (kThreads / 32);  // 64
+constexpr int kMmaBufs = 2;  // stages of a warp.  Three leave room for two CTAs on an SM instead of three: 20 to 30 % slower, the warps are needed
 // A staged row: K, V (each rounded up to 16 columns) and 16 bytes of padding, which makes the stride an odd multiple of 16 bytes, so
 // that the eight rows of an ldmatrix fall into different banks.
 __host__ __device__ constexpr int mma_row_bytes(int dk16, int dv16) { return (dk16 + dv16) * 2 + 16; }
 // The stage memory is reused for the warps' outputs, [4 warps][16 rows][dv16] fp32, which is never larger.
-constexpr int mma_smem(int dk16, int dv16) { return 4 * 2 * kMmaStageKeys * mma_row_bytes(dk16, dv16) + kPart * 4 + 4 * 16 * 2 * 4; }
+constexpr int mma_smem(int dk16, int dv16, int part) {
+  return 4 * kMmaBufs * kMmaStageKeys * mma_row_bytes(dk16, dv16) + part * 4 + 4 * 16 * 2 * 4 + 4 * kMmaBufs * 8 + 16;
+}
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
@@ -493,7 +522,7 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-template <int DKC, int DVC, bool kExact>
+template <int DKC, int DVC, bool kExact, bool kSplitP = false>
 __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p) {
   const int dk = kExact ? DKC : p.dk, dv = kExact ? DVC : p.dv;
   const int dk16 = (dk + 15) & ~15, dv16 = (dv + 15) & ~15;
@@ -502,13 +531,15 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
   const int G = p.H / p.KV;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   extern __shared__ __align__(16) uint8_t s_dyn[];
-  uint8_t* s_stage = s_dyn;                                   // [4 warps][2 stages][16 keys][row]; reused for the merge
-  int* s_rows = reinterpret_cast<int*>(s_dyn + 4 * 2 * kMmaStageBytes);  // [kPart]
-  float* s_ml = reinterpret_cast<float*>(s_rows + kPart);     // [4 warps][16 rows][2]
+  uint8_t* s_stage = s_dyn;                                   // [4 warps][kMmaBufs][16 keys][row]; reused for the merge
+  int* s_rows = reinterpret_cast<int*>(s_dyn + 4 * kMmaBufs * kMmaStageBytes);  // [p.part]
+  float* s_ml = reinterpret_cast<float*>(s_rows + p.part);    // [4 warps][16 rows][2]
+  uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_ml + 4 * 16 * 2);  // kExact: [4 warps][kMmaBufs], a stage's copies have landed
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(s_bar + 4 * kMmaBufs);
 
   int seq = 0, ctx = 0;
-  const bool live = locate(p, t, seq, ctx);
-  const int k0 = (live ? first_key(p, ctx) : 0) + part * kPart;
+  const bool live = locate_block<kThreads>(p, t, seq, ctx);
+  const int k0 = (live ? first_key(p, ctx) : 0) + part * p.part;
   if (!live || k0 >= ctx) {
     if (part == 0 && !live) {
       const int per = G / p.maps;
@@ -517,8 +548,9 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
     }
     return;
   }
-  const int nk = min(kPart, ctx - k0);
-  for (int i = threadIdx.x; i < kPart; i += kThreads) {
+  const int nk = min(p.part, ctx - k0);
+  const bool whole = ctx - first_key(p, ctx) <= p.part;  // the only partition of this token: nothing to merge
+  for (int i = threadIdx.x; i < p.part; i += kThreads) {
     int slot = -1;
     if (i < nk) {
       const int key = k0 + i;
@@ -526,6 +558,11 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       slot = (page >= 0 && page < p.num_pages) ? page * p.page_size + key % p.page_size : -1;
     }
     s_rows[i] = slot;
+  }
+  if (kExact && threadIdx.x == 0) {
+    *abort_flag = 0;
+    for (int i = 0; i < 4 * kMmaBufs; ++i) mbar_init(&s_bar[i], 1);
+    mbar_fence_init();
   }
   __syncthreads();
 
@@ -550,33 +587,40 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
   }
 
   const long long tok_stride = static_cast<long long>(p.KV) * (dk + dv);
-  const int wk0 = warp * kMmaWarpKeys;                       // this warp's first key inside the partition
-  const int wnk = max(0, min(kMmaWarpKeys, nk - wk0));       // and how many of its 64 are real
+  const int warp_keys = (nk + 63) / 64 * 16;                 // a quarter of the keys, in whole stages
+  const int wk0 = warp * warp_keys;                          // this warp's first key inside the partition
+  const int wnk = max(0, min(warp_keys, nk - wk0));          // and how many it has
   const int stages = (wnk + kMmaStageKeys - 1) / kMmaStageKeys;
-  uint8_t* my_stage = s_stage + warp * (2 * kMmaStageBytes);
+  uint8_t* my_stage = s_stage + warp * (kMmaBufs * kMmaStageBytes);
   // one stage: 16 rows of 16-byte pieces; rows without a key are zero-filled (0 * NaN would poison O), and so are the columns
   // between a size and the next multiple of 16
   const int per_row = (dk16 + dv16) / 8;
   const int lane_row = lane / per_row, lane_piece = lane % per_row, step_row = 32 / per_row, step_piece = 32 % per_row;
   auto issue = [&](int st) {
-    uint8_t* dst = my_stage + (st & 1) * kMmaStageBytes;
-    int r = lane_row, ch = lane_piece;  // row and piece of the lane's next copy
-#pragma unroll 4
-    for (int c = lane; c < kMmaStageKeys * per_row; c += 32) {
-      if constexpr (kExact) {
-        r = c / ((DKC + DVC) / 8);
-        ch = c % ((DKC + DVC) / 8);
-      } else {
-        if (ch >= per_row) { ch -= per_row; ++r; }
+    uint8_t* dst = my_stage + (st % kMmaBufs) * kMmaStageBytes;
+    if constexpr (kExact) {  // a lane per key: its K and V lie side by side
+      constexpr int kKeyBytes = (DKC + DVC) * 2;
+      uint64_t* bar = s_bar + warp * kMmaBufs + st % kMmaBufs;
+      const int i = st * kMmaStageKeys + lane;
+      const int slot = lane < kMmaStageKeys && i < wnk ? s_rows[wk0 + i] : -1;
+      const uint32_t have = __ballot_sync(0xffffffffu, slot >= 0);
+      if (lane == 0) mbar_expect_tx(bar, __popc(have) * kKeyBytes);
+      __syncwarp();
+      if (slot >= 0) {
+        bulk_load(dst + lane * kMmaRowBytes, p.kv_pages + slot * tok_stride + static_cast<long long>(kvh) * (dk + dv), kKeyBytes, bar);
+      } else if (lane < kMmaStageKeys) {
+        for (int c = 0; c < kKeyBytes; c += 16) *reinterpret_cast<uint4*>(dst + lane * kMmaRowBytes + c) = make_uint4(0u, 0u, 0u, 0u);
+        fence_proxy_async_smem();  // a later copy may write here
       }
-      const int i = wk0 + st * kMmaStageKeys + r;
-      const int slot = (st * kMmaStageKeys + r < wnk) ? s_rows[i] : -1;
-      uint8_t* d = dst + r * kMmaRowBytes + ch * 16;
-      const __nv_bfloat16* src = p.kv_pages + slot * tok_stride + static_cast<long long>(kvh) * (dk + dv);
-      if constexpr (kExact) {
-        if (slot >= 0) cp_async_16(d, src + ch * 8);
-        else *reinterpret_cast<uint4*>(d) = make_uint4(0u, 0u, 0u, 0u);
-      } else {
+    } else {
+      int r = lane_row, ch = lane_piece;  // row and piece of the lane's next copy
+#pragma unroll 4
+      for (int c = lane; c < kMmaStageKeys * per_row; c += 32) {
+        if (ch >= per_row) { ch -= per_row; ++r; }
+        const int i = wk0 + st * kMmaStageKeys + r;
+        const int slot = (st * kMmaStageKeys + r < wnk) ? s_rows[i] : -1;
+        uint8_t* d = dst + r * kMmaRowBytes + ch * 16;
+        const __nv_bfloat16* src = p.kv_pages + slot * tok_stride + static_cast<long long>(kvh) * (dk + dv);
         const bool is_k = ch * 8 < dk16;
         const int col = is_k ? ch * 8 : ch * 8 - dk16;  // column of the key or value row
         if (slot >= 0 && col < (is_k ? dk : dv)) cp_async_16(d, src + (is_k ? col : dk + col));
@@ -584,8 +628,8 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
         r += step_row;
         ch += step_piece;
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
   float o[DVC / 8][4];
@@ -594,13 +638,29 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
   float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;  // running max / sum of rows row_lo and row_hi
   const float sc_log2 = p.scale * 1.4426950408889634f;
 
-  if (stages > 0) issue(0);
+  auto issue_or_skip = [&](int st) {  // cp.async: one group of copies per stage, empty ones past the end
+    if (st < stages) issue(st);
+    else if (!kExact) asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto landed = [&](int st) {
+    if constexpr (kExact) {
+      const bool ok = mbar_wait(s_bar + warp * kMmaBufs + st % kMmaBufs, (st / kMmaBufs) & 1, abort_flag, p.status, 1700, st);
+      return __all_sync(0xffffffffu, ok) != 0;
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kMmaBufs - 1) : "memory");
+      return true;
+    }
+  };
+#pragma unroll
+  for (int st = 0; st < kMmaBufs - 1; ++st) issue_or_skip(st);
   for (int st = 0; st < stages; ++st) {
-    if (st + 1 < stages) issue(st + 1);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    issue_or_skip(st + kMmaBufs - 1);
+    if (!landed(st)) {  // recorded in the status word; the copies under way get another limited wait before the memory goes
+      for (int i = st; i < min(stages, st + kMmaBufs); ++i) mbar_wait_quiet(s_bar + warp * kMmaBufs + i % kMmaBufs, (i / kMmaBufs) & 1);
+      break;
+    }
     __syncwarp();
-    const uint32_t buf = smem_u32(my_stage + (st & 1) * kMmaStageBytes);
+    const uint32_t buf = smem_u32(my_stage + (st % kMmaBufs) * kMmaStageBytes);
     // ---- S[16 heads, 16 keys] = Q K^T: two n-tiles of 8 keys
     float sacc[2][4];
 #pragma unroll
@@ -640,7 +700,7 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
     const float a_lo = (m_lo == -INFINITY) ? 0.f : exp2f(m_lo - mn_lo);
     const float a_hi = (m_hi == -INFINITY) ? 0.f : exp2f(m_hi - mn_hi);
     float sum_lo = 0.f, sum_hi = 0.f;
-    uint32_t pa[4];
+    uint32_t pa[4], pl[4];
     {
       float pv[2][4];
 #pragma unroll
@@ -656,6 +716,13 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       pa[1] = pack_bf16x2(pv[0][2], pv[0][3]);  // (row_hi, keys 0-7 tile)
       pa[2] = pack_bf16x2(pv[1][0], pv[1][1]);  // (row_lo, keys 8-15 tile)
       pa[3] = pack_bf16x2(pv[1][2], pv[1][3]);  // (row_hi, keys 8-15 tile)
+      if constexpr (kSplitP) {  // what the rounding lost
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pa[i]));
+          pl[i] = pack_bf16x2(pv[i >> 1][2 * (i & 1)] - hi.x, pv[i >> 1][2 * (i & 1) + 1] - hi.y);
+        }
+      }
     }
     sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 1);
     sum_lo += __shfl_xor_sync(0xffffffffu, sum_lo, 2);
@@ -680,10 +747,14 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       ob[0] *= a_lo; ob[1] *= a_lo; ob[2] *= a_hi; ob[3] *= a_hi;
       mma_16816(o[2 * np], pa, b0, b1);
       mma_16816(o[2 * np + 1], pa, b2, b3);
+      if constexpr (kSplitP) {
+        mma_16816(o[2 * np], pl, b0, b1);
+        mma_16816(o[2 * np + 1], pl, b2, b3);
+      }
     }
-    __syncwarp();  // every lane is done with this buffer before the copy of stage st + 2 overwrites it
+    __syncwarp();  // every lane is done with this buffer before the copy of stage st + kMmaBufs overwrites it
   }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (!kExact) asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();  // all warps are out of their pipelines: the stage memory becomes the merge buffer
 
   // ---- merge the four warps: per row the global max, then the rescaled sums and outputs
@@ -702,7 +773,7 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
     *reinterpret_cast<float2*>(s_o + (warp * 16 + row_hi) * dv16 + d0) = make_float2(o[n][2], o[n][3]);
   }
   __syncthreads();
-  if (p.maps == 2 && p.parts == 1) {  // a warp per head: both maps of a head, their difference and its norm
+  if (p.maps == 2 && whole) {  // a warp per head: both maps of a head, their difference and its norm
     for (int j = warp; j < G / 2; j += 4) {
       float f[2][4];  // what a warp's sum of a map is multiplied by
 #pragma unroll
@@ -755,7 +826,7 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       l = fmaf(s_ml[(w * 16 + g) * 2 + 1], f, l);
     }
     const long long hrow = static_cast<long long>(t) * p.H + kvh * G + g;
-    if (p.parts == 1) {
+    if (whole) {
       p.out[hrow * dv + d] = __float2bfloat16(l > 0.f ? acc / l * gate_factor(p, t, kvh * G + g, d) : 0.f);
     } else {
       p.part_o[(hrow * p.parts + part) * dv + d] = acc;
@@ -768,29 +839,49 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
   }
 }
 
-// One CTA per (token, head): merge the partials of the partitions that were live for this token.
+// One CTA per (token, head): merge the partials of the partitions that were live for this token.  A thread per partition makes its weight, then
+// every thread sums its output dimensions over them.
 // kThreadsM: threads per CTA, a stride over the p.dv output dimensions.
 template <int kThreadsM>
 __global__ void __launch_bounds__(kThreadsM) paged_merge_kernel(Params p) {
+  __shared__ float s_w[kMaxParts], s_red[kThreadsM / 32];
   const int D = p.dv;
   const int t = blockIdx.x, h = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int seq = 0, ctx = 0;
-  if (!locate(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
-  const int np = (ctx - first_key(p, ctx) + kPart - 1) / kPart;
+  if (!locate_block<kThreadsM>(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
+  const int np = (ctx - first_key(p, ctx) + p.part - 1) / p.part;
+  if (np == 1 && p.by_mma) return;  // written by the attention kernel
   const long long hrow = static_cast<long long>(t) * p.H + h;
-  float m = -INFINITY;
-  for (int i = 0; i < np; ++i) m = fmaxf(m, p.part_ml[(hrow * p.parts + i) * 2]);
-  float l = 0.f;
-  for (int i = 0; i < np; ++i) {
-    const float mi = p.part_ml[(hrow * p.parts + i) * 2];
-    l += (mi == -INFINITY) ? 0.f : p.part_ml[(hrow * p.parts + i) * 2 + 1] * __expf(mi - m);
+  const float2* ml = reinterpret_cast<const float2*>(p.part_ml) + hrow * p.parts;
+  float m = -INFINITY, l = 0.f;
+  for (int i = threadIdx.x; i < np; i += kThreadsM) m = fmaxf(m, ml[i].x);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane == 0) s_red[warp] = m;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < kThreadsM / 32; ++w) m = fmaxf(m, s_red[w]);
+  for (int i = threadIdx.x; i < np; i += kThreadsM) {
+    const float2 x = ml[i];
+    const float w = x.x == -INFINITY ? 0.f : __expf(x.x - m);
+    s_w[i] = w;
+    l = fmaf(x.y, w, l);
   }
+  l = warp_sum(l);
+  __syncthreads();  // the maxima have been read, the weights are there
+  if (lane == 0) s_red[warp] = l;
+  __syncthreads();
+  l = 0.f;
+#pragma unroll
+  for (int w = 0; w < kThreadsM / 32; ++w) l += s_red[w];
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    const float* src = p.part_o + hrow * p.parts * D + d;
     float o = 0.f;
+#pragma unroll 4
     for (int i = 0; i < np; ++i) {
-      const float mi = p.part_ml[(hrow * p.parts + i) * 2];
-      if (mi == -INFINITY) continue;
-      o = fmaf(p.part_o[(hrow * p.parts + i) * D + d], __expf(mi - m), o);
+      const float w = s_w[i], x = src[static_cast<long long>(i) * D];
+      o = w > 0.f ? fmaf(x, w, o) : o;
     }
     p.out[hrow * D + d] = __float2bfloat16(l > 0.f ? o / l * gate_factor(p, t, h, d) : 0.f);
   }
@@ -803,8 +894,9 @@ __global__ void __launch_bounds__(kThreadsM) paged_merge_maps_kernel(Params p) {
   __shared__ float s_red[kThreadsM / 32];
   const int t = blockIdx.x, h = blockIdx.y;
   int seq = 0, ctx = 0;
-  if (!locate(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
-  const int np = (ctx - first_key(p, ctx) + kPart - 1) / kPart;
+  if (!locate_block<kThreadsM>(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
+  const int np = (ctx - first_key(p, ctx) + p.part - 1) / p.part;
+  if (np == 1 && p.by_mma) return;  // written by the attention kernel
   float o[kPer], ss = 0.f;
 #pragma unroll
   for (int n = 0; n < kPer; ++n) o[n] = 0.f;
@@ -843,7 +935,7 @@ __global__ void __launch_bounds__(kThreadsM) paged_merge_maps_kernel(Params p) {
 }
 
 // LVB_PAGED_ATTENTION=direct selects the kernel that reads the cache rows straight from global memory for every shape,
-// LVB_PAGED_ATTENTION=staged the scalar kernel on staged rows; the default for D = 128 is the tensor-core kernel.
+// LVB_PAGED_ATTENTION=staged the scalar kernel on staged rows; the default for D = 64 and 128 is the tensor-core kernel.
 inline int paged_variant() {
   static const int v = [] {
     const char* e = std::getenv("LVB_PAGED_ATTENTION");
@@ -854,14 +946,31 @@ inline int paged_variant() {
   return v;
 }
 
-template <int DKC, int DVC, bool kExact>
+// Keys per partition of the tensor-core kernel for T queries over KV heads and contexts of up to `keys`: as long as possible (a partition opens
+// with a chain of loads, ends with a merge of its warps and leaves a partial result, 5 us in all) while there are about eight CTAs for each of the
+// three places of an SM, so that ragged lengths even out; below 256 only where few queries leave half of the places empty.  64 sequences of up to
+// 4096, 8 KV heads: 512 keys, 167 us with 256 and a search per CTA, 134 now; 256 of up to 2304: 1024 keys, 357 -> 237.
+inline int part_keys(int T, int KV, int keys) {
+  int part = 1024;
+  const long long places = 3ll * num_sms();
+  auto ctas = [&] { return static_cast<long long>(T) * KV * ((keys + part - 1) / part); };
+  while (part > 256 && ctas() < 8 * places) part >>= 1;
+  while (part > 64 && 2 * ctas() < places) part >>= 1;
+  while ((keys + part - 1) / part > kMaxParts) part <<= 1;
+  return part;
+}
+
+inline bool by_mma(int D, int H, int KV) { return (D == 64 || D == 128) && H / KV <= 16 && paged_variant() == 2; }
+
+template <int DKC, int DVC, bool kExact, bool kSplitP = false>
 int launch_mma(const Params& p, cudaStream_t s) {
-  const int smem = kExact ? mma_smem(DKC, DVC) : mma_smem((p.dk + 15) & ~15, (p.dv + 15) & ~15);
-  auto kern = paged_attention_mma_kernel<DKC, DVC, kExact>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mma_smem(DKC, DVC)) != cudaSuccess) return kErrCuda;
-    attr_set = true;
+  const int smem = kExact ? mma_smem(DKC, DVC, p.part) : mma_smem((p.dk + 15) & ~15, (p.dv + 15) & ~15, p.part);
+  auto kern = paged_attention_mma_kernel<DKC, DVC, kExact, kSplitP>;
+  static int most = 0;  // 4096 keys per partition are those of contexts of a million tokens
+  if (smem > most) {
+    const int room = smem > mma_smem(DKC, DVC, 4096) ? smem : mma_smem(DKC, DVC, 4096);
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) return kErrCuda;
+    most = room;
   }
   kern<<<dim3(p.T, p.KV, p.parts), kThreads, smem, s>>>(p);
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
@@ -882,8 +991,8 @@ template <int D>
 int launch(const Params& p, cudaStream_t s) {
   dim3 grid(p.T, p.KV, p.parts);
   const int variant = paged_variant();
-  if (D == 128 && p.H / p.KV <= 16 && variant == 2) {
-    const int rc = launch_mma<128, 128, true>(p, s);
+  if (p.by_mma) {
+    const int rc = D == 128 ? launch_mma<128, 128, true>(p, s) : launch_mma<64, 64, true, true>(p, s);
     if (rc != kErrOk) return rc;
   } else if (D == 128 && p.H / p.KV <= kStagedMaxG && variant >= 1) {
     paged_attention_staged_kernel<<<grid, kThreads, 0, s>>>(p);
@@ -909,26 +1018,32 @@ extern "C" int lvb_kv_page_write(void* kv_pages, const void* k, const void* v, c
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }
 
-// Number of key partitions for a cache whose sequences hold at most max_context tokens: sizes the scratch buffers
-// part_o fp32 [T, H, parts, D] and part_ml fp32 [T, H, parts, 2] (unused when parts == 1).
-extern "C" int lvb_paged_attention_parts(int max_context) { return (max_context + lvb::paged::kPart - 1) / lvb::paged::kPart; }
+// Keys per partition for T queries of H heads over sequences of at most max_context tokens.  parts = ceil(max_context / that) sizes the scratch
+// buffers part_o fp32 [T, H, parts, D] and part_ml fp32 [T, H, parts, 2] (unused when parts == 1).
+extern "C" int lvb_paged_attention_part(int T, int H, int KV, int D, int max_context) {
+  using namespace lvb::paged;
+  return KV > 0 && by_mma(D, H, KV) ? part_keys(T, KV, max_context) : kPart;
+}
 
 extern "C" int lvb_paged_attention(const void* q, const void* kv_pages, const int* kv_lens, const int* page_indices,
                                    const int* cu_q_lens, const int* num_seqs, void* out, float* part_o, float* part_ml, int T,
                                    int H, int KV, int D, int S, int pages_per_seq, int page_size, int num_pages, float scale,
-                                   float soft_cap, void* stream) {
+                                   float soft_cap, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::paged;
   if (T <= 0) return kErrOk;
   if (H <= 0 || KV <= 0 || H % KV != 0 || H / KV > kMaxG || S <= 0) return kErrBadArg;
   Params p;
+  p.status = status;
   p.q = reinterpret_cast<const __nv_bfloat16*>(q);
   p.kv_pages = reinterpret_cast<const __nv_bfloat16*>(kv_pages);
   p.kv_lens = kv_lens; p.page_indices = page_indices; p.cu_q_lens = cu_q_lens; p.num_seqs = num_seqs;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.part_o = part_o; p.part_ml = part_ml;
   p.T = T; p.H = H; p.KV = KV; p.S = S; p.pages_per_seq = pages_per_seq; p.page_size = page_size; p.num_pages = num_pages;
-  p.parts = lvb_paged_attention_parts(pages_per_seq * page_size);
+  p.part = lvb_paged_attention_part(T, H, KV, D, pages_per_seq * page_size);
+  p.by_mma = by_mma(D, H, KV);
+  p.parts = (pages_per_seq * page_size + p.part - 1) / p.part;
   p.scale = scale; p.soft_cap = soft_cap;
   p.dk = p.dv = D; p.chunk = 0; p.window = 0; p.ldq = static_cast<long long>(H) * D; p.gate = nullptr; p.ldg = 0;
   p.gate_per_head = 0; p.maps = 1; p.weight = nullptr; p.diff_scale = p.eps = 0.f;
@@ -942,11 +1057,19 @@ extern "C" int lvb_paged_attention(const void* q, const void* kv_pages, const in
   }
 }
 
+namespace lvb {
+namespace paged {
+inline int general_keys(int max_context, int chunk, int window) {  // the most keys that a query sees
+  const int keys = chunk > 0 && chunk < max_context ? chunk : max_context;
+  return window > 0 && window < keys ? window : keys;
+}
+}  // namespace paged
+}  // namespace lvb
+
 // Partitions of keys per query of lvb_paged_attention_general: sizes part_o fp32 [T, H, parts, dv] and part_ml fp32 [T, H, parts, 2].
-extern "C" int lvb_paged_attention_general_parts(int max_context, int chunk, int window) {
-  int keys = chunk > 0 && chunk < max_context ? chunk : max_context;
-  keys = window > 0 && window < keys ? window : keys;
-  return (keys + lvb::paged::kPart - 1) / lvb::paged::kPart;
+extern "C" int lvb_paged_attention_general_parts(int T, int KV, int max_context, int chunk, int window) {
+  const int keys = lvb::paged::general_keys(max_context, chunk, window), part = lvb::paged::part_keys(T, KV, keys);
+  return (keys + part - 1) / part;
 }
 
 // lvb_paged_attention for any key and value size up to 256 (multiples of 8), with
@@ -961,7 +1084,7 @@ extern "C" int lvb_paged_attention_general(const void* q, const void* kv_pages, 
                                            const int* cu_q_lens, const int* num_seqs, const void* gate, void* out, float* part_o,
                                            float* part_ml, int T, int H, int KV, int dk, int dv, int ldq, int ldg, int gate_per_head, int S,
                                            int pages_per_seq, int page_size, int num_pages, int chunk, int window, float scale,
-                                           float soft_cap, const float* weight, float diff_scale, float eps, void* stream) {
+                                           float soft_cap, const float* weight, float diff_scale, float eps, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::paged;
   if (T <= 0) return kErrOk;
@@ -971,13 +1094,16 @@ extern "C" int lvb_paged_attention_general(const void* q, const void* kv_pages, 
   if (weight != nullptr) dk *= 2;
   if (dk > 256 || dv > 256) return kErrBadArg;
   Params p;
+  p.status = status;
   p.q = reinterpret_cast<const __nv_bfloat16*>(q);
   p.kv_pages = reinterpret_cast<const __nv_bfloat16*>(kv_pages);
   p.kv_lens = kv_lens; p.page_indices = page_indices; p.cu_q_lens = cu_q_lens; p.num_seqs = num_seqs;
   p.out = reinterpret_cast<__nv_bfloat16*>(out);
   p.part_o = part_o; p.part_ml = part_ml;
   p.T = T; p.H = H; p.KV = KV; p.S = S; p.pages_per_seq = pages_per_seq; p.page_size = page_size; p.num_pages = num_pages;
-  p.parts = lvb_paged_attention_general_parts(pages_per_seq * page_size, chunk, window);
+  p.by_mma = true;
+  p.part = part_keys(T, KV, general_keys(pages_per_seq * page_size, chunk, window));
+  p.parts = lvb_paged_attention_general_parts(T, KV, pages_per_seq * page_size, chunk, window);
   p.scale = scale; p.soft_cap = soft_cap;
   p.dk = dk; p.dv = dv; p.chunk = chunk; p.window = window; p.ldq = ldq; p.ldg = ldg;
   p.gate = reinterpret_cast<const __nv_bfloat16*>(gate); p.gate_per_head = gate_per_head;

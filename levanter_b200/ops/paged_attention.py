@@ -64,8 +64,8 @@ def ragged_paged_attention(q: torch.Tensor, kv_pages: torch.Tensor, kv_lens: tor
 def _paged_attention_cuda(q, kv_pages, kv_lens, page_indices, cu_q_lens, num_seqs, sm_scale, soft_cap):
     c = lib
     if "a" not in _f:
-        _f["a"] = lib.fn("lvb_paged_attention", [c.c_void_p] * 9 + [c.c_int] * 8 + [c.c_float, c.c_float, c.c_void_p], launches=2)
-        _f["parts"] = lib.fn("lvb_paged_attention_parts", [c.c_int], launches=0)
+        _f["a"] = lib.fn("lvb_paged_attention", [c.c_void_p] * 9 + [c.c_int] * 8 + [c.c_float, c.c_float, c.c_void_p, c.c_void_p], launches=2)
+        _f["part"] = lib.fn("lvb_paged_attention_part", [c.c_int] * 5, launches=0)
     T, H, D = q.shape
     P, ps, H2, _ = kv_pages.shape
     S, PP = page_indices.shape
@@ -73,7 +73,7 @@ def _paged_attention_cuda(q, kv_pages, kv_lens, page_indices, cu_q_lens, num_seq
     i32 = lambda t: t.to(device=dev, dtype=torch.int32).contiguous()  # noqa: E731
     ns = num_seqs if isinstance(num_seqs, torch.Tensor) else torch.tensor(int(num_seqs), dtype=torch.int32)
     ns = i32(ns.reshape(1))
-    parts = _f["parts"](PP * ps)
+    parts = -(-PP * ps // _f["part"](T, H, H2 // 2, D, PP * ps))
     key = (dev, T, H, parts, D)
     if parts > 1 and key not in _scratch:
         _scratch.clear()  # one live shape at a time: the engine calls with fixed T per phase
@@ -84,7 +84,7 @@ def _paged_attention_cuda(q, kv_pages, kv_lens, page_indices, cu_q_lens, num_seq
     out = torch.empty_like(qc)
     rc = _f["a"](qc.data_ptr(), kv_pages.data_ptr(), i32(kv_lens).data_ptr(), i32(page_indices).data_ptr(), i32(cu_q_lens).data_ptr(),
                  ns.data_ptr(), out.data_ptr(), lib.ptr(po), lib.ptr(pml), T, H, H2 // 2, D, S, PP, ps, P, float(sm_scale),
-                 float(soft_cap or 0.0), lib.stream_ptr())
+                 float(soft_cap or 0.0), lib.status_buffer().data_ptr(), lib.stream_ptr())
     lib.check_rc(rc, "lvb_paged_attention")
     return out
 
@@ -184,16 +184,16 @@ def paged_attention_general(q: torch.Tensor, kv_pages: torch.Tensor, kv_heads: i
         lib.check_rc(rc, "lvb_attention_any")
         return out
     if "g" not in _f:
-        _f["g"] = lib.fn("lvb_paged_attention_general", [c.c_void_p] * 10 + [c.c_int] * 14 + [c.c_float, c.c_float, c.c_void_p, c.c_float, c.c_float, c.c_void_p],
+        _f["g"] = lib.fn("lvb_paged_attention_general", [c.c_void_p] * 10 + [c.c_int] * 14 + [c.c_float, c.c_float, c.c_void_p, c.c_float, c.c_float, c.c_void_p, c.c_void_p],
                          launches=2)
-        _f["gparts"] = lib.fn("lvb_paged_attention_general_parts", [c.c_int] * 3, launches=0)
-    parts = _f["gparts"](PP * ps, int(chunk or 0), int(window or 0))
+        _f["gparts"] = lib.fn("lvb_paged_attention_general_parts", [c.c_int] * 5, launches=0)
+    parts = _f["gparts"](T, kv_heads, PP * ps, int(chunk or 0), int(window or 0))
     po = pml = None
     if parts > 1:
         po, pml = _part_scratch(dev, T * rows * parts * v_size, T * rows * parts * 2)
     rc = _f["g"](q.data_ptr(), kv.data_ptr(), lens.data_ptr(), pages.data_ptr(), cu.data_ptr(), ns.data_ptr(), lib.ptr(gate), out.data_ptr(), lib.ptr(po),
                  lib.ptr(pml), T, rows, kv_heads, dk, v_size, q.stride(0), ldg, per_head, S, PP, ps, P, int(chunk or 0), int(window or 0),
-                 float(sm_scale), float(soft_cap or 0.0), *diff, lib.stream_ptr())
+                 float(sm_scale), float(soft_cap or 0.0), *diff, lib.status_buffer().data_ptr(), lib.stream_ptr())
     lib.check_rc(rc, "lvb_paged_attention_general")
     return out
 

@@ -199,3 +199,24 @@ def test_sampler_rows_split_over_a_cluster(R, V, dtype):
     same = tok == tok_r  # scores that are closer than the rounding of the noise may swap
     assert int(tok[0]) == 1 and same.float().mean() > 0.95
     assert torch.allclose(lp[same], lp_r[same], atol=1e-4, rtol=1e-5)
+
+
+@pytest.mark.parametrize("D,KV,G,q_lens,kv_lens,per_seq", [
+    (64, 2, 4, [1, 1, 1], [1, 65, 1500], 96),                     # partitions of 64 keys, a quarter of one key
+    (64, 1, 16, [1] * 40, [16 * i + 7 for i in range(40)], 48),   # more sequences than a warp has lanes
+    (128, 8, 2, [700, 1], [700, 512], 44),                        # many queries: long partitions, most of them past their query
+    (128, 8, 1, [300] * 3, [300, 1100, 2000], 130),               # partitions of 512 and 1024 with remainders
+])
+def test_paged_attention_partitions_of_every_length(D, KV, G, q_lens, kv_lens, per_seq):
+    """Outputs are bf16 (2^-9); heads of 64 keep their probabilities in two bf16 parts, so that nothing else shows there."""
+    from levanter_b200.ops import paged_attention as PA
+
+    q, kv, lens, pages, cu, n = _random_case(len(q_lens) + 3, KV, G, D, 16, per_seq, q_lens, kv_lens, seed=9)
+    scale = 1.0 / math.sqrt(D)
+    got = PA.ragged_paged_attention(q, kv, lens, pages, cu, n, sm_scale=scale)
+    want = PA.ragged_paged_attention_reference(q.double(), kv.double(), lens, pages, cu, n, sm_scale=scale)
+    lib.check_status()
+    live = sum(q_lens)
+    err = (got[:live].double() - want[:live].double()).norm() / want[:live].double().norm()
+    assert err < (2 ** -9 if D == 64 else 2 ** -7), err
+    assert not got[live:].any()
