@@ -597,16 +597,23 @@ class Attention(nn.Module):
                 or c.head_temperature or c.value_mixing or c.head_gate or c.differential is not None or (self.rot is not None and not self.rot.is_plain):
             out, _ = self._paged_heads(x, kv_cache, batch_info, pos_ids)
             return (self.o_proj(out) if residual is None else self.o_proj(out) + residual), kv_cache
-        q, k, v = self._compute_qkv(x, pos_ids)
-        kv_cache = kv_cache.update(batch_info, k, v)
         scale = c.scaling_factor if c.scaling_factor is not None else 1.0 / math.sqrt(c.head_size)
         seg = getattr(batch_info, "prefill_segment_ids", None)
+        prepared = self._prepared_for_pages(x, kv_cache)
+        if prepared:
+            # rotary positions and the cache write in one pass over the rows, which a decode step's joint projection leaves side by side
+            q, k, v = self._project_and_prepare(x, kv_cache, batch_info, pos_ids, joint=x.shape[0] <= DECODE_ROWS)
+        else:
+            q, k, v = self._compute_qkv(x, pos_ids)
+            kv_cache = kv_cache.update(batch_info, k, v)
         if seg is not None and x.is_cuda:
             # pure prefill: nothing to read from the cache, so this is causal attention over the packed tokens with one segment
             # per sequence (the flash kernel), instead of the decode kernel walking pages
             m = AttentionMask.causal(sliding_window=c.sliding_window).with_segment_ids(seg.unsqueeze(0), sorted=True)
             out = dot_product_attention(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), m, attn_backend=c.attn_backend,
                                         logits_soft_cap=c.logits_soft_cap, scaling_factor=c.scaling_factor, inference=True).squeeze(0)
+        elif prepared:
+            out = PA.paged_attention_general(q, kv_cache.kv_pages, self.local_kv, c.head_size, batch_info, sm_scale=scale, soft_cap=c.logits_soft_cap)
         else:
             out = PA.ragged_paged_attention(q, kv_cache.kv_pages, batch_info.seq_lens, batch_info.page_indices,
                                             batch_info.cu_q_lens, batch_info.num_seqs, sm_scale=scale,
@@ -619,6 +626,34 @@ class Attention(nn.Module):
                 return linear_residual(out, self.o_proj.weight, self.o_proj.bias, residual), kv_cache
             return self.o_proj(out) + residual, kv_cache
         return self.o_proj(out), kv_cache
+
+    def _prepared_for_pages(self, x, kv_cache: "KvPageCache") -> bool:
+        """Whether a plain serving step takes the kernels between projections and pages: bf16 rows and pages on a GPU, heads of 64 or 128 in
+        groups that the tensor-core decode kernel has."""
+        from ..ops import lib
+
+        return (x.is_cuda and not torch.is_grad_enabled() and lib.available() and x.dim() == 2 and x.dtype == torch.bfloat16
+                and kv_cache.kv_pages.dtype == torch.bfloat16 and self.config.head_size in (64, 128) and self.local_heads // self.local_kv <= 16
+                and all(m.weight.dtype == torch.bfloat16 for m in self._projections() if type(m) is Linear))
+
+    def _project_and_prepare(self, x, kv_cache: "KvPageCache", batch_info, pos_ids, joint: bool):
+        """``q, k, v`` rows as attention reads them (slices of the joint product's rows with ``joint``), keys and values written to the pages."""
+        from ..ops import paged_attention as PA
+        from ..ops.qkv_prep import prepare_qkv
+        from ..ops.residual_stream import project
+
+        D = self.config.head_size
+        nq, nk = self.local_heads * D, self.local_kv * D
+        fused = self._fused_projection() if joint and self.q_norm is None else None
+        if fused is not None:
+            y = project(x, fused[0], bias=fused[1])
+            q, k, v = y[:, :nq].unflatten(1, (-1, D)), y[:, nq:nq + nk].unflatten(1, (-1, D)), y[:, nq + nk:nq + 2 * nk].unflatten(1, (-1, D))
+        else:
+            q, k, v = self._compute_qkv(x, pos_ids, rotate=False)
+        if self.rot is not None:
+            return prepare_qkv(q, k, v, kv_cache.kv_pages, batch_info.new_token_dests, pos_ids, rot=self.rot)
+        PA.kv_page_write_general(kv_cache.kv_pages, k, v, batch_info.new_token_dests)
+        return q, k, v
 
     def _fused_projection(self):
         """``(weight, bias or None)`` of the joint projection ``[q; k; v; gate]`` for serving: the projections read the same rows, so a
@@ -698,6 +733,12 @@ class Attention(nn.Module):
     def empty_page_cache(self, max_pages: int, page_size: int, *, dtype=torch.bfloat16, device=None) -> "KvPageCache":
         c = self.config
         return KvPageCache.init(max_pages, page_size, self.local_kv, c.maps * c.head_size, v_head_size=c.v_head_size, dtype=dtype, device=device)
+
+
+# Rows up to which a serving step's projections that read the same rows are one product over their weights laid out side by side.  Such products
+# stream their weights, and each of them costs about 7 us beside that: 8 rows of a Llama 3 8B layer, three products 33 us and three sums of their
+# parts 7, one product 15 and 2 (a round of four such layers 827 -> 726 us).  Larger steps are bound by the tensor cores, and their rows go to kernels that want them packed.
+DECODE_ROWS = 128
 
 
 class AttentionWithSink(Attention):

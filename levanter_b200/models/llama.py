@@ -18,7 +18,7 @@ import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
 from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
-from ..layers.attention import Attention, AttentionBackend, AttentionConfig, AttentionMask, KvPageCache
+from ..layers.attention import DECODE_ROWS, Attention, AttentionBackend, AttentionConfig, AttentionMask, KvPageCache
 from ..layers.normalization import LayerNormConfigBase, RmsNormConfig
 from ..layers.rotary import rope_config_from_hf, rope_to_hf_dict, DefaultRotaryEmbeddingsConfig, RotaryEmbeddingsConfig
 from ..nn import Embedding, FusedRows, Linear
@@ -192,7 +192,10 @@ class LlamaMlp(nn.Module):
     def forward(self, x: torch.Tensor, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
         if self.tp is not None and self.tp.size > 1:
             x = self.tp.copy_to_region(x)
-        h = gated_activation(self.gate_proj(x), self.up_proj(x), self.act)
+        if x.dim() == 2 and x.shape[0] <= DECODE_ROWS and not torch.is_grad_enabled() and x.dtype == self.gate_proj.weight.dtype == torch.bfloat16:
+            h = self._inner(x)
+        else:
+            h = gated_activation(self.gate_proj(x), self.up_proj(x), self.act)
         if self.tp is not None and self.tp.size > 1:
             out = self.tp.row_linear(h, self.down_proj)
             if self.down_proj.bias is not None:

@@ -97,6 +97,8 @@ class FusedRows:
                     break
                 at += p.numel() * p.element_size()
         if fused is None:
+            if params[0].is_cuda and torch.cuda.is_current_stream_capturing():
+                return None  # the copy would be recorded and not made, and what follows would read the new rows
             rows = [p.detach() for p in params]
             if self.pad:
                 rows.append(rows[0].new_zeros(self.pad, *rows[0].shape[1:]))

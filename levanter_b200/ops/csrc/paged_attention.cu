@@ -1112,6 +1112,7 @@ extern "C" int lvb_paged_attention_general(const void* q, const void* kv_pages, 
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   int rc;
   if (dk == 128 && dv == 128) rc = launch_mma<128, 128, true>(p, s);
+  else if (dk == 64 && dv == 64 && p.maps == 1) rc = launch_mma<64, 64, true, true>(p, s);
   else if (dk <= 64 && dv <= 64) rc = launch_mma<64, 64, false>(p, s);
   else if (dk <= 128 && dv <= 128) rc = launch_mma<128, 128, false>(p, s);
   else if (dk <= 192 && dv <= 128) rc = launch_mma<192, 128, false>(p, s);

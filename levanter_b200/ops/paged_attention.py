@@ -169,7 +169,7 @@ def paged_attention_general(q: torch.Tensor, kv_pages: torch.Tensor, kv_heads: i
     dev = q.device
     i32 = lambda t: t.to(device=dev, dtype=torch.int32).contiguous()  # noqa: E731
     lens, pages, cu = i32(b.seq_lens), i32(b.page_indices), i32(b.cu_q_lens)
-    ns = i32(b.num_seqs.reshape(1))
+    ns = i32(torch.as_tensor(b.num_seqs).reshape(1))
     q = _strided_rows(q, rows * dk)
     gate, ldg, per_head = _gate_args(gate, q.dtype, H, v_size)
     diff = _difference_args(difference)

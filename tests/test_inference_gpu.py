@@ -220,3 +220,44 @@ def test_paged_attention_partitions_of_every_length(D, KV, G, q_lens, kv_lens, p
     err = (got[:live].double() - want[:live].double()).norm() / want[:live].double().norm()
     assert err < (2 ** -9 if D == 64 else 2 ** -7), err
     assert not got[live:].any()
+
+
+@pytest.mark.parametrize("heads,kv,hidden,bias", [(4, 2, 512, False), (8, 8, 512, False), (2, 1, 256, True)])
+@pytest.mark.parametrize("tokens", [3, 200])
+def test_plain_serving_step_prepares_rows_in_one_pass(heads, kv, hidden, bias, tokens, monkeypatch):
+    """Joint projections, rotation and cache write in one kernel (up to 128 rows), separate projections above: the same pages and heads as the
+    separate kernels, up to the bf16 rounding of a sum whose parts were added in another order (2^-8 of a value)."""
+    from levanter_b200.inference.page_table import PageTable
+    from levanter_b200.layers.attention import Attention, AttentionConfig, KvPageCache
+    from levanter_b200.layers.rotary import DefaultRotaryEmbeddingsConfig
+
+    torch.manual_seed(0)
+    cfg = AttentionConfig(hidden_dim=hidden, num_heads=heads, num_kv_heads=kv, use_bias=bias, rope=DefaultRotaryEmbeddingsConfig())
+    with torch.device("cuda"):
+        attn = Attention(cfg).to(torch.bfloat16).eval()
+    if bias:
+        for m in (attn.q_proj, attn.k_proj, attn.v_proj):
+            m.bias.data.normal_(0, 0.1)
+    seqs = 3
+    lens = [tokens // seqs + (i < tokens % seqs) for i in range(seqs)]
+    table = PageTable.init(64, seqs, 16, 16)
+    for s in range(seqs):
+        table, _ = table.assign_seq_id_to_seq(s)
+    slots = np.concatenate([np.full(n, s, np.int32) for s, n in enumerate(lens)])
+    pos = np.concatenate([np.arange(n, dtype=np.int32) for n in lens])
+    table, info = table.allocate_for_seq(slots, pos)
+    info, pos = info.to("cuda"), torch.from_numpy(pos).cuda()
+    x = torch.randn(tokens, hidden, device="cuda").bfloat16()
+
+    def run():
+        cache = attn.empty_page_cache(64, 16, device="cuda")
+        with torch.no_grad():
+            out, cache = attn.paged_decode(x, cache, info, pos)
+        return out.float(), cache.kv_pages.float()
+
+    out, pages = run()
+    monkeypatch.setattr(Attention, "_prepared_for_pages", lambda *a: False)
+    out_r, pages_r = run()
+    lib.check_status()
+    assert (pages - pages_r).abs().max() <= 2 ** -7 * pages_r.abs().max()
+    assert (out - out_r).norm() <= 2 ** -7 * out_r.norm()
