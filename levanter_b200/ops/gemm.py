@@ -292,6 +292,12 @@ def _skinny_workspace(device, M: int, N: int) -> int:
 _SKINNY_SPLIT_MAX_TILES = 74  # more 128 x 128 tiles than half the SMs: the launcher does not split K
 
 
+def _linear_rows(x, weight, bias, residual):
+    shp = x.shape
+    y = gemm(x.reshape(-1, shp[-1]), weight, bias=bias, residual=None if residual is None else residual.reshape(-1, weight.shape[0]))
+    return y.view(*shp[:-1], weight.shape[0])
+
+
 class _LinearFn(torch.autograd.Function):
     """y = x W^T (+ b).  ``weight`` is ``[out, in]``.
 
@@ -303,16 +309,12 @@ class _LinearFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, weight, bias, residual=None):
-        shp = x.shape
-        x2 = x.reshape(-1, shp[-1])
-        r2 = residual.reshape(-1, weight.shape[0]) if residual is not None else None
-        y = gemm(x2, weight, bias=bias, residual=r2)
-        ctx.save_for_backward(x2, weight)
+        ctx.save_for_backward(x.reshape(-1, x.shape[-1]), weight)
         ctx.has_bias = bias is not None
         ctx.has_res = residual is not None
-        ctx.x_shape = shp
+        ctx.x_shape = x.shape
         ctx.weight_ref = weight
-        return y.view(*shp[:-1], weight.shape[0])
+        return _linear_rows(x, weight, bias, residual)
 
     @staticmethod
     def backward(ctx, dy):
@@ -350,7 +352,7 @@ def _tma_shapes_ok(weight: torch.Tensor) -> bool:
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Linear layer on the tcgen05 GEMM when running bf16 on a B200; ``F.linear`` otherwise."""
     if x.is_cuda and lib.available() and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and _tma_shapes_ok(weight):
-        return _LinearFn.apply(x, weight, bias, None)
+        return _linear_rows(x, weight, bias, None) if lib.plain_call() else _LinearFn.apply(x, weight, bias, None)
     return torch.nn.functional.linear(x, weight, bias)
 
 
@@ -362,5 +364,5 @@ def linear_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
         weight = weight.to(x.dtype)
         bias = bias.to(x.dtype) if bias is not None else None
     if x.is_cuda and lib.available() and x.dtype == torch.bfloat16 and residual.dtype == torch.bfloat16 and _tma_shapes_ok(weight):
-        return _LinearFn.apply(x, weight, bias, residual)
+        return _linear_rows(x, weight, bias, residual) if lib.plain_call() else _LinearFn.apply(x, weight, bias, residual)
     return torch.nn.functional.linear(x, weight, bias) + residual

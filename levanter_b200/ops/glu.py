@@ -46,20 +46,25 @@ def _bwd():
     return _f["b"]
 
 
+def _glu_rows(gate, up, act):
+    """``(out, gate, up)`` as rows."""
+    cols = gate.shape[-1]
+    g2 = gate.reshape(-1, cols)
+    u2 = up.reshape(-1, cols)
+    if g2.stride(1) != 1:
+        g2 = g2.contiguous()
+    if u2.stride(1) != 1:
+        u2 = u2.contiguous()
+    out = torch.empty(g2.shape, dtype=gate.dtype, device=gate.device)
+    rc = _fwd()(g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0], cols, g2.stride(0), u2.stride(0), out.stride(0), act, lib.stream_ptr())
+    lib.check_rc(rc, "lvb_glu_fwd")
+    return out, g2, u2
+
+
 class _GluFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, gate, up, act):
-        cols = gate.shape[-1]
-        g2 = gate.reshape(-1, cols)
-        u2 = up.reshape(-1, cols)
-        if g2.stride(1) != 1:
-            g2 = g2.contiguous()
-        if u2.stride(1) != 1:
-            u2 = u2.contiguous()
-        out = torch.empty(g2.shape, dtype=gate.dtype, device=gate.device)
-        rc = _fwd()(g2.data_ptr(), u2.data_ptr(), out.data_ptr(), g2.shape[0], cols, g2.stride(0), u2.stride(0), out.stride(0),
-                    act, lib.stream_ptr())
-        lib.check_rc(rc, "lvb_glu_fwd")
+        out, g2, u2 = _glu_rows(gate, up, act)
         ctx.save_for_backward(g2, u2)
         ctx.act = act
         ctx.shape = gate.shape
@@ -86,5 +91,5 @@ def gated_activation(gate: torch.Tensor, up: torch.Tensor, act: GatedActivation)
     act = ActivationFunctionEnum(act) if not isinstance(act, ActivationFunctionEnum) else act
     if (gate.is_cuda and lib.available() and gate.dtype == torch.bfloat16 and up.dtype == torch.bfloat16
             and gate.shape[-1] % 8 == 0 and act in _ACT):
-        return _GluFn.apply(gate, up, _ACT[act])
+        return _glu_rows(gate, up, _ACT[act])[0].view(gate.shape) if lib.plain_call() else _GluFn.apply(gate, up, _ACT[act])
     return act.to_fn()(gate) * up

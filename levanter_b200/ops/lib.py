@@ -51,10 +51,29 @@ def available() -> bool:
     """True when the native kernels can run here (a CUDA device of compute capability 10.x)."""
     if getattr(_tls, "reference", 0):
         return False
-    if not cuda_ok():
+    if not torch.cuda.is_initialized() and not cuda_ok():
         return False
-    major, _ = torch.cuda.get_device_capability()
+    dev = _current_device()
+    major = _major.get(dev)
+    if major is None:
+        major = _major[dev] = torch.cuda.get_device_capability()[0]
     return major == 10
+
+
+# A kernel's launch goes through here several times.  The public functions (current_stream, current_device, get_device_capability) make objects and
+# look up environment variables on the way, 30 us per launch in all on a layer of a few rows, more than the launch itself; these read the same state.
+_major: dict[int, int] = {}  # compute capability by device, which does not change while a process runs
+
+
+def _current_device() -> int:
+    torch.cuda.init()  # returns at once when done
+    return torch._C._cuda_getDevice()
+
+
+def plain_call() -> bool:
+    """No gradient is recorded and no transform (vmap, jvp, ...) or forward-mode level is active: an operation may run without its autograd
+    function."""
+    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
 
 
 _serving = False
@@ -102,7 +121,7 @@ def fn(name: str, argtypes: list, restype=c_int, launches: int = 1):
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(_current_device())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:
@@ -111,7 +130,7 @@ def ptr(t: Optional[torch.Tensor]) -> int:
 
 def status_buffer() -> torch.Tensor:
     """Per-device int32[8] word that kernels write a timeout / bounds code into."""
-    dev = torch.cuda.current_device()
+    dev = _current_device()
     buf = _status.get(dev)
     if buf is None:
         buf = torch.zeros(8, dtype=torch.int32, device=f"cuda:{dev}")

@@ -65,36 +65,45 @@ def _kernel_ok(x, weight, bias) -> bool:
     return True
 
 
+def _weights_fp32(weight, bias) -> int:
+    w = weight if weight is not None else bias
+    return int(w is not None and w.dtype == torch.float32)
+
+
+def _norm_rows(x, residual, weight, bias, eps, layer_norm, w_offset, stats: bool):
+    """``(y, what was normalised, rstd, mean)`` as rows; the last two only with ``stats`` (and a mean only for LayerNorm)."""
+    dim = x.shape[-1]
+    x2 = x.reshape(-1, dim)
+    if not x2.is_contiguous():
+        x2 = x2.contiguous()
+    rows = x2.shape[0]
+    r2 = None
+    h = None
+    if residual is not None:
+        r2 = residual.reshape(-1, dim).contiguous()
+        h = torch.empty_like(x2)
+    y = torch.empty_like(x2)
+    rstd = torch.empty(rows, dtype=torch.float32, device=x.device) if stats else None
+    mean = torch.empty(rows, dtype=torch.float32, device=x.device) if stats and layer_norm else None
+    rc = _fwd()(x2.data_ptr(), lib.ptr(r2), lib.ptr(weight), lib.ptr(bias), _weights_fp32(weight, bias), y.data_ptr(), lib.ptr(h),
+                lib.ptr(rstd), lib.ptr(mean), rows, dim, float(eps), float(w_offset), int(layer_norm), lib.stream_ptr())
+    lib.check_rc(rc, "lvb_norm_fwd")
+    return y, h if h is not None else x2, rstd, mean
+
+
 class _NormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, residual, weight, bias, eps, layer_norm, w_offset):
-        dim = x.shape[-1]
-        x2 = x.reshape(-1, dim)
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        rows = x2.shape[0]
-        r2 = None
-        h = None
-        if residual is not None:
-            r2 = residual.reshape(-1, dim).contiguous()
-            h = torch.empty_like(x2)
-        y = torch.empty_like(x2)
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device) if layer_norm else None
-        wf32 = int((weight if weight is not None else bias).dtype == torch.float32) if (weight is not None or bias is not None) else 0
-        rc = _fwd()(x2.data_ptr(), lib.ptr(r2), lib.ptr(weight), lib.ptr(bias), wf32, y.data_ptr(), lib.ptr(h),
-                    rstd.data_ptr(), lib.ptr(mean), rows, dim, float(eps), float(w_offset), int(layer_norm), lib.stream_ptr())
-        lib.check_rc(rc, "lvb_norm_fwd")
-        xin = h if h is not None else x2
+        y, xin, rstd, mean = _norm_rows(x, residual, weight, bias, eps, layer_norm, w_offset, True)
         ctx.save_for_backward(xin, weight, rstd, mean)
         ctx.layer_norm = layer_norm
         ctx.w_offset = w_offset
         ctx.has_bias = bias is not None
         ctx.has_res = residual is not None
         ctx.shape = x.shape
-        ctx.wf32 = wf32
+        ctx.wf32 = _weights_fp32(weight, bias)
         if residual is not None:
-            return y.view(x.shape), h.view(x.shape)
+            return y.view(x.shape), xin.view(x.shape)
         return y.view(x.shape), None
 
     @staticmethod
@@ -129,6 +138,9 @@ class _NormFn(torch.autograd.Function):
 def fused_norm(x, weight, bias, eps, *, layer_norm=False, w_offset=0.0, residual=None) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
     """Returns ``(norm(x + residual), x + residual)`` (second item None when there is no residual)."""
     if _kernel_ok(x, weight, bias) and (residual is None or residual.dtype == torch.bfloat16):
+        if lib.plain_call():
+            y, h, _, _ = _norm_rows(x, residual, weight, bias, eps, layer_norm, w_offset, False)
+            return y.view(x.shape), None if residual is None else h.view(x.shape)
         return _NormFn.apply(x, residual, weight, bias, eps, layer_norm, w_offset)
     h = None
     if residual is not None:
