@@ -292,6 +292,26 @@ def _skinny_workspace(device, M: int, N: int) -> int:
 _SKINNY_SPLIT_MAX_TILES = 74  # more 128 x 128 tiles than half the SMs: the launcher does not split K
 
 
+_col_sum = None
+
+
+def col_sum(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """Sums of the columns of bf16 ``x [rows, cols]`` in fp32, as ``dtype`` where that is bf16 and as fp32 otherwise."""
+    global _col_sum
+    rows, cols = x.shape
+    if not (x.is_cuda and lib.available() and rows > 0 and cols % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+        return x.float().sum(0)
+    if _col_sum is None:
+        c = lib
+        _col_sum = (lib.fn("lvb_col_sum", [c.c_void_p, c.c_longlong, c.c_void_p, c.c_int, c.c_void_p, c.c_int, c.c_int, c.c_void_p], launches=2),
+                    lib.fn("lvb_col_sum_shares", [c.c_int] * 2, launches=0))
+    out = torch.empty(cols, dtype=dtype if dtype == torch.bfloat16 else torch.float32, device=x.device)
+    scratch = torch.empty(_col_sum[1](rows, cols) * cols, dtype=torch.float32, device=x.device)
+    rc = _col_sum[0](x.data_ptr(), x.stride(0), out.data_ptr(), int(out.dtype == torch.bfloat16), scratch.data_ptr(), rows, cols, lib.stream_ptr())
+    lib.check_rc(rc, "lvb_col_sum")
+    return out
+
+
 def _linear_rows(x, weight, bias, residual):
     shp = x.shape
     y = gemm(x.reshape(-1, shp[-1]), weight, bias=bias, residual=None if residual is None else residual.reshape(-1, weight.shape[0]))
@@ -311,6 +331,7 @@ class _LinearFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, residual=None):
         ctx.save_for_backward(x.reshape(-1, x.shape[-1]), weight)
         ctx.has_bias = bias is not None
+        ctx.bias_dtype = None if bias is None else bias.dtype
         ctx.has_res = residual is not None
         ctx.x_shape = x.shape
         ctx.weight_ref = weight
@@ -337,7 +358,7 @@ class _LinearFn(torch.autograd.Function):
             else:
                 dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=weight.dtype if weight.dtype in (torch.bfloat16, torch.float32) else torch.float32)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0)
+            db = col_sum(dy2, ctx.bias_dtype)
         dres = dy if ctx.has_res else None
         return dx, dw, db, dres
 

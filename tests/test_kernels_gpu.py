@@ -178,3 +178,15 @@ def test_norm_block_shapes(rows, dim, ln, residual, wdtype):
         assert (got.double() - want).norm() <= 2 ** -8 * want.norm() + 1e-6
     if residual:
         assert torch.equal(r.grad, x.grad)
+
+
+@pytest.mark.parametrize("rows,cols,dtype", [(1, 8, torch.bfloat16), (31, 264, torch.float32), (33, 768, torch.bfloat16), (999, 2304, torch.float32), (5000, 6144, torch.bfloat16)])
+def test_col_sum(rows, cols, dtype):
+    """fp32 sums of up to 5000 bf16 numbers (2^-24 sqrt(rows) relative to their norm), then at most one bf16 rounding."""
+    from levanter_b200.ops.gemm import col_sum
+
+    x = torch.randn(rows, cols + 8, device="cuda").bfloat16()[:, 8:]
+    got = col_sum(x, dtype)
+    want = x.double().sum(0)
+    assert got.dtype == dtype
+    assert (got.double() - want).norm() <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
