@@ -278,6 +278,15 @@ def _structured_only(mask) -> bool:
     return True
 
 
+def default_flash(q, k, v, mask, bias, no_dropout: bool, attention_dtype, attn_backend) -> bool:
+    """Whether :func:`dot_product_attention` with this backend takes the hand-written flash kernels for these rows."""
+    from ..ops import flash_attention as KFA
+
+    backend = AttentionBackend(attn_backend) if attn_backend is not None else AttentionBackend.DEFAULT
+    own = (AttentionBackend.DEFAULT, AttentionBackend.B200, AttentionBackend.NVTE, AttentionBackend.SPLASH)
+    return backend in own and KFA.supported(q, k, v, mask, bias, no_dropout, attention_dtype)
+
+
 def dot_product_attention(q, k, v, mask: Union[None, torch.Tensor, AttentionMask] = None, bias=None, *,
                           attention_dtype: Optional[torch.dtype] = None, dropout: float = 0.0, inference: bool = True,
                           use_flash: Optional[bool] = None, attn_backend: Optional[AttentionBackend] = None,

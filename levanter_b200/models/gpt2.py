@@ -13,8 +13,9 @@ import torch.nn as nn
 from torch.utils.checkpoint import checkpoint
 
 from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
-from ..layers.attention import AttentionBackend, AttentionMask, dot_product_attention
+from ..layers.attention import AttentionBackend, AttentionMask, default_flash, dot_product_attention
 from ..nn import Dropout, Embedding, LayerNorm, Linear, trunc_normal_
+from ..ops.flash_attention import flash_attention_joint
 from ..utils.activation import ActivationFunctionEnum
 from ..utils.flop_utils import lm_flops_per_token
 from ..utils.remat import should_recompute
@@ -121,12 +122,17 @@ class Gpt2Attention(nn.Module):
         B, S, E = x.shape
         qkv = self.c_attn(x).view(B, S, 3, c.num_heads, c.head_size)
         q, k, v = qkv[:, :, 0], qkv[:, :, 1], qkv[:, :, 2]
+        dtype = torch.float32 if c.upcast_attn else None
+        if c.use_flash_attention is not False and default_flash(q, k, v, mask, None, c.attn_pdrop == 0.0 or not self.training, dtype, c.attn_backend):
+            # the kernels read the projection's rows where they are, and the scale of the layer joins that of the scores
+            scale = c.head_size ** -0.5 / (layer_idx + 1.0 if c.scale_attn_by_inverse_layer_idx else 1.0)
+            return self.c_proj(flash_attention_joint(qkv, mask, scaling_factor=scale).reshape(B, S, E))
         if c.scale_attn_by_inverse_layer_idx:
             q = q / (layer_idx + 1.0)
         out = dot_product_attention(q, k, v, mask, inference=not self.training, dropout=c.attn_pdrop,
                                     use_flash=c.use_flash_attention, attn_backend=c.attn_backend,
                                     flash_block_size=c.flash_attention_block_size,
-                                    attention_dtype=torch.float32 if c.upcast_attn else None)
+                                    attention_dtype=dtype)
         return self.c_proj(out.reshape(B, S, E).to(x.dtype))
 
 

@@ -477,6 +477,24 @@ inline int make_tmap_2d_bf16(CUtensorMap* out, const void* ptr, uint64_t rows, u
   return r == CUDA_SUCCESS ? kErrOk : kErrTensorMap;
 }
 
+// Rows of several sequences, [batch, rows, cols] bf16 with element strides ld and ld_batch: a box is box_rows rows of one sequence by 64 columns;
+// rows past a sequence's end are filled with zeros, whatever follows them in memory.
+inline int make_tmap_rows_bf16(CUtensorMap* out, const void* ptr, uint64_t batch, uint64_t rows, uint64_t cols, uint64_t ld, uint64_t ld_batch,
+                               uint32_t box_rows) {
+  ensure_context_for(ptr);
+  EncodeTiledFn enc = get_encode_tiled();
+  if (enc == nullptr) return kErrTensorMap;
+  if ((reinterpret_cast<uintptr_t>(ptr) & 15) != 0 || (ld * 2) % 16 != 0 || (ld_batch * 2) % 16 != 0) return kErrBadArg;
+  cuuint64_t gdim[3] = {cols, rows, batch};
+  cuuint64_t gstr[2] = {ld * 2, ld_batch * 2};
+  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstr, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? kErrOk : kErrTensorMap;
+}
+
 // Rows of several heads, [rows, heads, size] bf16 with row stride ld (elements): a box is 64 columns of one head in box_rows rows;
 // columns past `size` are filled with zeros.
 inline int make_tmap_heads_bf16(CUtensorMap* out, const void* ptr, uint64_t rows, uint64_t heads, uint64_t size, uint64_t ld,

@@ -37,8 +37,9 @@ constexpr int kBwdThreads = 320;  // warp0 TMA, warp1 MMA, warps 2-5 key columns
 
 struct BwdParams {
   float* dQ32;                 // [B, S, Hq, D] fp32, zero-initialised by the caller
-  __nv_bfloat16* dK;           // [B, S, Hkv, D]
-  __nv_bfloat16* dV;           // [B, S, Hkv, D]
+  __nv_bfloat16* dK;           // [B, Sk, Hkv, D], element strides ldk_batch and ldk of sequences and rows
+  __nv_bfloat16* dV;           // the same
+  long long ldk_batch, ldk;
   const float* lse2;           // [B, Hq, S]
   const float* delta;          // [B, Hq, S]
   const int* q_seg;
@@ -89,7 +90,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int nqb = p.S / BM;
+  const int nqb = (p.S + BM - 1) / BM, nkb = (p.Sk + BN - 1) / BN;
   const int jb = blockIdx.x;
   const int b = blockIdx.y / p.Hkv;
   const int hkv = blockIdx.y % p.Hkv;
@@ -104,7 +105,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last query block that can see one of the keys
   if constexpr (kSeg) {
     if (warp == 2) {
-      const uint2 own = __ldg(p.ranges + p.B * nqb + b * (p.Sk / BN) + jb);
+      const uint2 own = __ldg(p.ranges + p.B * nqb + b * nkb + jb);
       const int2 m = seg::meeting_blocks(p.ranges + b * nqb, own, ilo, ihi, lane);
       if (lane == 0) {  // at least one, so that dK and dV are written
         bounds[0] = m.x <= m.y ? m.x : ilo;
@@ -149,26 +150,25 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (warp == 0) {
     if (lane == 0) {
-      const int row_k = b * p.Sk + k0;
       mbar_expect_tx(kv_full, 2 * kQKV);
 #pragma unroll
       for (int c = 0; c < D / 64; ++c) {
-        tma_load_2d(smem + SmemB::kK + c * kChunkBytes, &tmK, kv_full, hkv * D + 64 * c, row_k);
-        tma_load_2d(smem + SmemB::kV + c * kChunkBytes, &tmV, kv_full, hkv * D + 64 * c, row_k);
+        tma_load_3d(smem + SmemB::kK + c * kChunkBytes, &tmK, kv_full, hkv * D + 64 * c, k0, b);
+        tma_load_3d(smem + SmemB::kV + c * kChunkBytes, &tmV, kv_full, hkv * D + 64 * c, k0, b);
       }
       bool ok = true;
       for (int t = 0; t < iters && ok; ++t) {
         const int g = t / nq;
         const int i = ilo + (t % nq);
         const int h = hkv * G + g;
-        const int row_q = b * p.S + i * BM;
+        const int row_q = i * BM;
         ok = mbar_wait(qdo_empty, (t & 1) ^ 1, abort_flag, p.status, 900, t);
         if (!ok) break;
         mbar_expect_tx(qdo_full, 2 * kQKV);
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
-          tma_load_2d(smem + SmemB::kQ + c * kChunkBytes, &tmQ, qdo_full, h * D + 64 * c, row_q);
-          tma_load_2d(smem + SmemB::kDO + c * kChunkBytes, &tmDO, qdo_full, h * D + 64 * c, row_q);
+          tma_load_3d(smem + SmemB::kQ + c * kChunkBytes, &tmQ, qdo_full, h * D + 64 * c, row_q, b);
+          tma_load_3d(smem + SmemB::kDO + c * kChunkBytes, &tmDO, qdo_full, h * D + 64 * c, row_q, b);
         }
       }
     }
@@ -236,7 +236,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int dbase = half * (D / 2);
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float scale_log2 = p.scale * 1.4426950408889634f;
-    const int* kseg_g = kSeg ? p.k_seg + b * p.Sk + k0 : nullptr;
+    const int* kseg_g = kSeg ? p.k_seg + b * p.Sk : nullptr;
     uint8_t* sPp = smem + SmemB::kP;
     uint8_t* sDSp = smem + SmemB::kDS;
     bool ok = true;
@@ -247,26 +247,28 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       const int h = hkv * G + g;
       const int qi = i * BM + r;
       const size_t stat_idx = (static_cast<size_t>(b) * p.Hq + h) * p.S + qi;
-      const float lse = p.lse2[stat_idx];
-      const float dlt = p.delta[stat_idx];
+      // rows past the end: probabilities of 2^-inf, and their queries and gradients are zeros
+      const bool inside = qi < p.S;
+      const float lse = inside ? p.lse2[stat_idx] : INFINITY;
+      const float dlt = inside ? p.delta[stat_idx] : 0.f;
       const float neg_lse = (lse == -INFINITY) ? -INFINITY : -lse;
-      const int my_seg = kSeg ? p.q_seg[b * p.S + qi] : 0;
+      const int my_seg = kSeg ? p.q_seg[b * p.S + min(qi, p.S - 1)] : 0;
       int ids[2] = {0, 0};
       if constexpr (kSeg) {
-        ids[0] = __ldg(kseg_g + cbase + lane);
-        ids[1] = __ldg(kseg_g + cbase + 32 + lane);
+        ids[0] = __ldg(kseg_g + min(k0 + cbase + lane, p.Sk - 1));
+        ids[1] = __ldg(kseg_g + min(k0 + cbase + 32 + lane, p.Sk - 1));
       }
       ok = mbar_wait(sdp_full, ph, abort_flag, p.status, 1100, t);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
       uint32_t visible[2] = {0xffffffffu, 0xffffffffu};  // a bit per key of this warp's columns
-      bool need_mask = (causal && i == jb) || (p.window > 0 && k0 <= i * BM + BM - 1 - p.window);
+      bool need_mask = (causal && i == jb) || (p.window > 0 && k0 <= i * BM + BM - 1 - p.window) || (!causal && k0 + BN > p.Sk);
       if constexpr (kSeg) need_mask = !seg::same_segment<2>(my_seg, ids, visible) || need_mask;
       if (need_mask) {
         const int kc = k0 + cbase;
 #pragma unroll
-        for (int u = 0; u < 2; ++u) visible[u] &= seg::bit_range((p.window > 0 ? qi - p.window + 1 : 0) - kc - 32 * u, causal ? qi - kc - 32 * u : 64);
+        for (int u = 0; u < 2; ++u) visible[u] &= seg::bit_range((p.window > 0 ? qi - p.window + 1 : 0) - kc - 32 * u, (causal ? qi : p.Sk - 1) - kc - 32 * u);
       }
 #pragma unroll 1
       for (int c = cbase; c < cbase + 64; c += 32) {
@@ -323,6 +325,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t v[32];
         tmem_ld_32x32(tmem_S + lane_addr + c, v);
         tmem_ld_wait();
+        if (!inside) continue;
 #pragma unroll
         for (int q4 = 0; q4 < 8; ++q4) {
           asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dq + c + q4 * 4),
@@ -339,7 +342,8 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // epilogue: dK, dV -> bf16 (this warp's D / 2 columns)
     if (ok) {
       tc_fence_after();
-      const size_t row = (static_cast<size_t>(b) * p.Sk + k0 + r) * (static_cast<size_t>(p.Hkv) * D) + static_cast<size_t>(hkv) * D;
+      const bool inside = k0 + r < p.Sk;
+      const size_t row = b * p.ldk_batch + (k0 + r) * p.ldk + static_cast<size_t>(hkv) * D;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         __nv_bfloat16* dst = (which == 0 ? p.dV : p.dK) + row;
@@ -349,6 +353,7 @@ flash_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           uint32_t v[32];
           tmem_ld_32x32(src + c, v);
           tmem_ld_wait();
+          if (!inside) continue;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             uint4 w;
@@ -399,7 +404,7 @@ __global__ void flash_delta_kernel(const __nv_bfloat16* __restrict__ O, const __
 
 
 template <int HD>
-int launch_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o, BwdParams p, cudaStream_t st) {
+int launch_bwd(const void* q, const void* k, const void* v, const long long* strides, const void* o, const void* d_o, BwdParams p, cudaStream_t st) {
   using SmemB = SmemBT<HD>;
   {
     const long long rows = static_cast<long long>(p.B) * p.S * p.Hq;
@@ -410,17 +415,13 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
                                                                           const_cast<float*>(p.delta), p.B, p.S, p.Hq);
   }
   CUtensorMap tmQ, tmK, tmV, tmDO;
-  const uint64_t rows = static_cast<uint64_t>(p.B) * p.S;
-  int rc = make_tmap_2d_bf16(&tmQ, q, rows, static_cast<uint64_t>(p.Hq) * HD, static_cast<uint64_t>(p.Hq) * HD, BM, 64);
+  const uint64_t wide = static_cast<uint64_t>(p.Hq) * HD, narrow = static_cast<uint64_t>(p.Hkv) * HD;
+  int rc = make_tmap_rows_bf16(&tmQ, q, p.B, p.S, wide, strides[1], strides[0], BM);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmDO, d_o, p.B, p.S, wide, wide, wide * p.S, BM);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmK, k, p.B, p.Sk, narrow, strides[3], strides[2], BN);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmV, v, p.B, p.Sk, narrow, strides[5], strides[4], BN);
   if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmDO, d_o, rows, static_cast<uint64_t>(p.Hq) * HD, static_cast<uint64_t>(p.Hq) * HD, BM, 64);
-  if (rc != kErrOk) return rc;
-  const uint64_t rows_k = static_cast<uint64_t>(p.B) * p.Sk;
-  rc = make_tmap_2d_bf16(&tmK, k, rows_k, static_cast<uint64_t>(p.Hkv) * HD, static_cast<uint64_t>(p.Hkv) * HD, BN, 64);
-  if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmV, v, rows_k, static_cast<uint64_t>(p.Hkv) * HD, static_cast<uint64_t>(p.Hkv) * HD, BN, 64);
-  if (rc != kErrOk) return rc;
-  dim3 grid(p.Sk / BN, p.B * p.Hkv);
+  dim3 grid((p.Sk + BN - 1) / BN, p.B * p.Hkv);
   const bool seg = p.q_seg != nullptr;
   const bool cap = p.soft_cap > 0.f;
 #define LVB_LAUNCH_BWD(SEG, CAP)                                                                                      \
@@ -447,20 +448,21 @@ int launch_bwd(const void* q, const void* k, const void* v, const void* o, const
 
 // Backward of lvb_flash_attn_fwd_hd.  dq32: fp32 [B,S,Hq,D], must be zero on entry.  delta: fp32 [B,Hq,S] scratch.  D = head_dim
 // is 64 or 128; causal and Sk (keys per sequence: k / v / dk / dv are [B, Sk, Hkv, D]) as in the forward.  ranges: of
-// lvb_segment_ranges, with segment ids.
-extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+// lvb_segment_ranges, with segment ids.  strides: (sequence, row) in elements of q, k, v, and of dk and dv.  Any S and Sk.
+extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v, const long long* strides, const void* o, const void* d_o,
                                      const float* lse2, float* delta, float* dq32, void* dk, void* dv, const int* q_seg,
                                      const int* k_seg, const void* ranges, int B, int S, int Sk, int Hq, int Hkv, int head_dim, int causal, float scale,
                                      float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fa;
-  if (B <= 0 || S <= 0 || (S % BM) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
+  if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
   if (!causal && window != 0) return kErrBadArg;
-  if (Sk <= 0 || (Sk % BN) != 0 || (causal && Sk != S)) return kErrBadArg;
+  if (Sk <= 0 || (causal && Sk != S) || ((strides[6] | strides[7]) & 7)) return kErrBadArg;
   BwdParams p;
   p.dQ32 = dq32;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
+  p.ldk_batch = strides[6]; p.ldk = strides[7];
   p.lse2 = lse2;
   p.delta = delta;
   p.q_seg = q_seg;
@@ -471,16 +473,7 @@ extern "C" int lvb_flash_attn_bwd_hd(const void* q, const void* k, const void* v
   p.causal = causal ? 1 : 0;
   p.status = status;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (head_dim == 128) return launch_bwd<128>(q, k, v, o, d_o, p, st);
-  if (head_dim == 64) return launch_bwd<64>(q, k, v, o, d_o, p, st);
+  if (head_dim == 128) return launch_bwd<128>(q, k, v, strides, o, d_o, p, st);
+  if (head_dim == 64) return launch_bwd<64>(q, k, v, strides, o, d_o, p, st);
   return kErrBadArg;
-}
-
-// Causal, head_dim 128 (the original entry point).
-extern "C" int lvb_flash_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* d_o,
-                                  const float* lse2, float* delta, float* dq32, void* dk, void* dv, const int* q_seg,
-                                  const int* k_seg, const void* ranges, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
-                                  int window, int* status, void* stream) {
-  return lvb_flash_attn_bwd_hd(q, k, v, o, d_o, lse2, delta, dq32, dk, dv, q_seg, k_seg, ranges, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window,
-                               status, stream);
 }

@@ -42,8 +42,9 @@ constexpr int kThreads = 320;           // warp0 TMA, warp1 MMA, warps 2-5 warpg
 
 struct Params {
   float* dQ32;         // [B, S, Hq, D] fp32, zero-initialised by the caller
-  __nv_bfloat16* dK;   // [B, S, Hkv, D]
-  __nv_bfloat16* dV;   // [B, S, Hkv, D]
+  __nv_bfloat16* dK;   // [B, S, Hkv, D], element strides ldk_batch and ldk of sequences and rows
+  __nv_bfloat16* dV;   // the same
+  long long ldk_batch, ldk;
   const float* lse2;   // [B, Hq, S]
   const float* delta;  // [B, Hq, S]
   const int* q_seg;
@@ -118,7 +119,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int nqb = p.S / BQ;
+  const int nqb = (p.S + BQ - 1) / BQ, blocks = (p.S + BKEYS - 1) / BKEYS;
   const int jb = blockIdx.x;
   const int b = blockIdx.y / p.Hkv;
   const int hkv = blockIdx.y % p.Hkv;
@@ -133,8 +134,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last block of 128 queries that can see one
   if constexpr (kSeg) {
     if (warp == 2) {
-      const uint2 own = __ldg(p.ranges + p.B * (p.S / BKEYS) + b * (p.S / BKEYS) + jb);
-      const int2 m = seg::meeting_blocks(p.ranges + b * (p.S / BKEYS), own, ilo * BQ / BKEYS, ihi * BQ / BKEYS, lane);
+      const uint2 own = __ldg(p.ranges + p.B * blocks + b * blocks + jb);
+      const int2 m = seg::meeting_blocks(p.ranges + b * blocks, own, ilo * BQ / BKEYS, ihi * BQ / BKEYS, lane);
       if (lane == 0) {  // at least one, so that dK and dV are written
         bounds[0] = m.x <= m.y ? m.x : jb;
         bounds[1] = m.x <= m.y ? m.y : jb;
@@ -171,7 +172,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t tmem_base = *tmem_holder;
   if constexpr (kSeg) {
     ilo = max(ilo, bounds[0] * (BKEYS / BQ));
-    ihi = min(ihi, bounds[1] * (BKEYS / BQ) + BKEYS / BQ - 1);
+    ihi = max(ilo, min(ihi, bounds[1] * (BKEYS / BQ) + BKEYS / BQ - 1));
   }
   const int nq = ihi - ilo + 1;
   const int iters = nq * G;
@@ -182,28 +183,27 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      const int row_k = b * p.S + k0;
       mbar_expect_tx(kv_full, 2 * kKVTile);
-      tma_load_2d(smem + Smem::kK, &tmK, kv_full, hkv * D, row_k);
-      tma_load_2d(smem + Smem::kK + kKVChunk, &tmK, kv_full, hkv * D + 64, row_k);
-      tma_load_2d(smem + Smem::kV, &tmV, kv_full, hkv * D, row_k);
-      tma_load_2d(smem + Smem::kV + kKVChunk, &tmV, kv_full, hkv * D + 64, row_k);
+      tma_load_3d(smem + Smem::kK, &tmK, kv_full, hkv * D, k0, b);
+      tma_load_3d(smem + Smem::kK + kKVChunk, &tmK, kv_full, hkv * D + 64, k0, b);
+      tma_load_3d(smem + Smem::kV, &tmV, kv_full, hkv * D, k0, b);
+      tma_load_3d(smem + Smem::kV + kKVChunk, &tmV, kv_full, hkv * D + 64, k0, b);
       bool ok = true;
       for (int t = 0; t < iters && ok; ++t) {
         const int g = t / nq;
         const int i = ilo + (t % nq);
         const int h = hkv * G + g;
-        const int row_q = b * p.S + i * BQ;
+        const int row_q = i * BQ;
         const int bf = t & 1;
         ok = mbar_wait(&qdo_empty[bf], ((t >> 1) & 1) ^ 1, abort_flag, p.status, 900, t);
         if (!ok) break;
         uint8_t* sq = smem + Smem::kQ + bf * (2 * kQTile);
         uint8_t* sdo = sq + kQTile;
         mbar_expect_tx(&qdo_full[bf], 2 * kQTile);
-        tma_load_2d(sq, &tmQ, &qdo_full[bf], h * D, row_q);
-        tma_load_2d(sq + kQChunk, &tmQ, &qdo_full[bf], h * D + 64, row_q);
-        tma_load_2d(sdo, &tmDO, &qdo_full[bf], h * D, row_q);
-        tma_load_2d(sdo + kQChunk, &tmDO, &qdo_full[bf], h * D + 64, row_q);
+        tma_load_3d(sq, &tmQ, &qdo_full[bf], h * D, row_q, b);
+        tma_load_3d(sq + kQChunk, &tmQ, &qdo_full[bf], h * D + 64, row_q, b);
+        tma_load_3d(sdo, &tmDO, &qdo_full[bf], h * D, row_q, b);
+        tma_load_3d(sdo + kQChunk, &tmDO, &qdo_full[bf], h * D + 64, row_q, b);
       }
     }
   } else if (warp == 1) {
@@ -278,7 +278,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
     const float scale_log2 = p.scale * 1.4426950408889634f;
     const int kj = k0 + r;
-    const int my_kseg = kSeg ? p.k_seg[b * p.S + kj] : 0;
+    const int my_kseg = kSeg ? p.k_seg[b * p.S + min(kj, p.S - 1)] : 0;
     float* s_lse = reinterpret_cast<float*>(smem + Smem::kStat + wg * (2 * 64 * 4));
     float* s_dlt = s_lse + 64;
     uint8_t* sPT = smem + Smem::kP + wg * (2 * kPTile);
@@ -294,10 +294,12 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int hh = hkv * G + tt / nq;
       const int qq = (ilo + (tt % nq)) * BQ;
       const size_t stat = (static_cast<size_t>(b) * p.Hq + hh) * p.S + qq;
-      pre_stat = (wtid < 64) ? p.lse2[stat + wtid] : p.delta[stat + wtid - 64];
+      // rows past the end: probabilities of 2^-inf, and their queries and gradients are zeros
+      const bool inside = qq + (wtid & 63) < p.S;
+      pre_stat = (wtid < 64) ? (inside ? p.lse2[stat + wtid] : INFINITY) : inside ? p.delta[stat + wtid - 64] : 0.f;
       if constexpr (kSeg) {
-        ids[0] = __ldg(p.q_seg + b * p.S + qq + lane);
-        ids[1] = __ldg(p.q_seg + b * p.S + qq + 32 + lane);
+        ids[0] = __ldg(p.q_seg + b * p.S + min(qq + lane, p.S - 1));
+        ids[1] = __ldg(p.q_seg + b * p.S + min(qq + 32 + lane, p.S - 1));
       }
     };
     fetch_stats(wg);
@@ -402,9 +404,9 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       wg_bar_sync(wg);
       if (ok && wtid == 0) {
         // dQ[b, q0 .. q0 + 63, h, :] += tile, one bulk tensor reduction
-        asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+        asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                          reinterpret_cast<uint64_t>(&tmDQ)),
-                     "r"(smem_u32(sPT)), "r"(h * D), "r"(b * p.S + q0)
+                     "r"(smem_u32(sPT)), "r"(h * D), "r"(q0), "r"(b)
                      : "memory");
         bulk_commit();  // waited for (read side) at the top of this warpgroup's next step
       }
@@ -421,7 +423,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (ok) {
       tc_fence_after();
       const int cbase = wg * 64;
-      const size_t row = (static_cast<size_t>(b) * p.S + k0 + r) * (static_cast<size_t>(p.Hkv) * D) + static_cast<size_t>(hkv) * D;
+      const bool inside = kj < p.S;
+      const size_t row = b * p.ldk_batch + (k0 + r) * p.ldk + static_cast<size_t>(hkv) * D;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
         __nv_bfloat16* dst = (which == 0 ? p.dV : p.dK) + row;
@@ -431,6 +434,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           uint32_t v[32];
           tmem_ld_32x32(src + c, v);
           tmem_ld_wait();
+          if (!inside) continue;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             uint4 w;
@@ -457,13 +461,13 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }  // namespace lvb
 
 // Backward of lvb_flash_attn_fwd, pipelined form (arguments of lvb_flash_attn_bwd, whose ranges come from lvb_segment_ranges).  dq32: fp32 [B,S,Hq,128], must be
-// zero on entry.  delta: fp32 [B,Hq,S] scratch.
-extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse2,
+// zero on entry.  delta: fp32 [B,Hq,S] scratch.  strides: (sequence, row) in elements of q, k, v, and of dk and dv.  Any S.
+extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, const long long* strides, const void* o, const void* d_o, const float* lse2,
                                    float* delta, float* dq32, void* dk, void* dv, const int* q_seg, const int* k_seg, const void* ranges, int B, int S,
                                    int Hq, int Hkv, float scale, float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fab2;
-  if (B <= 0 || S <= 0 || (S % BKEYS) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
+  if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0 || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   {
     const long long rows = static_cast<long long>(B) * S * Hq;
@@ -473,26 +477,25 @@ extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, 
                                                                 reinterpret_cast<const __nv_bfloat16*>(d_o), delta, B, S, Hq);
   }
   CUtensorMap tmQ, tmK, tmV, tmDO;
-  const uint64_t rows = static_cast<uint64_t>(B) * S;
-  int rc = make_tmap_2d_bf16(&tmQ, q, rows, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(Hq) * D, BQ, 64);
+  const uint64_t wide = static_cast<uint64_t>(Hq) * D, narrow = static_cast<uint64_t>(Hkv) * D;
+  int rc = make_tmap_rows_bf16(&tmQ, q, B, S, wide, strides[1], strides[0], BQ);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmDO, d_o, B, S, wide, wide, wide * S, BQ);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmK, k, B, S, narrow, strides[3], strides[2], BKEYS);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmV, v, B, S, narrow, strides[5], strides[4], BKEYS);
   if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmDO, d_o, rows, static_cast<uint64_t>(Hq) * D, static_cast<uint64_t>(Hq) * D, BQ, 64);
-  if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmK, k, rows, static_cast<uint64_t>(Hkv) * D, static_cast<uint64_t>(Hkv) * D, BKEYS, 64);
-  if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmV, v, rows, static_cast<uint64_t>(Hkv) * D, static_cast<uint64_t>(Hkv) * D, BKEYS, 64);
-  if (rc != kErrOk) return rc;
-  // dQ accumulator as a [B * S, Hq * D] fp32 matrix, box [64 rows, 128 columns], no swizzle (the shared-memory tile is row-major)
+  if ((strides[6] | strides[7]) & 7) return kErrBadArg;
+  // dQ accumulator as [B, S, Hq * D] fp32, box [64 rows of a sequence, 128 columns], no swizzle (the shared-memory tile is row-major); rows past a
+  // sequence's end are not written
   CUtensorMap tmDQ;
   {
     EncodeTiledFn enc = get_encode_tiled();
     if (enc == nullptr) return kErrTensorMap;
     if ((reinterpret_cast<uintptr_t>(dq32) & 15) != 0) return kErrBadArg;
-    cuuint64_t gdim[2] = {static_cast<cuuint64_t>(Hq) * D, rows};
-    cuuint64_t gstr[1] = {static_cast<cuuint64_t>(Hq) * D * 4};
-    cuuint32_t box[2] = {static_cast<cuuint32_t>(D), static_cast<cuuint32_t>(BQ)};
-    cuuint32_t estr[2] = {1, 1};
-    if (enc(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, dq32, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+    cuuint64_t gdim[3] = {wide, static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(B)};
+    cuuint64_t gstr[2] = {wide * 4, wide * 4 * S};
+    cuuint32_t box[3] = {static_cast<cuuint32_t>(D), static_cast<cuuint32_t>(BQ), 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    if (enc(&tmDQ, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, dq32, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return kErrTensorMap;
   }
@@ -500,6 +503,7 @@ extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, 
   p.dQ32 = dq32;
   p.dK = reinterpret_cast<__nv_bfloat16*>(dk);
   p.dV = reinterpret_cast<__nv_bfloat16*>(dv);
+  p.ldk_batch = strides[6]; p.ldk = strides[7];
   p.lse2 = lse2;
   p.delta = delta;
   p.q_seg = q_seg;
@@ -508,7 +512,7 @@ extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, 
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   p.scale = scale; p.soft_cap = soft_cap; p.window = window;
   p.status = status;
-  dim3 grid(S / BKEYS, B * Hkv);
+  dim3 grid((S + BKEYS - 1) / BKEYS, B * Hkv);
   const bool seg = q_seg != nullptr;
   const bool cap = soft_cap > 0.f;
 #define LVB_LAUNCH_BWD2(SEG, CAP)                                                                                    \

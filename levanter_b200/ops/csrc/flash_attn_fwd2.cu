@@ -1,4 +1,5 @@
-// Flash attention forward, two query tiles per CTA (sequence length a multiple of 256, head_dim 128).
+// Flash attention forward, two query tiles per CTA (head_dim 64 or 128, sequences of any length: rows past a sequence's end arrive as zeros and
+// are not stored).
 //
 // Compared with the one-tile kernel in flash_attn.cu this variant
 //   * keeps two 128-row query tiles A and B per CTA, so every K/V tile fetched by TMA is used twice and
@@ -42,7 +43,7 @@ struct Params {
   float* lse2;
   const int* q_seg;
   const int* k_seg;
-  const uint2* ranges;   // with segment ids: (lowest, highest) id per 128 rows, [B, S / 128] of the queries, then [B, Sk / 128] of the keys
+  const uint2* ranges;   // with segment ids: (lowest, highest) id per 128 rows, [B, blocks of S] of the queries, then [B, blocks of Sk] of the keys
   const float* sink;     // optional [Hq]: a learned logit per head that takes part in the softmax denominator only
   int B, S, Hq, Hkv;  // S: query positions per sequence
   int Sk;             // key positions per sequence (= S unless the mask has no causal part: cross attention)
@@ -139,7 +140,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int ncta = p.S / kRows;
+  const int ncta = (p.S + kRows - 1) / kRows;
+  const int q_blocks = (p.S + BT - 1) / BT, k_blocks = (p.Sk + BT - 1) / BT;
   const int cb = ncta - 1 - static_cast<int>(blockIdx.x);  // heaviest first
   const int b = blockIdx.y / p.Hq;
   const int h = blockIdx.y % p.Hq;
@@ -153,13 +155,13 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     jlo = first_key > 0 ? first_key / BT : 0;
   }
   if constexpr (kPacked) jlo = row_lower_bound(p, q0) / BT;  // bounds do not decrease along the packed rows
-  int jend = causal ? jdiagB : p.Sk / BT - 1;
+  int jend = causal ? min(jdiagB, k_blocks - 1) : k_blocks - 1;  // (tile B may lie past the end)
   volatile int* bounds = reinterpret_cast<volatile int*>(tmem_holder + 2);  // kSeg: first and last key block that these rows can see
   if constexpr (kSeg) {
     if (warp == 2) {
-      const uint2* own = p.ranges + b * (p.S / BT) + 2 * cb;
-      const uint2 ra = __ldg(own), rb = __ldg(own + 1);
-      const int2 m = seg::meeting_blocks(p.ranges + p.B * (p.S / BT) + b * (p.Sk / BT), make_uint2(min(ra.x, rb.x), max(ra.y, rb.y)), jlo, jend, lane);
+      const uint2* own = p.ranges + b * q_blocks + 2 * cb;
+      const uint2 ra = __ldg(own), rb = 2 * cb + 1 < q_blocks ? __ldg(own + 1) : ra;
+      const int2 m = seg::meeting_blocks(p.ranges + p.B * q_blocks + b * k_blocks, make_uint2(min(ra.x, rb.x), max(ra.y, rb.y)), jlo, jend, lane);
       if (lane == 0) {  // at least one block (and the diagonal ones), so that rows that see nothing are written too
         bounds[0] = min(m.x, causal ? jdiagA : jend);
         bounds[1] = max(m.y, jlo);
@@ -201,12 +203,12 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (!causal) jend = max(bounds[1], jlo);
   }
   const int nB = jend - jlo + 1;                  // blocks processed by tile B
-  const int nA = causal && !kMaps ? nB - 1 : nB;  // causal: tile A stops one block earlier (its diagonal)
+  const int nA = causal && !kMaps ? min(jdiagA, jend) - jlo + 1 : nB;  // causal: tile A stops at its diagonal, one block earlier
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      const int row_q = b * p.S + q0;
+      const int row_q = q0;
       const int ck = kPacked ? (p.dk + 63) / 64 : HDK / 64, cv = kPacked ? (p.dv + 63) / 64 : HDV / 64;  // 64-column chunks
       mbar_expect_tx(q_full, 2 * ck * kChunkBytes);
 #pragma unroll
@@ -216,10 +218,10 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           if constexpr (kPacked) {
             if (c < ck) tma_load_3d(smem + Smem::kQ + t * kQKTile + c * kChunkBytes, &tmQ, q_full, 64 * c, kMaps ? 2 * h + t : h, kMaps ? row_q : row_q + t * BT);
           } else
-          tma_load_2d(smem + Smem::kQ + t * kQKTile + c * kChunkBytes, &tmQ, q_full, h * HDK + 64 * c, row_q + t * BT);
+          tma_load_3d(smem + Smem::kQ + t * kQKTile + c * kChunkBytes, &tmQ, q_full, h * HDK + 64 * c, row_q + t * BT, b);
       bool ok = true;
       for (int it = 0; it < nB && ok; ++it) {
-        const int row_k = b * p.Sk + (jlo + it) * BT;
+        const int row_k = (jlo + it) * BT;
 #pragma unroll
         for (int t = 0; t < (kMaps ? 2 : 1); ++t) {
           const int n = kMaps ? 2 * it + t : it, st = n % kKStages;
@@ -232,7 +234,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             if constexpr (kPacked) {
               if (c < ck) tma_load_3d(ks + c * kChunkBytes, &tmK, &k_full[st], 64 * c, kMaps ? 2 * hkv + t : hkv, row_k);
             } else
-            tma_load_2d(ks + c * kChunkBytes, &tmK, &k_full[st], hkv * HDK + 64 * c, row_k);
+            tma_load_3d(ks + c * kChunkBytes, &tmK, &k_full[st], hkv * HDK + 64 * c, row_k, b);
         }
         if (!ok) break;
         const int sv = it % kVStages;
@@ -245,7 +247,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           if constexpr (kPacked) {
             if (c < cv) tma_load_3d(vs + c * kChunkBytes, &tmV, &v_full[sv], 64 * c, hkv, row_k);
           } else
-          tma_load_2d(vs + c * kChunkBytes, &tmV, &v_full[sv], hkv * HDV + 64 * c, row_k);
+          tma_load_3d(vs + c * kChunkBytes, &tmV, &v_full[sv], hkv * HDV + 64 * c, row_k, b);
       }
     }
   } else if (warp == 1) {
@@ -342,7 +344,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const uint32_t tO = tmem_base + 2 * BT + tile * HDV + lane_addr;
     const float scale_log2 = p.scale * kLog2e;
     const float cap_inv = kCap ? __fdividef(p.scale, p.soft_cap) : 0.f;
-    const int my_seg = kSeg ? p.q_seg[b * p.S + qi] : 0;
+    const int my_seg = kSeg ? p.q_seg[b * p.S + min(qi, p.S - 1)] : 0;
     const int* kseg_row = kSeg ? p.k_seg + b * p.Sk : nullptr;
     float m_used = -INFINITY, l_sum = 0.f;
     bool ok = true;
@@ -358,7 +360,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       int ids[4] = {0, 0, 0, 0};
       if constexpr (kSeg) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ids[i] = __ldg(kseg_row + k0 + 32 * i + lane);
+        for (int i = 0; i < 4; ++i) ids[i] = __ldg(kseg_row + min(k0 + 32 * i + lane, p.Sk - 1));
       }
       ok = mbar_wait(&s_full[tile], it & 1, abort_flag, p.status, 1400 + tile, it);
       ok = __all_sync(0xffffffffu, ok);
@@ -367,13 +369,15 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       bool need_mask = (j == jdiag) || (kPacked && k0 < tile_lo) || (!kPacked && p.window > 0 && k0 <= q0 + tile * BT + BT - 1 - p.window);
       // what the row sees of the block: columns col_lo .. col_lo + col_span (with segment ids: those of its segment, a bit per column)
       const int col_lo = (kPacked ? row_lo : p.window > 0 ? qi - p.window + 1 : 0) - k0;
-      const unsigned col_span = causal ? static_cast<unsigned>(qi - k0 - col_lo) : 0x7fffffffu;
+      const int col_hi = causal ? qi - k0 : p.Sk - 1 - k0;  // (a causal row past the keys' end is past the rows' end too)
+      const unsigned col_span = static_cast<unsigned>(col_hi - col_lo);
+      if (!kPacked && !causal && k0 + BT > p.Sk) need_mask = true;
       uint32_t visible[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
       if constexpr (kSeg) {
         need_mask = !seg::same_segment<4>(my_seg, ids, visible) || need_mask;
         if (need_mask) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) visible[i] &= seg::bit_range(col_lo - 32 * i, (causal ? qi - k0 : BT) - 32 * i);
+          for (int i = 0; i < 4; ++i) visible[i] &= seg::bit_range(col_lo - 32 * i, col_hi - 32 * i);
         }
       }
       auto mask = [&](uint32_t (&v)[2][32], int c) {
@@ -587,12 +591,14 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             if (c + 8 * q4 < p.dv) store_row_piece(orow + c + 8 * q4, e + 8 * q4, f, grow != nullptr ? grow + c + 8 * q4 : nullptr);
         }
       } else {
+      const bool inside = qi < p.S;
       __nv_bfloat16* orow = p.O + (static_cast<size_t>(b) * p.S + qi) * (static_cast<size_t>(p.Hq) * HDV) + static_cast<size_t>(h) * HDV;
 #pragma unroll 1
       for (int c = 0; c < HDV; c += 32) {
         uint32_t v[32];
         tmem_ld_32x32(tO + c, v);
         tmem_ld_wait();
+        if (!inside) continue;
 #pragma unroll
         for (int q4 = 0; q4 < 4; ++q4) {
           uint4 w;
@@ -603,7 +609,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           reinterpret_cast<uint4*>(orow + c)[q4] = w;
         }
       }
-      p.lse2[(static_cast<size_t>(b) * p.Hq + h) * p.S + qi] = (l_sum > 0.f) ? m_used + log2f(l_sum) : -INFINITY;
+      if (inside) p.lse2[(static_cast<size_t>(b) * p.Hq + h) * p.S + qi] = (l_sum > 0.f) ? m_used + log2f(l_sum) : -INFINITY;
       }
     }
     }
@@ -627,7 +633,8 @@ int launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tm
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::kTotal) != cudaSuccess) return kErrCuda;
     attr_set = true;
   }
-  dim3 grid(p.S / (kMaps ? BT : 2 * BT), p.B * p.Hq);
+  constexpr int rows = kMaps ? BT : 2 * BT;
+  dim3 grid((p.S + rows - 1) / rows, p.B * p.Hq);
   kern<<<grid, kThreads, Smem::kTotal, st>>>(tmQ, tmK, tmV, p);
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }
@@ -638,15 +645,11 @@ int launch(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tm
 namespace lvb {
 namespace fa2 {
 template <int HD>
-int launch_hd(const void* q, const void* k, const void* v, const Params& p, cudaStream_t st) {
+int launch_hd(const void* q, const void* k, const void* v, const long long* strides, const Params& p, cudaStream_t st) {
   CUtensorMap tmQ, tmK, tmV;
-  const uint64_t rows = static_cast<uint64_t>(p.B) * p.S;
-  int rc = make_tmap_2d_bf16(&tmQ, q, rows, static_cast<uint64_t>(p.Hq) * HD, static_cast<uint64_t>(p.Hq) * HD, BT, 64);
-  if (rc != kErrOk) return rc;
-  const uint64_t rows_k = static_cast<uint64_t>(p.B) * p.Sk;
-  rc = make_tmap_2d_bf16(&tmK, k, rows_k, static_cast<uint64_t>(p.Hkv) * HD, static_cast<uint64_t>(p.Hkv) * HD, BT, 64);
-  if (rc != kErrOk) return rc;
-  rc = make_tmap_2d_bf16(&tmV, v, rows_k, static_cast<uint64_t>(p.Hkv) * HD, static_cast<uint64_t>(p.Hkv) * HD, BT, 64);
+  int rc = make_tmap_rows_bf16(&tmQ, q, p.B, p.S, static_cast<uint64_t>(p.Hq) * HD, strides[1], strides[0], BT);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmK, k, p.B, p.Sk, static_cast<uint64_t>(p.Hkv) * HD, strides[3], strides[2], BT);
+  if (rc == kErrOk) rc = make_tmap_rows_bf16(&tmV, v, p.B, p.Sk, static_cast<uint64_t>(p.Hkv) * HD, strides[5], strides[4], BT);
   if (rc != kErrOk) return rc;
   const bool seg = p.q_seg != nullptr;
   const bool cap = p.soft_cap > 0.f;
@@ -660,47 +663,52 @@ int launch_hd(const void* q, const void* k, const void* v, const Params& p, cuda
 
 namespace lvb {
 namespace seg {
-// ranges[i] = (lowest, highest) of the ids of block i; blocks [0, nq) are q_seg's, the following ones k_seg's
-__global__ void block_ranges_kernel(const int* __restrict__ q_seg, const int* __restrict__ k_seg, uint2* __restrict__ ranges, int nq, int n) {
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// ranges[i] = (lowest, highest) of the ids of block i: q_seg's blocks, sequence by sequence, and then k_seg's
+__global__ void block_ranges_kernel(const int* __restrict__ q_seg, const int* __restrict__ k_seg, uint2* __restrict__ ranges, int B, int S, int Sk) {
+  int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (i >= n) return;
-  const int* src = i < nq ? q_seg + static_cast<long long>(i) * kBlock : k_seg + static_cast<long long>(i - nq) * kBlock;
+  const int nq = (S + kBlock - 1) / kBlock, nk = (Sk + kBlock - 1) / kBlock;
+  if (i >= B * (nq + nk)) return;
+  uint2* out = ranges + i;
+  const bool keys = i >= B * nq;
+  if (keys) i -= B * nq;
+  const int n = keys ? nk : nq, len = keys ? Sk : S;
+  const int* src = (keys ? k_seg : q_seg) + static_cast<long long>(i / n) * len;
   uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll
   for (int t = 0; t < kBlock / 32; ++t) {
-    const uint32_t v = static_cast<uint32_t>(__ldg(src + 32 * t + lane));
+    const uint32_t v = static_cast<uint32_t>(__ldg(src + min(i % n * kBlock + 32 * t + lane, len - 1)));
     lo = min(lo, v);
     hi = max(hi, v);
   }
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
-  if (lane == 0) ranges[i] = make_uint2(lo, hi);
+  if (lane == 0) *out = make_uint2(lo, hi);
 }
 }  // namespace seg
 }  // namespace lvb
 
-// ranges[0 .. B (S + Sk) / 128): (lowest, highest) segment id, as unsigned numbers, per 128 rows of q_seg [B, S] and then of k_seg [B, Sk]
-// (S and Sk multiples of 128).
+// ranges: (lowest, highest) segment id, as unsigned numbers, per 128 rows of each sequence (the last block may be shorter) of q_seg [B, S] and then
+// of k_seg [B, Sk].
 extern "C" int lvb_segment_ranges(const int* q_seg, const int* k_seg, int B, int S, int Sk, void* ranges, void* stream) {
   using namespace lvb;
-  if (B <= 0 || S <= 0 || Sk <= 0 || (S % seg::kBlock) != 0 || (Sk % seg::kBlock) != 0 || q_seg == nullptr || k_seg == nullptr) return kErrBadArg;
-  const int nq = B * (S / seg::kBlock), n = nq + B * (Sk / seg::kBlock);
-  seg::block_ranges_kernel<<<(n + 3) / 4, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(q_seg, k_seg, reinterpret_cast<uint2*>(ranges), nq, n);
+  if (B <= 0 || S <= 0 || Sk <= 0 || q_seg == nullptr || k_seg == nullptr) return kErrBadArg;
+  const int n = B * ((S + seg::kBlock - 1) / seg::kBlock + (Sk + seg::kBlock - 1) / seg::kBlock);
+  seg::block_ranges_kernel<<<(n + 3) / 4, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(q_seg, k_seg, reinterpret_cast<uint2*>(ranges), B, S, Sk);
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }
 
-// Same contract as lvb_flash_attn_fwd_hd (head_dim 64 or 128, causal or not, optional sink logits [Hq]), but S must be a
-// multiple of 256: two query tiles per CTA.  Sk: keys per sequence, a multiple of 128 (k / v are [B, Sk, Hkv, D], k_seg [B, Sk]);
-// Sk must equal S when causal.  ranges: what lvb_segment_ranges makes of the segment ids.
-extern "C" int lvb_flash_attn_fwd2_hd(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
+// Same contract as lvb_flash_attn_fwd_hd (head_dim 64 or 128, causal or not, optional sink logits [Hq]) for sequences of any length S and Sk (Sk = S
+// when causal), two query tiles per CTA.  strides: (sequence, row) in elements of q, k and v, whose rows hold their heads side by side; multiples
+// of 8, the pointers 16-byte aligned.  o [B, S, Hq, D] and lse2 [B, Hq, S] are packed.  ranges: what lvb_segment_ranges makes of the segment ids.
+extern "C" int lvb_flash_attn_fwd2_hd(const void* q, const void* k, const void* v, const long long* strides, void* o, float* lse2, const int* q_seg,
                                       const int* k_seg, const void* ranges, const float* sink, int B, int S, int Sk, int Hq, int Hkv,
                                       int head_dim, int causal, float scale, float soft_cap, int window, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::fa2;
-  if (B <= 0 || S <= 0 || (S % (2 * BT)) != 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
+  if (B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || (Hq % Hkv) != 0) return kErrBadArg;
   if ((!causal && window != 0) || ((q_seg != nullptr) != (ranges != nullptr))) return kErrBadArg;
-  if (Sk <= 0 || (Sk % BT) != 0 || (causal && Sk != S)) return kErrBadArg;
+  if (Sk <= 0 || (causal && Sk != S)) return kErrBadArg;
   Params p;
   p.O = reinterpret_cast<__nv_bfloat16*>(o);
   p.lse2 = lse2;
@@ -715,16 +723,9 @@ extern "C" int lvb_flash_attn_fwd2_hd(const void* q, const void* k, const void* 
   p.pos = nullptr; p.chunk = 0; p.dk = p.dv = head_dim; p.gate = nullptr; p.ldg = 0; p.gate_per_head = 0;
   p.weight = nullptr; p.diff_scale = p.eps = 0.f;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (head_dim == 128) return launch_hd<128>(q, k, v, p, st);
-  if (head_dim == 64) return launch_hd<64>(q, k, v, p, st);
+  if (head_dim == 128) return launch_hd<128>(q, k, v, strides, p, st);
+  if (head_dim == 64) return launch_hd<64>(q, k, v, strides, p, st);
   return kErrBadArg;
-}
-
-// Causal, head_dim 128 (the original entry point).
-extern "C" int lvb_flash_attn_fwd2(const void* q, const void* k, const void* v, void* o, float* lse2, const int* q_seg,
-                                   const int* k_seg, const void* ranges, int B, int S, int Hq, int Hkv, float scale, float soft_cap,
-                                   int window, int* status, void* stream) {
-  return lvb_flash_attn_fwd2_hd(q, k, v, o, lse2, q_seg, k_seg, ranges, nullptr, B, S, S, Hq, Hkv, 128, 1, scale, soft_cap, window, status, stream);
 }
 
 // Causal attention over T packed rows (T a multiple of 256) of sequences that each start at position 0:

@@ -1,5 +1,5 @@
 """Flash attention on tcgen05 tensor cores (``csrc/flash_attn*.cu``): head sizes 64 and 128, causal (with sliding window) or
-not, GQA, segment ids, any sequence length (padded to a multiple of 128 behind a segment id of its own).
+not, GQA, segment ids, any sequence length.
 
 Replaces the reference's fused-attention call sites (TransformerEngine/cuDNN on GPU, src/levanter/layers/attention.py:
 533-544; pure-JAX flash attention, src/levanter/models/flash_attention.py:143-385)."""
@@ -99,3 +99,10 @@ def flash_attention(q, k, v, mask, *, logits_soft_cap: Optional[float] = None, s
     from ._flash_impl import flash_attention_cuda
 
     return flash_attention_cuda(q, k, v, mask, logits_soft_cap=logits_soft_cap, scaling_factor=scaling_factor, sink=sink)
+
+
+def flash_attention_joint(qkv, mask, *, scaling_factor: float):
+    """Attention of ``qkv [B, S, 3, H, D]``, the rows of a joint projection, for which :func:`supported` holds part by part -> ``[B, S, H, D]``."""
+    from ._flash_impl import flash_attention_joint_cuda
+
+    return flash_attention_joint_cuda(qkv, mask, scaling_factor=scaling_factor)

@@ -268,3 +268,47 @@ def test_blocks_of_other_segments_are_left_out(layout, D, causal, window):
     mask = (AttentionMask.causal(sliding_window=window) if causal else AttentionMask(is_causal=False)).with_segment_ids(seg)
     _run(2, S, 4, 2, mask, D=D, seed=3)
     _run(2, S, 2, 2, mask, D=D, seed=4, soft_cap=15.0)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("S,causal", [(2, True), (63, True), (129, False), (255, True), (257, True), (333, False), (333, True), (641, True)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_any_length_and_nothing_of_the_next_sequence(D, S, causal, masked):
+    """Tiles that end inside, at and past the sequence, against fp32; a second sequence of NaN behind the first one must not reach it."""
+    mask = AttentionMask.causal(sliding_window=100 if masked else None) if causal else AttentionMask(is_causal=False)
+    if masked and not causal:
+        mask = mask.with_segment_ids((torch.arange(S, device="cuda") // 50).int()[None].expand(2, S))
+    _run(2, S, 4, 2, mask, D=D, seed=S)
+    torch.manual_seed(S)
+    q, k, v, g = (torch.randn(2, S, 2, D, device="cuda").bfloat16() for _ in range(4))
+    results = []
+    for bad in (False, True):
+        args = [t.clone() for t in (q, k, v)]
+        if bad:
+            for t in args:
+                t[1] = float("nan")
+        args = [t.requires_grad_() for t in args]
+        o = flash_attention_cuda(*args, mask)
+        o.backward(g)
+        results.append([o[0]] + [t.grad[0] for t in args])
+    lib.check_status()
+    for a, b in zip(*results):
+        assert (a.float() - b.float()).abs().max() <= 2 ** -7 * b.float().abs().max()  # (sums over blocks in another order)
+
+
+@pytest.mark.parametrize("D,S,mask", [(64, 333, AttentionMask.causal()), (128, 256, AttentionMask.causal()), (64, 130, None)])
+def test_joint_rows_give_what_separate_ones_give(D, S, mask):
+    from levanter_b200.ops.flash_attention import flash_attention_joint
+
+    torch.manual_seed(2)
+    B, H = 2, 3
+    rows = torch.randn(B, S, 3 * H * D, device="cuda").bfloat16().requires_grad_()
+    g = torch.randn(B, S, H, D, device="cuda").bfloat16()
+    flash_attention_joint(rows.view(B, S, 3, H, D), mask, scaling_factor=0.07).backward(g)
+    joint, rows.grad = rows.grad, None
+    q, k, v = (t.contiguous() for t in rows.view(B, S, 3, H, D).unbind(2))
+    o = flash_attention_cuda(q, k, v, mask, scaling_factor=0.07)
+    o.backward(g)
+    with torch.no_grad():
+        assert torch.equal(flash_attention_joint(rows.view(B, S, 3, H, D), mask, scaling_factor=0.07), o)
+    assert (joint.float() - rows.grad.float()).norm() <= 2 ** -8 * rows.grad.float().norm()  # dq is summed by atomics
