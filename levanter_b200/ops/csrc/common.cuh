@@ -218,6 +218,18 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// ---------------------------------------------------------------- chained kernels (launch_chained)
+// Waits until the kernels before this one are done and their results are visible, and only then lets the next kernel of the chain start: what that
+// one may do ahead of its own wait then overlaps this kernel and no earlier one.  Ahead of the wait a kernel sets up its barriers and tensor
+// memory and may bring weights into the L2 (a hint, whoever wrote them last); it reads and writes nothing.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
+
 // ---------------------------------------------------------------- TMEM
 template <int kCols>
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_holder) {
@@ -457,6 +469,23 @@ inline void ensure_context_for(const void* /*ptr*/) {
     cudaFree(nullptr);
   }
   bound = true;
+}
+
+// Launch of a kernel of the serving chain: it may start while the kernel before it on the stream still runs, and every thread of it calls chain_wait()
+// before it touches global memory.  In a graph of some sixty kernels of 2 to 20 us the hand-over from one to the next costs over 1 us each.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 // Row-major 2-D bf16 tensor [rows, cols] with row stride ld (elements);

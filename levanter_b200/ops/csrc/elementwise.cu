@@ -94,6 +94,7 @@ __device__ __forceinline__ float act_bwd(float g, int act) {
 __global__ void glu_fwd_kernel(const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ up,
                                __nv_bfloat16* __restrict__ out, int rows, int cols, long long ldg, long long ldu,
                                long long ldo, int act) {
+  chain_wait();
   const int vec_per_row = cols >> 3;
   const long long total = static_cast<long long>(rows) * vec_per_row;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
@@ -176,10 +177,11 @@ extern "C" int lvb_glu_fwd(const void* gate, const void* up, void* out, int rows
   if (rows <= 0 || cols <= 0 || (cols & 7) || (ldg & 7) || (ldu & 7) || (ldo & 7)) return kErrBadArg;
   const long long total = static_cast<long long>(rows) * (cols >> 3);
   const int block = 256;
-  ew::glu_fwd_kernel<<<ew::grid_for(total, block), block, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(gate), reinterpret_cast<const __nv_bfloat16*>(up),
-      reinterpret_cast<__nv_bfloat16*>(out), rows, cols, ldg, ldu, ldo, act);
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  return launch_chained(ew::glu_fwd_kernel, ew::grid_for(total, block), block, 0, reinterpret_cast<cudaStream_t>(stream),
+                        reinterpret_cast<const __nv_bfloat16*>(gate), reinterpret_cast<const __nv_bfloat16*>(up),
+                        reinterpret_cast<__nv_bfloat16*>(out), rows, cols, ldg, ldu, ldo, act) == cudaSuccess
+             ? kErrOk
+             : kErrCuda;
 }
 
 extern "C" int lvb_glu_bwd(const void* dout, const void* gate, const void* up, void* dgate, void* dup, int rows,

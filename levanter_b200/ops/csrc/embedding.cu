@@ -13,6 +13,7 @@ namespace emb {
 // out[t, :] = weight[ids[t], :]; 16 bytes per thread and step.  Ids outside [0, vocab) leave a bounds code and a zero row.
 __global__ void embedding_fwd_kernel(const int* __restrict__ ids, const __nv_bfloat16* __restrict__ weight, __nv_bfloat16* __restrict__ out,
                                      int tokens, int dim, int vocab, int* status) {
+  chain_wait();
   const int vec = dim >> 3;
   for (int t = blockIdx.x; t < tokens; t += gridDim.x) {
     const int id = ids[t];
@@ -69,9 +70,10 @@ extern "C" int lvb_embedding_fwd(const int* ids, const void* weight, void* out, 
   if (tokens <= 0 || dim <= 0 || (dim & 7) || vocab <= 0) return kErrBadArg;
   const int threads = dim >= 2048 ? 256 : 128;
   int grid = tokens < 8 * num_sms() ? tokens : 8 * num_sms();
-  emb::embedding_fwd_kernel<<<grid, threads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      ids, reinterpret_cast<const __nv_bfloat16*>(weight), reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, vocab, status);
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  return launch_chained(emb::embedding_fwd_kernel, grid, threads, 0, reinterpret_cast<cudaStream_t>(stream), ids,
+                        reinterpret_cast<const __nv_bfloat16*>(weight), reinterpret_cast<__nv_bfloat16*>(out), tokens, dim, vocab, status) == cudaSuccess
+             ? kErrOk
+             : kErrCuda;
 }
 
 // grad[vocab, dim] (fp32) += scale * scatter(dy[tokens, dim] (bf16)) with the positions sorted by id (see the kernel).

@@ -105,6 +105,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if constexpr (!kGrouped) {
+    // B is a weight more often than not: the first ring of it is on its way to the L2 while the kernel before this one ends
+    if (warp == 0 && blockIdx.x < num_work && blockIdx.x % p.tiles_m == 0) {
+      const int u = blockIdx.x / p.tiles_m, kb0 = (u % p.splits) * p.kb_per_split;
+      if (lane < min(stages, min(k_blocks, kb0 + p.kb_per_split) - kb0)) tma_prefetch_2d(&tmB, (kb0 + lane) * BK, (u / p.splits) * BN);
+    }
+  }
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -311,6 +319,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 // out[m, n] = type(alpha * sum_s ws[s, m, n] + bias[n] + residual[m, n]); four columns per thread, slabs summed in order.
 __global__ void splitk_finalize_kernel(const float* __restrict__ ws, int splits, int M, int N, float alpha, int flags, const void* bias,
                                        const __nv_bfloat16* residual, int ldr, void* C, int ldc) {
+  chain_wait();
   const int n4 = N >> 2;
   const long long total = static_cast<long long>(M) * n4;
   const size_t slab = static_cast<size_t>(M) * N;
@@ -383,14 +392,8 @@ int launch(const void* A, const void* B, Params p, int lda, int ldb, cudaStream_
   }
   const int work = p.tiles_n * p.splits * p.tiles_m;
   const int grid = work < num_sms() ? work : num_sms();
-  kern<<<grid, kThreads, smem_bytes, stream>>>(tmA, tmB, p);
-  if (cudaGetLastError() != cudaSuccess) return kErrCuda;
-  if (p.splits > 1) {
-    const long long total = static_cast<long long>(p.M) * (p.N / 4);
-    const int blocks = static_cast<int>((total + 255) / 256 < 4LL * num_sms() ? (total + 255) / 256 : 4LL * num_sms());
-    splitk_finalize_kernel<<<blocks, 256, 0, stream>>>(p.ws, p.splits, p.M, p.N, p.alpha, p.flags, p.bias, p.residual, p.ldr, p.C, p.ldc);
-    if (cudaGetLastError() != cudaSuccess) return kErrCuda;
-  }
+  if (launch_chained(kern, grid, kThreads, smem_bytes, stream, tmA, tmB, p) != cudaSuccess) return kErrCuda;
+  if (p.splits > 1) return launch_splitk_finalize(p.ws, p.splits, p.M, p.N, p.alpha, p.flags, p.bias, p.residual, p.ldr, p.C, p.ldc, stream);
   return kErrOk;
 }
 
@@ -400,9 +403,10 @@ int launch_splitk_finalize(const float* ws, int splits, int M, int N, float alph
                            int ldr, void* C, int ldc, cudaStream_t stream) {
   const long long total = static_cast<long long>(M) * (N / 4);
   const int blocks = static_cast<int>((total + 255) / 256 < 4LL * num_sms() ? (total + 255) / 256 : 4LL * num_sms());
-  skinny::splitk_finalize_kernel<<<blocks, 256, 0, stream>>>(ws, splits, M, N, alpha, flags, bias,
-                                                             reinterpret_cast<const __nv_bfloat16*>(residual), ldr, C, ldc);
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  return launch_chained(skinny::splitk_finalize_kernel, blocks, 256, 0, stream, ws, splits, M, N, alpha, flags, bias,
+                        reinterpret_cast<const __nv_bfloat16*>(residual), ldr, C, ldc) == cudaSuccess
+             ? kErrOk
+             : kErrCuda;
 }
 }  // namespace lvb
 

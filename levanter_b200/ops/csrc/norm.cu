@@ -177,6 +177,7 @@ norm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __
                     const void* __restrict__ b, int wf32, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ h_out,
                     float* __restrict__ rstd_out, float* __restrict__ mean_out, int rows, int dim, float eps, float w_offset) {
   extern __shared__ float scratch[];
+  chain_wait();
   const int col = threadIdx.x * 8;
   const int row = blockIdx.x * blockDim.y + threadIdx.y;
   const bool active = row < rows && col < dim;  // the others take part in the sums
@@ -565,11 +566,8 @@ extern "C" int lvb_norm_fwd(const void* x, const void* residual, const void* w, 
     const int vpl = dim / 256;
     const bool by_warp = dim % 256 == 0 && (vpl == 1 || vpl == 2 || vpl == 4 || vpl == 8 || vpl == 16);
     if ((dim >> 3) <= TX && (!by_warp || rows <= kFewRows)) {
-      if (layer_norm)
-        norm_fwd_row_kernel<true><<<grid, block, smem, s>>>(X, R, w, b, w_is_f32, Y, H, rstd_out, mean_out, rows, dim, eps, w_offset);
-      else
-        norm_fwd_row_kernel<false><<<grid, block, smem, s>>>(X, R, w, b, w_is_f32, Y, H, rstd_out, mean_out, rows, dim, eps, w_offset);
-      return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+      auto kern = layer_norm ? norm_fwd_row_kernel<true> : norm_fwd_row_kernel<false>;
+      return launch_chained(kern, grid, block, smem, s, X, R, w, b, w_is_f32, Y, H, rstd_out, mean_out, rows, dim, eps, w_offset) == cudaSuccess ? kErrOk : kErrCuda;
     }
     if (by_warp) {
       const dim3 wgrid((rows + 3) / 4);

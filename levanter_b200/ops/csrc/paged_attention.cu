@@ -537,6 +537,7 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
   uint64_t* s_bar = reinterpret_cast<uint64_t*>(s_ml + 4 * 16 * 2);  // kExact: [4 warps][kMmaBufs], a stage's copies have landed
   volatile int* abort_flag = reinterpret_cast<volatile int*>(s_bar + 4 * kMmaBufs);
 
+  chain_wait();
   int seq = 0, ctx = 0;
   const bool live = locate_block<kThreads>(p, t, seq, ctx);
   const int k0 = (live ? first_key(p, ctx) : 0) + part * p.part;
@@ -848,6 +849,7 @@ __global__ void __launch_bounds__(kThreadsM) paged_merge_kernel(Params p) {
   const int D = p.dv;
   const int t = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  chain_wait();
   int seq = 0, ctx = 0;
   if (!locate_block<kThreadsM>(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
   const int np = (ctx - first_key(p, ctx) + p.part - 1) / p.part;
@@ -893,6 +895,7 @@ __global__ void __launch_bounds__(kThreadsM) paged_merge_maps_kernel(Params p) {
   constexpr int kPer = 256 / kThreadsM;  // output dimensions per thread, at most
   __shared__ float s_red[kThreadsM / 32];
   const int t = blockIdx.x, h = blockIdx.y;
+  chain_wait();
   int seq = 0, ctx = 0;
   if (!locate_block<kThreadsM>(p, t, seq, ctx)) return;  // zeros were written by the attention kernel
   const int np = (ctx - first_key(p, ctx) + p.part - 1) / p.part;
@@ -972,19 +975,14 @@ int launch_mma(const Params& p, cudaStream_t s) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) return kErrCuda;
     most = room;
   }
-  kern<<<dim3(p.T, p.KV, p.parts), kThreads, smem, s>>>(p);
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  return launch_chained(kern, dim3(p.T, p.KV, p.parts), kThreads, smem, s, p) == cudaSuccess ? kErrOk : kErrCuda;
 }
 
 int launch_merge(const Params& p, cudaStream_t s) {
-  if (p.parts > 1 && p.maps == 2) {
-    if (p.dv <= 128) paged_merge_maps_kernel<128><<<dim3(p.T, p.H / 2), 128, 0, s>>>(p);
-    else paged_merge_maps_kernel<256><<<dim3(p.T, p.H / 2), 256, 0, s>>>(p);
-  } else if (p.parts > 1) {
-    if (p.dv <= 128) paged_merge_kernel<128><<<dim3(p.T, p.H), 128, 0, s>>>(p);
-    else paged_merge_kernel<256><<<dim3(p.T, p.H), 256, 0, s>>>(p);
-  }
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  if (p.parts == 1) return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  const bool narrow = p.dv <= 128;
+  auto kern = p.maps == 2 ? (narrow ? paged_merge_maps_kernel<128> : paged_merge_maps_kernel<256>) : narrow ? paged_merge_kernel<128> : paged_merge_kernel<256>;
+  return launch_chained(kern, dim3(p.T, p.H / p.maps), narrow ? 128 : 256, 0, s, p) == cudaSuccess ? kErrOk : kErrCuda;
 }
 
 template <int D>

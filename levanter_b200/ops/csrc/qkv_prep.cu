@@ -161,6 +161,7 @@ struct QkvParams {
 template <typename T>
 __global__ void __launch_bounds__(kThreads) qkv_prep_kernel(QkvParams p) {
   extern __shared__ float s_angles[];
+  chain_wait();
   const int half = p.rot.inv_freq != nullptr ? p.rot.dims / 2 : 0;
   float* s_cos = s_angles;
   float* s_sin = s_angles + half;
@@ -398,9 +399,7 @@ extern "C" int lvb_qkv_prep(void* q, void* k, void* v, const void* v_first, cons
           aligned16(v) && aligned16(kv_pages) && groups_of_8(inv_freq, p.rot.dims, interleaved);
   const size_t smem = static_cast<size_t>(p.rot.dims) * 4;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (is_f32) qkv_prep_kernel<float><<<T, kThreads, smem, s>>>(p);
-  else qkv_prep_kernel<__nv_bfloat16><<<T, kThreads, smem, s>>>(p);
-  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+  return launch_chained(is_f32 ? qkv_prep_kernel<float> : qkv_prep_kernel<__nv_bfloat16>, T, kThreads, smem, s, p) == cudaSuccess ? kErrOk : kErrCuda;
 }
 
 // Latent attention.  Row t of down (stride ldd) holds `rank` compressed dimensions and a key part of rot_dims dimensions shared by the

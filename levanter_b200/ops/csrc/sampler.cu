@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const T* __restrict__ 
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
   const int parts = static_cast<int>(cluster.num_blocks()), part = static_cast<int>(cluster.block_rank());
+  chain_wait();
   const int row = blockIdx.x / parts;
   const T* z = logits + static_cast<long long>(row) * row_stride;
   const float t = temps[row];
@@ -164,12 +165,14 @@ int launch(const T* logits, long long row_stride, int rows, int vocab, const flo
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * parts);
   cfg.blockDim = dim3(kThreads);
   cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = parts;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, sample_kernel<T>, logits, row_stride, vocab, temps, seeds, tokens, logprobs) == cudaSuccess ? kErrOk : kErrCuda;
 }
 
