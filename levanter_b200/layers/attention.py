@@ -611,7 +611,7 @@ class Attention(nn.Module):
         prepared = self._prepared_for_pages(x, kv_cache)
         if prepared:
             # rotary positions and the cache write in one pass over the rows, which a decode step's joint projection leaves side by side
-            q, k, v = self._project_and_prepare(x, kv_cache, batch_info, pos_ids, joint=x.shape[0] <= DECODE_ROWS)
+            q, k, v = self._project_and_prepare(x, kv_cache, batch_info, pos_ids, decoding=seg is None)
         else:
             q, k, v = self._compute_qkv(x, pos_ids)
             kv_cache = kv_cache.update(batch_info, k, v)
@@ -645,15 +645,16 @@ class Attention(nn.Module):
                 and kv_cache.kv_pages.dtype == torch.bfloat16 and self.config.head_size in (64, 128) and self.local_heads // self.local_kv <= 16
                 and all(m.weight.dtype == torch.bfloat16 for m in self._projections() if type(m) is Linear))
 
-    def _project_and_prepare(self, x, kv_cache: "KvPageCache", batch_info, pos_ids, joint: bool):
-        """``q, k, v`` rows as attention reads them (slices of the joint product's rows with ``joint``), keys and values written to the pages."""
+    def _project_and_prepare(self, x, kv_cache: "KvPageCache", batch_info, pos_ids, decoding: bool):
+        """``q, k, v`` rows as attention reads them (for a few rows slices of the joint product's rows), keys and values written to the pages."""
         from ..ops import paged_attention as PA
         from ..ops.qkv_prep import prepare_qkv
         from ..ops.residual_stream import project
 
         D = self.config.head_size
         nq, nk = self.local_heads * D, self.local_kv * D
-        fused = self._fused_projection() if joint and self.q_norm is None else None
+        # the weights are laid out by the first decode step, not by a prompt that waits for its first token
+        fused = self._fused_projection(build=decoding) if x.shape[0] <= DECODE_ROWS and self.q_norm is None else None
         if fused is not None:
             y = project(x, fused[0], bias=fused[1])
             q, k, v = y[:, :nq].unflatten(1, (-1, D)), y[:, nq:nq + nk].unflatten(1, (-1, D)), y[:, nq + nk:nq + 2 * nk].unflatten(1, (-1, D))
@@ -664,7 +665,7 @@ class Attention(nn.Module):
         PA.kv_page_write_general(kv_cache.kv_pages, k, v, batch_info.new_token_dests)
         return q, k, v
 
-    def _fused_projection(self):
+    def _fused_projection(self, build: bool = True):
         """``(weight, bias or None)`` of the joint projection ``[q; k; v; gate]`` for serving: the projections read the same rows, so a
         decode step streams one matrix instead of launching four products.  None when a projection is wrapped (LoRA, fp8) or only
         some of q, k, v have a bias, and for a model in training.  (The gate per head has none: its rows of the bias are zeros.)"""
@@ -675,8 +676,8 @@ class Attention(nn.Module):
         biased = [m.bias is not None for m in with_bias]
         if any(biased) != all(biased):
             return None
-        w = self._rows.get([m.weight for m in mods])
-        b = self._bias_rows.get([m.bias for m in with_bias]) if w is not None and biased[0] else None
+        w = self._rows.get([m.weight for m in mods], build)
+        b = self._bias_rows.get([m.bias for m in with_bias], build) if w is not None and biased[0] else None
         return None if w is None or (biased[0] and b is None) else (w, b)
 
     def _paged_heads(self, x, kv_cache: "KvPageCache", batch_info, pos_ids, v_first: Optional[torch.Tensor] = None):
@@ -746,8 +747,8 @@ class Attention(nn.Module):
 
 # Rows up to which a serving step's projections that read the same rows are one product over their weights laid out side by side.  Such products
 # stream their weights, and each of them costs about 7 us beside that: 8 rows of a Llama 3 8B layer, three products 33 us and three sums of their
-# parts 7, one product 15 and 2 (a round of four such layers 827 -> 726 us).  Larger steps are bound by the tensor cores, and their rows go to kernels that want them packed.
-DECODE_ROWS = 128
+# parts 7, one product 15 and 2 (a round of four such layers 827 -> 726 us).  Larger steps are bound by the tensor cores.
+DECODE_ROWS = 256
 
 
 class AttentionWithSink(Attention):

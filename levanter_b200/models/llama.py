@@ -164,12 +164,12 @@ class LlamaMlp(nn.Module):
         self.act = activation if isinstance(activation, (ActivationFunctionEnum, ClampedGlu)) else ActivationFunctionEnum(activation)
         self._rows = FusedRows()
 
-    def _inner(self, x: torch.Tensor) -> torch.Tensor:
+    def _inner(self, x: torch.Tensor, build: bool = True) -> torch.Tensor:
         """The gated activation of packed rows; gate and up are one product when serving (no biases)."""
         mods = (self.gate_proj, self.up_proj)
         w = None
         if all(type(m) is Linear and m.bias is None for m in mods) and x.is_cuda and not self.training and not torch.is_grad_enabled():
-            w = self._rows.get([m.weight for m in mods])
+            w = self._rows.get([m.weight for m in mods], build)
         if w is not None:
             return glu_of_rows(project(x, w), self.gate_proj.weight.shape[0], self.act)
         return gated_activation(self.gate_proj(x), self.up_proj(x), self.act)
@@ -193,7 +193,7 @@ class LlamaMlp(nn.Module):
         if self.tp is not None and self.tp.size > 1:
             x = self.tp.copy_to_region(x)
         if x.dim() == 2 and x.shape[0] <= DECODE_ROWS and not torch.is_grad_enabled() and x.dtype == self.gate_proj.weight.dtype == torch.bfloat16:
-            h = self._inner(x)
+            h = self._inner(x, build=x.shape[0] <= 128)  # decode steps; a prompt's rows are a multiple of 256
         else:
             h = gated_activation(self.gate_proj(x), self.up_proj(x), self.act)
         if self.tp is not None and self.tp.size > 1:

@@ -78,14 +78,14 @@ class Linear(nn.Module):
 class FusedRows:
     """One matrix (or vector) whose row slices are the given parameters: projections that read the same rows become one product when
     a model serves, and nothing is stored twice.  :meth:`get` returns it, building it first when the parameters are not (or, after
-    a move or a conversion, no longer) its slices; None for parameters in training, which belong to the gradient engine's own
+    a move or a conversion, no longer) its slices (None there with ``build`` off); None for parameters in training, which belong to the gradient engine's own
     flat buffers.  ``pad``: zero rows at the end."""
 
     def __init__(self, pad: int = 0):
         self.pad = pad
         self._fused: Optional[torch.Tensor] = None
 
-    def get(self, params: Sequence[torch.Tensor]) -> Optional[torch.Tensor]:
+    def get(self, params: Sequence[torch.Tensor], build: bool = True) -> Optional[torch.Tensor]:
         if any(getattr(p, "main_grad", None) is not None or getattr(p, "grad_sink", None) is not None for p in params):
             return None
         fused = self._fused
@@ -97,6 +97,8 @@ class FusedRows:
                     break
                 at += p.numel() * p.element_size()
         if fused is None:
+            if not build:
+                return None
             if params[0].is_cuda and torch.cuda.is_current_stream_capturing():
                 return None  # the copy would be recorded and not made, and what follows would read the new rows
             rows = [p.detach() for p in params]

@@ -335,6 +335,16 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
   cluster_sync_all();  // the peer's barriers are initialised before anything is signalled on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
+  if constexpr (MODE == kPlain && !A_MN && !B_MN) {
+    // B is a weight more often than not: its first tiles are on their way to the L2 while the kernel before this one ends
+    if (warp == 0 && first_tile < num_work && p.k_wrap == 0) {
+      int mb, nb;
+      tile_coords(first_tile / splits, p.tiles_m, p.tiles_n, mb, nb);
+      const int kb0 = (first_tile % splits) * kbps;
+      if (mb == 0 && lane < min(kStages, min(k_blocks, kb0 + kbps) - kb0)) tma_prefetch_2d(&tmB, (kb0 + lane) * BK, nb * BN + static_cast<int>(cta) * BNH);
+    }
+  }
+  chain_wait();  // (returns at once in the forms that are not launched as part of a chain)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (one per CTA)
@@ -880,8 +890,7 @@ int launch_maps(const CUtensorMap& tmA, const CUtensorMap& tmB, Params p, cudaSt
   p.splits = (k_blocks + p.kb_per_split - 1) / p.kb_per_split;  // no empty split
   int pairs = tiles * p.splits;
   if (pairs > cap) pairs = cap;
-  kern<<<2 * pairs, kNumThreads, L::kTotal, stream>>>(tmA, tmB, p);
-  if (cudaGetLastError() != cudaSuccess) return kErrCuda;
+  if (launch_chained(kern, 2 * pairs, kNumThreads, L::kTotal, stream, tmA, tmB, p) != cudaSuccess) return kErrCuda;
   if (p.splits > 1)
     return launch_splitk_finalize(p.ws, p.splits, p.M, p.N, p.alpha, p.flags, p.bias, p.residual, p.ldr, p.C, p.ldc, stream);
   return kErrOk;

@@ -223,9 +223,9 @@ def test_paged_attention_partitions_of_every_length(D, KV, G, q_lens, kv_lens, p
 
 
 @pytest.mark.parametrize("heads,kv,hidden,bias", [(4, 2, 512, False), (8, 8, 512, False), (2, 1, 256, True)])
-@pytest.mark.parametrize("tokens", [3, 200])
+@pytest.mark.parametrize("tokens", [3, 200, 300])
 def test_plain_serving_step_prepares_rows_in_one_pass(heads, kv, hidden, bias, tokens, monkeypatch):
-    """Joint projections, rotation and cache write in one kernel (up to 128 rows), separate projections above: the same pages and heads as the
+    """Joint projections, rotation and cache write in one kernel (up to 256 rows), separate projections above: the same pages and heads as the
     separate kernels, up to the bf16 rounding of a sum whose parts were added in another order (2^-8 of a value)."""
     from levanter_b200.inference.page_table import PageTable
     from levanter_b200.layers.attention import Attention, AttentionConfig, KvPageCache
@@ -240,7 +240,7 @@ def test_plain_serving_step_prepares_rows_in_one_pass(heads, kv, hidden, bias, t
             m.bias.data.normal_(0, 0.1)
     seqs = 3
     lens = [tokens // seqs + (i < tokens % seqs) for i in range(seqs)]
-    table = PageTable.init(64, seqs, 16, 16)
+    table = PageTable.init(64, seqs, 16, 20)
     for s in range(seqs):
         table, _ = table.assign_seq_id_to_seq(s)
     slots = np.concatenate([np.full(n, s, np.int32) for s, n in enumerate(lens)])
