@@ -531,6 +531,49 @@ col_sum_kernel(const __nv_bfloat16* __restrict__ x, long long ld, float* __restr
   }
 }
 
+// dW[o, c] = sum over the rows of dy[r, o] x[r, c] for a few outputs o (a head's decay or gate, a router): a tensor-core tile would be one CTA that
+// walks all rows (8 outputs of 1024 columns over 16384 rows: 101 us), while reading x once takes 6.  A lane holds eight columns by eight outputs, a
+// block of eight warps 256 columns of its share of the rows; part[share][o][c] is summed by norm_bwd_reduce_kernel.  blockIdx.z: eight outputs.
+__global__ void __launch_bounds__(256)
+few_outputs_dw_kernel(const __nv_bfloat16* __restrict__ dy, long long ldy, const __nv_bfloat16* __restrict__ x, long long ldx, float* __restrict__ part,
+                      int rows, int outputs, int cols, int rows_per_share) {
+  __shared__ __align__(16) float sm[8][256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col = blockIdx.x * 256 + lane * 8, o0 = blockIdx.z * 8;
+  const int begin = blockIdx.y * rows_per_share, end = min(rows, begin + rows_per_share);
+  float acc[8][8];
+#pragma unroll
+  for (int o = 0; o < 8; ++o)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[o][j] = 0.f;
+  if (col < cols) {
+#pragma unroll 2
+    for (int r = begin + warp; r < end; r += 8) {
+      const Vec8 a = unpack8(__ldg(reinterpret_cast<const uint4*>(x + r * ldx + col)));
+      const Vec8 g = unpack8(__ldg(reinterpret_cast<const uint4*>(dy + r * ldy + o0)));
+#pragma unroll
+      for (int o = 0; o < 8; ++o)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[o][j] = fmaf(g.v[o], a.v[j], acc[o][j]);
+    }
+  }
+  const int c = blockIdx.x * 256 + threadIdx.x;
+#pragma unroll
+  for (int o = 0; o < 8; ++o) {
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 8; j += 4)
+      *reinterpret_cast<float4*>(&sm[warp][lane * 8 + j]) = make_float4(acc[o][j], acc[o][j + 1], acc[o][j + 2], acc[o][j + 3]);
+    __syncthreads();
+    if (c < cols) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) s += sm[w][threadIdx.x];
+      part[(static_cast<size_t>(blockIdx.y) * outputs + o0 + o) * cols + c] = s;
+    }
+  }
+}
+
 // TX threads per row: one vector each where 512 threads allow it, whole warps (or a power of two below one); TY rows per block of about 256
 inline void pick_block(int dim, int& TX, int& TY) {
   const int nvec = dim >> 3;
@@ -673,5 +716,30 @@ extern "C" int lvb_col_sum(const void* x, long long ld, void* out, int out_bf16,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   col_sum_kernel<<<dim3((cols + 255) / 256, shares), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), ld, scratch, rows, cols, per);
   norm_bwd_reduce_kernel<<<dim3((cols + 31) / 32, 1), 1024, 0, s>>>(scratch, nullptr, out, nullptr, out_bf16, shares, cols);
+  return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
+}
+
+// Shares of the rows that lvb_few_outputs_dw works on: about two blocks per SM, at least 64 rows each.
+extern "C" int lvb_few_outputs_dw_shares(int rows, int outputs, int cols) {
+  const int wanted = 2 * lvb::num_sms() / ((cols + 255) / 256 * (outputs / 8 > 0 ? outputs / 8 : 1)), most = (rows + 63) / 64;
+  return wanted < 1 ? 1 : wanted < most ? wanted : most;
+}
+
+// dw[outputs, cols] = dy[rows, outputs]^T x[rows, cols], fp32 sums stored as bf16 or fp32; outputs, cols and the row strides multiples of 8, the
+// pointers 16-byte aligned.  scratch: fp32 [lvb_few_outputs_dw_shares(...), outputs, cols].
+extern "C" int lvb_few_outputs_dw(const void* dy, long long ldy, const void* x, long long ldx, void* dw, int out_bf16, float* scratch, int rows, int outputs,
+                                  int cols, void* stream) {
+  using namespace lvb;
+  using namespace lvb::norm;
+  if (rows <= 0 || outputs <= 0 || cols <= 0 || ((outputs | cols | ldy | ldx) & 7) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy)) & 15))
+    return kErrBadArg;
+  int shares = lvb_few_outputs_dw_shares(rows, outputs, cols);
+  const int per = (rows + shares - 1) / shares;
+  shares = (rows + per - 1) / per;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  few_outputs_dw_kernel<<<dim3((cols + 255) / 256, shares, outputs / 8), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(dy), ldy,
+                                                                                     reinterpret_cast<const __nv_bfloat16*>(x), ldx, scratch, rows, outputs, cols, per);
+  const int dim = outputs * cols;
+  norm_bwd_reduce_kernel<<<dim3((dim + 31) / 32, 1), 1024, 0, s>>>(scratch, nullptr, dw, nullptr, out_bf16, shares, dim);
   return cudaGetLastError() == cudaSuccess ? kErrOk : kErrCuda;
 }

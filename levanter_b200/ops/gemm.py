@@ -312,10 +312,48 @@ def col_sum(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     return out
 
 
+_few_dw = None
+
+
+def few_outputs_dw(dy: torch.Tensor, x: torch.Tensor, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
+    """``dy^T x`` of rows ``dy [rows, outputs]`` and ``x [rows, cols]`` with few outputs and many rows, or None where the GEMM is the better form: from
+    1024 rows on and up to 32 outputs its one or two tiles leave the SMs idle."""
+    global _few_dw
+    (rows, outputs), cols = dy.shape, x.shape[1]
+    if not (outputs <= 32 and rows >= 1024 and x.is_cuda and lib.available() and outputs % 8 == 0 and cols % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32)
+            and dy.dtype == x.dtype == torch.bfloat16 and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (dy, x))):
+        return None
+    if _few_dw is None:
+        c = lib
+        _few_dw = (lib.fn("lvb_few_outputs_dw", [c.c_void_p, c.c_longlong] * 2 + [c.c_void_p, c.c_int, c.c_void_p] + [c.c_int] * 3 + [c.c_void_p], launches=2),
+                   lib.fn("lvb_few_outputs_dw_shares", [c.c_int] * 3, launches=0))
+    out = torch.empty(outputs, cols, dtype=out_dtype, device=x.device)
+    scratch = torch.empty(_few_dw[1](rows, outputs, cols) * outputs * cols, dtype=torch.float32, device=x.device)
+    rc = _few_dw[0](dy.data_ptr(), dy.stride(0), x.data_ptr(), x.stride(0), out.data_ptr(), int(out_dtype == torch.bfloat16), scratch.data_ptr(), rows, outputs,
+                    cols, lib.stream_ptr())
+    lib.check_rc(rc, "lvb_few_outputs_dw")
+    return out
+
+
 def _linear_rows(x, weight, bias, residual):
     shp = x.shape
     y = gemm(x.reshape(-1, shp[-1]), weight, bias=bias, residual=None if residual is None else residual.reshape(-1, weight.shape[0]))
     return y.view(*shp[:-1], weight.shape[0])
+
+
+def _weight_grad(weight, dy2, x2) -> Optional[torch.Tensor]:
+    """``dy^T x`` for a parameter, or None when it goes into the parameter's own buffer (see :class:`_LinearFn`)."""
+    main_grad = getattr(weight, "main_grad", None)
+    sink = getattr(weight, "grad_sink", None)
+    if sink is not None:
+        sink(dy2, x2)  # fully sharded weights: the product is reduce-scattered to the rows' owners as it is computed
+        return None
+    if main_grad is not None:
+        gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=True)
+        return None
+    dtype = weight.dtype if weight.dtype in (torch.bfloat16, torch.float32) else torch.float32
+    dw = few_outputs_dw(dy2, x2, dtype)
+    return dw if dw is not None else gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=dtype)
 
 
 class _LinearFn(torch.autograd.Function):
@@ -347,16 +385,7 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = gemm(dy2, weight, b_mn=True).view(ctx.x_shape)
         if ctx.needs_input_grad[1]:
-            main_grad = getattr(ctx.weight_ref, "main_grad", None)
-            sink = getattr(ctx.weight_ref, "grad_sink", None)
-            if sink is not None:
-                sink(dy2, x2)  # fully sharded weights: the product is reduce-scattered to the rows' owners as it is computed
-                dw = None
-            elif main_grad is not None:
-                gemm(dy2, x2, a_mn=True, b_mn=True, out=main_grad, accumulate=True)
-                dw = None
-            else:
-                dw = gemm(dy2, x2, a_mn=True, b_mn=True, out_dtype=weight.dtype if weight.dtype in (torch.bfloat16, torch.float32) else torch.float32)
+            dw = _weight_grad(ctx.weight_ref, dy2, x2)
         if ctx.has_bias and ctx.needs_input_grad[2]:
             db = col_sum(dy2, ctx.bias_dtype)
         dres = dy if ctx.has_res else None

@@ -190,3 +190,16 @@ def test_col_sum(rows, cols, dtype):
     want = x.double().sum(0)
     assert got.dtype == dtype
     assert (got.double() - want).norm() <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
+
+
+@pytest.mark.parametrize("rows,outputs,cols,dtype", [(1024, 8, 8, torch.float32), (1500, 8, 1024, torch.bfloat16), (5003, 24, 776, torch.float32), (16384, 32, 264, torch.bfloat16)])
+def test_few_outputs_dw(rows, outputs, cols, dtype):
+    """Exact products of bf16 numbers in fp32 sums (2^-24 sqrt(rows)), then at most one bf16 rounding; fewer rows or more outputs are the GEMM's."""
+    from levanter_b200.ops.gemm import few_outputs_dw
+
+    dy, x = (torch.randn(rows, n + 8, device="cuda").bfloat16()[:, 8:] for n in (outputs, cols))
+    got = few_outputs_dw(dy, x, dtype)
+    want = dy.double().t() @ x.double()
+    assert got.dtype == dtype
+    assert (got.double() - want).norm() <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
+    assert few_outputs_dw(dy[:1000], x[:1000], dtype) is None
