@@ -375,7 +375,7 @@ def dot_product_attention_with_sink(q, k, v, sink: torch.Tensor, mask=None, bias
 
 
 # --------------------------------------------------------------------------------------------- module
-from ..nn import FusedRows, Linear, RmsNorm  # noqa: E402  (after function definitions to keep the file readable)
+from ..nn import FusedRows, Linear, RmsNorm, linear_many  # noqa: E402  (after function definitions to keep the file readable)
 
 
 @dataclass(frozen=True)
@@ -501,9 +501,8 @@ class Attention(nn.Module):
         c = self.config
         D = c.head_size
         lead = x.shape[:-1]
-        q = self.q_proj(x).view(*lead, c.maps * self.local_heads, D)
-        k = self.k_proj(x).view(*lead, c.maps * self.local_kv, D)
-        v = self.v_proj(x).view(*lead, self.local_kv, c.v_head_size)
+        q, k, v = linear_many(x, self.q_proj, self.k_proj, self.v_proj)
+        q, k, v = q.view(*lead, c.maps * self.local_heads, D), k.view(*lead, c.maps * self.local_kv, D), v.view(*lead, self.local_kv, c.v_head_size)
         if self.q_norm is not None:
             q = self.q_norm(q)
             k = self.k_norm(k)

@@ -24,9 +24,10 @@ import torch.nn.functional as F
 from torch.utils.checkpoint import checkpoint
 
 from ..layers.normalization import LayerNormConfigBase, RmsNormConfig
-from ..nn import Embedding, Linear
+from ..nn import Embedding, Linear, linear_many
 from ..ops.delta_rule import chunk_state_scan, gated_delta_rule, gated_delta_rule_supported, gated_out_norm
 from ..ops.dwconv import causal_dwconv
+from ..ops.gemm import MANY_ROWS
 from ..utils.activation import ActivationFunctionEnum
 from ..utils.flop_utils import lm_flops_per_token
 from ..utils.remat import should_recompute
@@ -178,14 +179,17 @@ class GatedDeltaNetLayer(nn.Module):
         c = self.config
         B, L, _ = x.shape
         H, Hk, dk, dv = c.num_heads, c.k_heads, c.head_k_dim, c.head_v_dim
-        q = self._conv(self.q_conv1d, self.q_proj(x)).view(B, L, Hk, dk)
-        k = self._conv(self.k_conv1d, self.k_proj(x)).view(B, L, Hk, dk)
-        v = self._conv(self.v_conv1d, self.v_proj(x)).view(B, L, H, dv)
-        beta = torch.sigmoid(self.b_proj(x).float())  # [B, L, H]
-        g = -self.A_log.float().exp() * F.softplus(self.a_proj(x).float() + self.dt_bias.float())
+        mods = (self.q_proj, self.k_proj, self.v_proj, self.g_proj, self.a_proj, self.b_proj)
+        # for many rows each product directly before what reads it, so that it finds the product in the L2
+        q, k, v, gate, a, b = linear_many(x, *mods) if B * L <= MANY_ROWS else (None,) * 6
+        q = self._conv(self.q_conv1d, self.q_proj(x) if q is None else q).view(B, L, Hk, dk)
+        k = self._conv(self.k_conv1d, self.k_proj(x) if k is None else k).view(B, L, Hk, dk)
+        v = self._conv(self.v_conv1d, self.v_proj(x) if v is None else v).view(B, L, H, dv)
+        beta = torch.sigmoid((self.b_proj(x) if b is None else b).float())  # [B, L, H]
+        g = -self.A_log.float().exp() * F.softplus((self.a_proj(x) if a is None else a).float() + self.dt_bias.float())
         if Hk == H and dv <= 512 and gated_delta_rule_supported(q, k, v, c.chunk_size):
             o, _ = gated_delta_rule(q, k, v, g, beta, scale=dk ** -0.5, normalize=True)
-            y = gated_out_norm(o, self.g_proj(x).view(B, L, H, dv), self.o_norm_weight, c.layer_norm_epsilon)
+            y = gated_out_norm(o, (self.g_proj(x) if gate is None else gate).view(B, L, H, dv), self.o_norm_weight, c.layer_norm_epsilon)
             return self.o_proj(y.view(B, L, H * dv).to(x.dtype))
         q = F.normalize(q.float(), dim=-1)
         k = F.normalize(k.float(), dim=-1)
@@ -196,7 +200,7 @@ class GatedDeltaNetLayer(nn.Module):
                                        beta.transpose(1, 2), chunk_size=c.chunk_size)
         o = o.transpose(1, 2)  # [B, L, H, dv]
         o = o * torch.rsqrt(o.pow(2).mean(-1, keepdim=True) + c.layer_norm_epsilon) * self.o_norm_weight.float()
-        o = o * F.silu(self.g_proj(x).float().view(B, L, H, dv))
+        o = o * F.silu((self.g_proj(x) if gate is None else gate).float().view(B, L, H, dv))
         return self.o_proj(o.reshape(B, L, H * dv).to(x.dtype))
 
 

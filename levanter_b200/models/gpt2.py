@@ -14,8 +14,9 @@ from torch.utils.checkpoint import checkpoint
 
 from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
 from ..layers.attention import AttentionBackend, AttentionMask, default_flash, dot_product_attention
-from ..nn import Dropout, Embedding, LayerNorm, Linear, trunc_normal_
+from ..nn import Dropout, Embedding, LayerNorm, Linear, fork_norm, trunc_normal_
 from ..ops.flash_attention import flash_attention_joint
+from ..ops.gemm import linear_residual
 from ..utils.activation import ActivationFunctionEnum
 from ..utils.flop_utils import lm_flops_per_token
 from ..utils.remat import should_recompute
@@ -103,8 +104,9 @@ class Gpt2Mlp(nn.Module):
         self.c_proj = Linear(m, e, bias=config.use_bias, init_std=config.initializer_range, out_first=False)
         self.act = config.activation_function.to_fn()
 
-    def forward(self, x):
-        return self.c_proj(self.act(self.c_fc(x)))
+    def forward(self, x, residual=None):
+        h = self.act(self.c_fc(x))
+        return self.c_proj(h) if residual is None else linear_residual(h, self.c_proj.weight, self.c_proj.bias, residual)
 
 
 class Gpt2Attention(nn.Module):
@@ -117,7 +119,10 @@ class Gpt2Attention(nn.Module):
         self.c_proj = Linear(e, e, bias=config.use_bias, init_std=config.initializer_range, out_first=False,
                              lev_out=(e,), lev_in=(h, d))
 
-    def forward(self, x, mask, layer_idx: int):
+    def _out(self, heads, residual):
+        return self.c_proj(heads) if residual is None else linear_residual(heads, self.c_proj.weight, self.c_proj.bias, residual)
+
+    def forward(self, x, mask, layer_idx: int, residual=None):
         c = self.config
         B, S, E = x.shape
         qkv = self.c_attn(x).view(B, S, 3, c.num_heads, c.head_size)
@@ -126,14 +131,14 @@ class Gpt2Attention(nn.Module):
         if c.use_flash_attention is not False and default_flash(q, k, v, mask, None, c.attn_pdrop == 0.0 or not self.training, dtype, c.attn_backend):
             # the kernels read the projection's rows where they are, and the scale of the layer joins that of the scores
             scale = c.head_size ** -0.5 / (layer_idx + 1.0 if c.scale_attn_by_inverse_layer_idx else 1.0)
-            return self.c_proj(flash_attention_joint(qkv, mask, scaling_factor=scale).reshape(B, S, E))
+            return self._out(flash_attention_joint(qkv, mask, scaling_factor=scale).reshape(B, S, E), residual)
         if c.scale_attn_by_inverse_layer_idx:
             q = q / (layer_idx + 1.0)
         out = dot_product_attention(q, k, v, mask, inference=not self.training, dropout=c.attn_pdrop,
                                     use_flash=c.use_flash_attention, attn_backend=c.attn_backend,
                                     flash_block_size=c.flash_attention_block_size,
                                     attention_dtype=dtype)
-        return self.c_proj(out.reshape(B, S, E).to(x.dtype))
+        return self._out(out.reshape(B, S, E).to(x.dtype), residual)
 
 
 class Gpt2Block(nn.Module):
@@ -147,9 +152,15 @@ class Gpt2Block(nn.Module):
         self.resid_dropout = Dropout(config.resid_pdrop)
 
     def forward(self, x, mask):
-        x = x + self.resid_dropout(self.attn(self.ln_1(x), mask, self.layer_idx))
-        x = x + self.resid_dropout(self.mlp(self.ln_2(x)))
-        return x
+        h, x = fork_norm(self.ln_1, x)
+        if (self.resid_dropout.p == 0.0 or not self.training) and all(type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks
+                                                                      for m in (self.attn.c_proj, self.mlp.c_proj)):
+            x = self.attn(h, mask, self.layer_idx, residual=x)  # added in the projections' epilogues
+            h, x = fork_norm(self.ln_2, x)
+            return self.mlp(h, residual=x)
+        x = x + self.resid_dropout(self.attn(h, mask, self.layer_idx))
+        h, x = fork_norm(self.ln_2, x)
+        return x + self.resid_dropout(self.mlp(h))
 
 
 class Gpt2Transformer(nn.Module):

@@ -21,7 +21,7 @@ from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
 from ..layers.attention import DECODE_ROWS, Attention, AttentionBackend, AttentionConfig, AttentionMask, KvPageCache
 from ..layers.normalization import LayerNormConfigBase, RmsNormConfig
 from ..layers.rotary import rope_config_from_hf, rope_to_hf_dict, DefaultRotaryEmbeddingsConfig, RotaryEmbeddingsConfig
-from ..nn import Embedding, FusedRows, Linear
+from ..nn import Embedding, FusedRows, Linear, fork_norm, linear_many
 from ..ops.gemm import linear_residual
 from ..ops.glu import ClampedGlu, GatedActivation, gated_activation
 from ..ops.residual_stream import add_linear, glu_of_rows, project
@@ -195,7 +195,7 @@ class LlamaMlp(nn.Module):
         if x.dim() == 2 and x.shape[0] <= DECODE_ROWS and not torch.is_grad_enabled() and x.dtype == self.gate_proj.weight.dtype == torch.bfloat16:
             h = self._inner(x, build=x.shape[0] <= 128)  # decode steps; a prompt's rows are a multiple of 256
         else:
-            h = gated_activation(self.gate_proj(x), self.up_proj(x), self.act)
+            h = gated_activation(*linear_many(x, self.gate_proj, self.up_proj), self.act)
         if self.tp is not None and self.tp.size > 1:
             out = self.tp.row_linear(h, self.down_proj)
             if self.down_proj.bias is not None:
@@ -227,7 +227,7 @@ class LlamaDecoderLayer(nn.Module):
     def _attn_block(self, x, mask, pos_ids):
         """``x + attn(norm(x))`` with the residual add folded into the output-projection GEMM epilogue."""
         a = self.self_attn
-        h = self.input_layernorm(x)
+        h, x = fork_norm(self.input_layernorm, x)
         tp_on = self.tp is not None and self.tp.size > 1
         if self.post_attn_layernorm is not None or tp_on:
             if tp_on:
@@ -247,7 +247,7 @@ class LlamaDecoderLayer(nn.Module):
 
     def forward(self, x: torch.Tensor, mask=None, pos_ids=None) -> torch.Tensor:
         x = self._attn_block(x, mask, pos_ids)
-        h = self.post_attention_layernorm(x)
+        h, x = fork_norm(self.post_attention_layernorm, x)
         if self.post_mlp_layernorm is not None:
             return x + self.post_mlp_layernorm(self.mlp(h))
         return self.mlp(h, residual=x)

@@ -167,10 +167,11 @@ class RmsNorm(nn.Module):
         else:
             self.register_parameter("bias", None)
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from .ops.norm import rms_norm
+    def forward(self, x: torch.Tensor, fork: bool = False):
+        """``fork``: ``(norm(x), x)``, see ``ops.norm.norm_and_input``."""
+        from .ops.norm import norm_and_input, rms_norm
 
-        return rms_norm(x, self.weight, self.bias, self.eps)
+        return norm_and_input(x, self.weight, self.bias, self.eps, layer_norm=False) if fork else rms_norm(x, self.weight, self.bias, self.eps)
 
     def from_stream(self, x: torch.Tensor, rows: Optional[torch.Tensor] = None) -> torch.Tensor:
         """The norm of an fp32 residual stream, in the weight's dtype (``rows``: of these rows only)."""
@@ -223,10 +224,28 @@ class LayerNorm(nn.Module):
         else:
             self.register_parameter("bias", None)
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from .ops.norm import layer_norm
+    def forward(self, x: torch.Tensor, fork: bool = False):
+        """``fork``: ``(norm(x), x)``, see ``ops.norm.norm_and_input``."""
+        from .ops.norm import layer_norm, norm_and_input
 
-        return layer_norm(x, self.weight, self.bias, self.eps)
+        return norm_and_input(x, self.weight, self.bias, self.eps, layer_norm=True) if fork else layer_norm(x, self.weight, self.bias, self.eps)
+
+
+def fork_norm(norm: nn.Module, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(norm(x), x)`` of any norm module; this module's own add the two gradients of ``x`` in the norm's backward pass."""
+    return norm(x, fork=True) if type(norm) in (RmsNorm, LayerNorm) else (norm(x), x)
+
+
+def linear_many(x: torch.Tensor, *projections: nn.Module):
+    """The projections of the same rows, one by one; in training their input gradients are summed in the epilogues of their products."""
+    from .ops.gemm import linear_many as many
+
+    if x.requires_grad and torch.is_grad_enabled() and all(type(m) is Linear and m.bias is None and not m._forward_hooks and not m._forward_pre_hooks
+                                                          and getattr(m.weight, "grad_sink", None) is None for m in projections):
+        got = many(x, [m.weight for m in projections])
+        if got is not None:
+            return got
+    return tuple(m(x) for m in projections)
 
 
 class Dropout(nn.Module):

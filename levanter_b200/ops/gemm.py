@@ -416,3 +416,40 @@ def linear_residual(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.
     if x.is_cuda and lib.available() and x.dtype == torch.bfloat16 and residual.dtype == torch.bfloat16 and _tma_shapes_ok(weight):
         return _linear_rows(x, weight, bias, residual) if lib.plain_call() else _LinearFn.apply(x, weight, bias, residual)
     return torch.nn.functional.linear(x, weight, bias) + residual
+
+
+class _LinearManyFn(torch.autograd.Function):
+    """Several projections of the same rows: every product of the backward pass adds its input gradient to that of the ones before it in its
+    epilogue, and one function stands where there were several."""
+
+    @staticmethod
+    def forward(ctx, x, *weights):
+        ctx.save_for_backward(x.reshape(-1, x.shape[-1]), *weights)
+        ctx.x_shape = x.shape
+        ctx.refs = weights
+        return tuple(_linear_rows(x, w, None, None) for w in weights)
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x2, *weights = ctx.saved_tensors
+        dx, dws = None, []
+        for i, (dy, w, ref) in enumerate(zip(dys, weights, ctx.refs)):
+            dy2 = dy.reshape(-1, dy.shape[-1])
+            if dy2.dtype != torch.bfloat16:
+                dy2 = dy2.to(torch.bfloat16)
+            if ctx.needs_input_grad[0]:
+                dx = gemm(dy2, w, b_mn=True, out=dx, accumulate=dx is not None)
+            dws.append(_weight_grad(ref, dy2, x2) if ctx.needs_input_grad[1 + i] else None)
+        return (None if dx is None else dx.view(ctx.x_shape), *dws)
+
+
+MANY_ROWS = 2048
+
+
+def linear_many(x: torch.Tensor, weights):
+    """``[x W^T for W in weights]`` on the tcgen05 GEMM, or None where :func:`linear` would not take it for all of them, and for more rows than the
+    launches bound: an epilogue that reads back what it adds to costs a large product more than a pass of its own (Gated DeltaNet, two layers:
+    1500 rows 5.40 -> 4.95 ms, 16384 rows 22.96 -> 23.71)."""
+    if not (x.numel() <= MANY_ROWS * x.shape[-1] and x.is_cuda and lib.available() and x.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 and _tma_shapes_ok(w) for w in weights)):
+        return None
+    return _LinearManyFn.apply(x, *weights)

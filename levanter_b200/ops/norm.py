@@ -93,7 +93,7 @@ def _norm_rows(x, residual, weight, bias, eps, layer_norm, w_offset, stats: bool
 
 class _NormFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, residual, weight, bias, eps, layer_norm, w_offset):
+    def forward(ctx, x, residual, weight, bias, eps, layer_norm, w_offset, fork=False):
         y, xin, rstd, mean = _norm_rows(x, residual, weight, bias, eps, layer_norm, w_offset, True)
         ctx.save_for_backward(xin, weight, rstd, mean)
         ctx.layer_norm = layer_norm
@@ -104,7 +104,7 @@ class _NormFn(torch.autograd.Function):
         ctx.wf32 = _weights_fp32(weight, bias)
         if residual is not None:
             return y.view(x.shape), xin.view(x.shape)
-        return y.view(x.shape), None
+        return y.view(x.shape), x if fork else None
 
     @staticmethod
     def backward(ctx, dy, dh):
@@ -132,7 +132,7 @@ class _NormFn(torch.autograd.Function):
                     int(ctx.layer_norm), lib.stream_ptr())
         lib.check_rc(rc, "lvb_norm_bwd")
         dxv = dx.view(ctx.shape)
-        return dxv, (dxv if ctx.has_res else None), dw, db, None, None, None
+        return dxv, (dxv if ctx.has_res else None), dw, db, None, None, None, None
 
 
 def fused_norm(x, weight, bias, eps, *, layer_norm=False, w_offset=0.0, residual=None) -> Tuple[torch.Tensor, Optional[torch.Tensor]]:
@@ -147,6 +147,13 @@ def fused_norm(x, weight, bias, eps, *, layer_norm=False, w_offset=0.0, residual
         h = (x.float() + residual.float()).to(x.dtype)
         return norm_reference(h, weight, bias, eps, layer_norm=layer_norm, w_offset=w_offset), h
     return norm_reference(x, weight, bias, eps, layer_norm=layer_norm, w_offset=w_offset), None
+
+
+def norm_and_input(x, weight, bias, eps, *, layer_norm: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``(norm(x), x)`` for a block whose input goes on beside its norm: the gradient of the second is added where the norm's is made."""
+    if _kernel_ok(x, weight, bias) and not lib.plain_call():
+        return _NormFn.apply(x, None, weight, bias, eps, layer_norm, 0.0, True)
+    return fused_norm(x, weight, bias, eps, layer_norm=layer_norm)[0], x
 
 
 def rms_norm(x, weight, bias=None, eps: float = 1e-6, w_offset: float = 0.0) -> torch.Tensor:

@@ -203,3 +203,33 @@ def test_few_outputs_dw(rows, outputs, cols, dtype):
     assert got.dtype == dtype
     assert (got.double() - want).norm() <= (2 ** -8 if dtype == torch.bfloat16 else 1e-5) * want.norm()
     assert few_outputs_dw(dy[:1000], x[:1000], dtype) is None
+
+
+@pytest.mark.parametrize("rows", [7, 1100])
+def test_projections_of_the_same_rows_and_a_norm_that_forks(rows):
+    """Sums of input gradients in the products' epilogues, and a block's input beside its norm: what separate functions give, with fewer roundings
+    (2^-8 of a gradient's norm)."""
+    from levanter_b200.nn import LayerNorm, Linear, fork_norm, linear_many
+
+    torch.manual_seed(0)
+    with torch.device("cuda"):
+        mods = [Linear(264, n).bfloat16() for n in (264, 8, 520)]
+        ln = LayerNorm(264).bfloat16()
+    x = torch.randn(rows, 264, device="cuda").bfloat16().requires_grad_()
+    gs = [torch.randn(rows, n, device="cuda").bfloat16() for n in (264, 8, 520)]
+    params = [m.weight for m in mods] + [ln.weight, ln.bias]
+
+    def grads(joint):
+        for p in params + [x]:
+            p.grad = None
+        h, r = fork_norm(ln, x) if joint else (ln(x), x)
+        ys = linear_many(h, *mods) if joint else [m(h) for m in mods]
+        torch.autograd.backward([*ys, r * 1], [*gs, gs[0]])
+        return [t.detach() for t in ys], [p.grad.float() for p in params + [x]]
+
+    (y1, g1), (y2, g2) = grads(True), grads(False)
+    assert all(torch.equal(a, b) for a, b in zip(y1, y2))
+    for a, b in zip(g1, g2):
+        assert (a - b).norm() <= 2 ** -7 * b.norm()
+    h, r = fork_norm(ln, x.detach())
+    assert torch.equal(h, ln(x.detach())) and torch.equal(r, x.detach())
