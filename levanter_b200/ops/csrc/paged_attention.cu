@@ -8,7 +8,7 @@
 // rows of a kv head are adjacent 2*D-element runs.
 //
 // paged_attention is bandwidth bound (every step re-reads the context once), so the work is cut for parallelism, not for
-// tensor cores: one CTA per (query token, kv head, partition of 64 to 1024 keys).  A CTA scores its keys against the G query heads
+// tensor cores: one CTA per (query token, kv head, partition of 256 keys).  A CTA scores its keys against the G query heads
 // that share the kv head (one key per thread, 16-byte loads), soft-maxes within the partition in shared memory,
 // accumulates P.V with eight output dimensions per thread, and writes an un-normalised partial (o, max, sum).  A second small
 // kernel merges the partitions of each (token, head).  Nothing here synchronises with the host: sequence boundaries,
@@ -21,7 +21,7 @@ namespace lvb {
 namespace paged {
 
 constexpr int kPart = 256;     // keys per partition of the scalar kernels; the tensor-core kernel's come from part_keys
-constexpr int kMaxParts = 256;
+constexpr int kMaxParts = 256;  // of the tensor-core kernel, whose partitions grow with the context beyond that
 constexpr int kThreads = 128;  // 4 warps
 constexpr int kMaxG = 16;      // query heads per kv head
 
@@ -841,12 +841,15 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
 }
 
 // One CTA per (token, head): merge the partials of the partitions that were live for this token.  A thread per partition makes its weight, then
-// every thread sums its output dimensions over them.
-// kThreadsM: threads per CTA, a stride over the p.dv output dimensions.
+// every thread sums its output dimension over them, kMergeParts partitions at a time: the scalar kernels' partitions are 256 keys, so a context
+// may have any number of them.
+constexpr int kMergeParts = 256;
+
+// kThreadsM: threads per CTA, at least p.dv.
 template <int kThreadsM>
 __global__ void __launch_bounds__(kThreadsM) paged_merge_kernel(Params p) {
-  __shared__ float s_w[kMaxParts], s_red[kThreadsM / 32];
-  const int D = p.dv;
+  __shared__ float s_w[kMergeParts], s_red[kThreadsM / 32];
+  const int D = p.dv, d = threadIdx.x;
   const int t = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   chain_wait();
@@ -864,29 +867,33 @@ __global__ void __launch_bounds__(kThreadsM) paged_merge_kernel(Params p) {
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kThreadsM / 32; ++w) m = fmaxf(m, s_red[w]);
-  for (int i = threadIdx.x; i < np; i += kThreadsM) {
-    const float2 x = ml[i];
-    const float w = x.x == -INFINITY ? 0.f : __expf(x.x - m);
-    s_w[i] = w;
-    l = fmaf(x.y, w, l);
+  float o = 0.f;
+  for (int p0 = 0; p0 < np; p0 += kMergeParts) {
+    const int n = min(kMergeParts, np - p0);
+    if (p0 > 0) __syncthreads();  // the weights before these have been read
+    for (int i = threadIdx.x; i < n; i += kThreadsM) {
+      const float2 x = ml[p0 + i];
+      const float w = x.x == -INFINITY ? 0.f : __expf(x.x - m);
+      s_w[i] = w;
+      l = fmaf(x.y, w, l);
+    }
+    __syncthreads();  // the weights are there, and the maxima have been read
+    if (d < D) {
+      const float* src = p.part_o + (hrow * p.parts + p0) * D + d;
+#pragma unroll 4
+      for (int i = 0; i < n; ++i) {
+        const float w = s_w[i], x = src[static_cast<long long>(i) * D];
+        o = w > 0.f ? fmaf(x, w, o) : o;
+      }
+    }
   }
   l = warp_sum(l);
-  __syncthreads();  // the maxima have been read, the weights are there
   if (lane == 0) s_red[warp] = l;
   __syncthreads();
   l = 0.f;
 #pragma unroll
   for (int w = 0; w < kThreadsM / 32; ++w) l += s_red[w];
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    const float* src = p.part_o + hrow * p.parts * D + d;
-    float o = 0.f;
-#pragma unroll 4
-    for (int i = 0; i < np; ++i) {
-      const float w = s_w[i], x = src[static_cast<long long>(i) * D];
-      o = w > 0.f ? fmaf(x, w, o) : o;
-    }
-    p.out[hrow * D + d] = __float2bfloat16(l > 0.f ? o / l * gate_factor(p, t, h, d) : 0.f);
-  }
+  if (d < D) p.out[hrow * D + d] = __float2bfloat16(l > 0.f ? o / l * gate_factor(p, t, h, d) : 0.f);
 }
 
 // The same with two score maps per head: one CTA per (token, head) merges both, and their difference is normed.

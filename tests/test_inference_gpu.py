@@ -222,6 +222,22 @@ def test_paged_attention_partitions_of_every_length(D, KV, G, q_lens, kv_lens, p
     assert not got[live:].any()
 
 
+@pytest.mark.parametrize("kv_lens", [[65536, 3], [65537, 65280], [131072 + 700, 256]])
+def test_heads_of_256_over_more_partitions_than_the_merge_takes_at_once(kv_lens):
+    """The scalar kernel's partitions are 256 keys, the merge takes 256 of them at a time: 256, 257, 255 and 515 of them.  Sums are fp32, outputs
+    bf16 (2^-9)."""
+    from levanter_b200.ops import paged_attention as PA
+
+    q, kv, lens, pages, cu, n = _random_case(2, 1, 2, 256, 256, -(-max(kv_lens) // 256), [1, 1], kv_lens, seed=11)
+    got = PA.ragged_paged_attention(q, kv, lens, pages, cu, n, sm_scale=0.0625)
+    lib.check_status()
+    for s, m in enumerate(kv_lens):
+        rows = kv[pages[s].long()].reshape(-1, 2, 256)[:m].double()
+        want = torch.softmax(q[s].double() @ rows[:, 0].t() * 0.0625, dim=-1) @ rows[:, 1]
+        assert (got[s].double() - want).norm() / want.norm() < 2 ** -9
+    assert not got[2:].any()
+
+
 @pytest.mark.parametrize("heads,kv,hidden,bias", [(4, 2, 512, False), (8, 8, 512, False), (2, 1, 256, True)])
 @pytest.mark.parametrize("tokens", [3, 200, 300])
 def test_plain_serving_step_prepares_rows_in_one_pass(heads, kv, hidden, bias, tokens, monkeypatch):
