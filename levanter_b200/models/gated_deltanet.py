@@ -62,6 +62,7 @@ def delta_rule_chunked_scan(q, k, v, g, beta, chunk_size: int = 64, initial_stat
         q, k, v = q.float(), k.float(), v.float()
     g, beta = g.float(), beta.float()
     if gated_delta_rule_supported(q, k, v, chunk_size):
+        g, beta = g.reshape(B, H, L), beta.reshape(B, H, L)
         out, S = gated_delta_rule(*(t.transpose(1, 2) for t in (q, k, v, g, beta)), initial_state, scale=dk ** -0.5)
         return out.reshape(B, H, -1, dv)[:, :, :L].to(dtype), S
     q, k, v = q.float(), k.float(), v.float()

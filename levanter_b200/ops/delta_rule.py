@@ -118,7 +118,7 @@ def gated_delta_rule_supported(q, k, v, chunk_size: int = CHUNK) -> bool:
     """Whether :func:`gated_delta_rule` takes ``q, k [.., dk]`` and ``v [.., dv]``."""
     return (q.is_cuda and lib.available() and chunk_size == CHUNK and q.numel() > 0 and q.shape[-1] in (64, 128) and v.shape[-1] % 64 == 0
             and v.shape[-1] > 0 and q.dtype == k.dtype == v.dtype and q.dtype in (torch.float32, torch.bfloat16) and q.shape[:-1] == v.shape[:-1]
-            and q.shape == k.shape)
+            and q.shape == k.shape and q.device == k.device == v.device)
 
 
 _chunks = {}
@@ -199,7 +199,15 @@ def gated_delta_rule(q, k, v, g, beta, S0: Optional[torch.Tensor] = None, *, sca
     """The gated delta rule over ``q, k [B, L, H, dk]``, ``v [B, L, H, dv]`` (bf16 or fp32), ``g`` (log decay) and ``beta [B, L, H]`` fp32 ->
     ``(out [B, H, ceil(L / 64), 64, dv], final state [B, H, dk, dv])`` in fp32; rows past ``L`` of the last chunk are no results.  Queries are
     multiplied by ``scale``; with ``normalize`` queries and keys are divided by their 2-norms first.  ``exact`` as in :func:`chunk_state_scan`.  For what
-    :func:`gated_delta_rule_supported` takes."""
+    :func:`gated_delta_rule_supported` takes.  Gates or a state of another size, or on another device, raise."""
+    B, L, H, dk = q.shape
+    for t in (g, beta, S0):
+        if t is not None and t.device != q.device:
+            raise RuntimeError(f"the gates and the state have to be where the queries are ({q.device}), not on {t.device}")
+    for t in (g, beta):  # the kernels read what the queries' shape says
+        if t.shape != (B, L, H):
+            raise RuntimeError(f"gates of shape {tuple(t.shape)} for {B} sequences of {L} positions and {H} heads")
+    S0 = None if S0 is None else S0.reshape(B, H, dk, v.shape[3])
     return _GatedDeltaRule.apply(q, k, v, g.float(), beta.float(), S0, scale, normalize, exact)
 
 

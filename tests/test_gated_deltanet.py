@@ -60,3 +60,30 @@ def test_model_trains_and_is_causal():
         opt.step()
         losses.append(loss.item())
     assert losses[-1] < losses[0]
+
+
+@pytest.mark.parametrize("wrong", [dict(g=(2, 3, 69)), dict(beta=(2, 3, 71)), dict(g=(1, 3, 70)), dict(beta=(2, 1, 70)), dict(state=(3, 64, 64)),
+                                   dict(state=(2, 3, 64, 32)), dict(device="g"), dict(device="beta"), dict(device="state")])
+def test_gates_and_states_of_another_size_or_device_never_reach_the_kernels(wrong, monkeypatch):
+    """The kernels take the sizes of the gates and of the state from the queries: what does not fit has to raise before."""
+    from levanter_b200.models import gated_deltanet
+    from levanter_b200.ops import delta_rule
+
+    class Kernels:
+        @staticmethod
+        def apply(*a):
+            raise AssertionError("the kernels were reached")
+
+    monkeypatch.setattr(gated_deltanet, "gated_delta_rule_supported", lambda *a: True)
+    monkeypatch.setattr(delta_rule, "_GatedDeltaRule", Kernels)
+    args = dict(g=torch.zeros(wrong.get("g", (2, 3, 70))), beta=torch.zeros(wrong.get("beta", (2, 3, 70))),
+                initial_state=torch.zeros(wrong.get("state", (2, 3, 64, 64))))
+    if "device" in wrong:
+        name = "initial_state" if wrong["device"] == "state" else wrong["device"]
+        args[name] = args[name].to("meta")
+    q, k, v = (torch.zeros(2, 3, 70, 64) for _ in range(3))
+    with pytest.raises(RuntimeError):
+        gated_deltanet.delta_rule_chunked_scan(q, k, v, **args)
+    if "device" not in wrong and "state" not in wrong:  # rows as the layer has them
+        with pytest.raises(RuntimeError):
+            delta_rule.gated_delta_rule(*(t.transpose(1, 2) for t in (q, k, v, args["g"], args["beta"])), scale=1.0)
