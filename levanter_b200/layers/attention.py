@@ -501,6 +501,7 @@ class Attention(nn.Module):
         c = self.config
         D = c.head_size
         lead = x.shape[:-1]
+        self._rows.hold([m.weight for m in (self.q_proj, self.k_proj, self.v_proj) if type(m) is Linear])
         q, k, v = linear_many(x, self.q_proj, self.k_proj, self.v_proj)
         q, k, v = q.view(*lead, c.maps * self.local_heads, D), k.view(*lead, c.maps * self.local_kv, D), v.view(*lead, self.local_kv, c.v_head_size)
         if self.q_norm is not None:
@@ -601,8 +602,7 @@ class Attention(nn.Module):
         from ..ops import paged_attention as PA
 
         c = self.config
-        if c.output_gate or c.attention_chunk_size is not None or c.v_head_size != c.head_size or c.sliding_window is not None \
-                or c.head_temperature or c.value_mixing or c.head_gate or c.differential is not None or (self.rot is not None and not self.rot.is_plain):
+        if not self._plain_pages():
             out, _ = self._paged_heads(x, kv_cache, batch_info, pos_ids)
             return (self.o_proj(out) if residual is None else self.o_proj(out) + residual), kv_cache
         scale = c.scaling_factor if c.scaling_factor is not None else 1.0 / math.sqrt(c.head_size)
@@ -610,7 +610,7 @@ class Attention(nn.Module):
         prepared = self._prepared_for_pages(x, kv_cache)
         if prepared:
             # rotary positions and the cache write in one pass over the rows, which a decode step's joint projection leaves side by side
-            q, k, v = self._project_and_prepare(x, kv_cache, batch_info, pos_ids, decoding=seg is None)
+            q, k, v = self._project_and_prepare(x, kv_cache, batch_info, pos_ids)
         else:
             q, k, v = self._compute_qkv(x, pos_ids)
             kv_cache = kv_cache.update(batch_info, k, v)
@@ -635,16 +635,31 @@ class Attention(nn.Module):
             return self.o_proj(out) + residual, kv_cache
         return self.o_proj(out), kv_cache
 
+    def _plain_pages(self) -> bool:
+        """Whether serving steps need none of what :meth:`_paged_heads` is for."""
+        c = self.config
+        return not (c.output_gate or c.attention_chunk_size is not None or c.v_head_size != c.head_size or c.sliding_window is not None
+                    or c.head_temperature or c.value_mixing or c.head_gate or c.differential is not None or (self.rot is not None and not self.rot.is_plain))
+
+    def _prepared_heads(self) -> bool:
+        """bf16 weights, heads of 64 or 128 in groups that the tensor-core decode kernel has."""
+        return (self.config.head_size in (64, 128) and self.local_heads // self.local_kv <= 16
+                and all(m.weight.dtype == torch.bfloat16 for m in self._projections() if type(m) is Linear))
+
     def _prepared_for_pages(self, x, kv_cache: "KvPageCache") -> bool:
-        """Whether a plain serving step takes the kernels between projections and pages: bf16 rows and pages on a GPU, heads of 64 or 128 in
-        groups that the tensor-core decode kernel has."""
+        """Whether a plain serving step takes the kernels between projections and pages: bf16 rows and pages on a GPU."""
         from ..ops import lib
 
         return (x.is_cuda and not torch.is_grad_enabled() and lib.available() and x.dim() == 2 and x.dtype == torch.bfloat16
-                and kv_cache.kv_pages.dtype == torch.bfloat16 and self.config.head_size in (64, 128) and self.local_heads // self.local_kv <= 16
-                and all(m.weight.dtype == torch.bfloat16 for m in self._projections() if type(m) is Linear))
+                and kv_cache.kv_pages.dtype == torch.bfloat16 and self._prepared_heads())
 
-    def _project_and_prepare(self, x, kv_cache: "KvPageCache", batch_info, pos_ids, decoding: bool):
+    def lay_out_for_serving(self) -> None:
+        """Lays the projections' weights side by side where serving steps of a few rows read them as one matrix.  Done with the cache, before a step
+        or a CUDA graph knows where they lie; what was taken from the parameters before (a ``state_dict``) keeps the values and no longer follows them."""
+        if self.q_norm is None and self._plain_pages() and self._prepared_heads() and all(type(m) is Linear and m.weight.is_cuda for m in self._projections()):
+            self._fused_projection(build=True)
+
+    def _project_and_prepare(self, x, kv_cache: "KvPageCache", batch_info, pos_ids):
         """``q, k, v`` rows as attention reads them (for a few rows slices of the joint product's rows), keys and values written to the pages."""
         from ..ops import paged_attention as PA
         from ..ops.qkv_prep import prepare_qkv
@@ -652,8 +667,7 @@ class Attention(nn.Module):
 
         D = self.config.head_size
         nq, nk = self.local_heads * D, self.local_kv * D
-        # the weights are laid out by the first decode step, not by a prompt that waits for its first token
-        fused = self._fused_projection(build=decoding) if x.shape[0] <= DECODE_ROWS and self.q_norm is None else None
+        fused = self._fused_projection() if x.shape[0] <= DECODE_ROWS and self.q_norm is None and not self.training else None
         if fused is not None:
             y = project(x, fused[0], bias=fused[1])
             q, k, v = y[:, :nq].unflatten(1, (-1, D)), y[:, nq:nq + nk].unflatten(1, (-1, D)), y[:, nq + nk:nq + 2 * nk].unflatten(1, (-1, D))
@@ -664,12 +678,12 @@ class Attention(nn.Module):
         PA.kv_page_write_general(kv_cache.kv_pages, k, v, batch_info.new_token_dests)
         return q, k, v
 
-    def _fused_projection(self, build: bool = True):
+    def _fused_projection(self, build: bool = False):
         """``(weight, bias or None)`` of the joint projection ``[q; k; v; gate]`` for serving: the projections read the same rows, so a
         decode step streams one matrix instead of launching four products.  None when a projection is wrapped (LoRA, fp8) or only
-        some of q, k, v have a bias, and for a model in training.  (The gate per head has none: its rows of the bias are zeros.)"""
+        some of q, k, v have a bias, and where the weights are not laid out for it.  (The gate per head has none: its rows of the bias are zeros.)"""
         mods = self._projections()
-        if self.training or not all(type(m) is Linear for m in mods):
+        if not all(type(m) is Linear for m in mods):
             return None
         with_bias = mods[:3] if self.config.head_gate else mods
         biased = [m.bias is not None for m in with_bias]
@@ -691,7 +705,7 @@ class Attention(nn.Module):
         c = self.config
         T, D, Dv = x.shape[0], c.head_size, c.v_head_size
         nq, nk, nv = c.maps * self.local_heads * D, c.maps * self.local_kv * D, self.local_kv * Dv
-        fused = self._fused_projection() if (x.is_cuda and not torch.is_grad_enabled() and self.q_norm is None) else None
+        fused = self._fused_projection(build=True) if (x.is_cuda and not torch.is_grad_enabled() and self.q_norm is None and not self.training) else None
         gate = None
         if fused is not None:
             y = project(x, fused[0], bias=fused[1])
@@ -741,6 +755,7 @@ class Attention(nn.Module):
 
     def empty_page_cache(self, max_pages: int, page_size: int, *, dtype=torch.bfloat16, device=None) -> "KvPageCache":
         c = self.config
+        self.lay_out_for_serving()
         return KvPageCache.init(max_pages, page_size, self.local_kv, c.maps * c.head_size, v_head_size=c.v_head_size, dtype=dtype, device=device)
 
 

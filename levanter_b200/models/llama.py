@@ -164,6 +164,12 @@ class LlamaMlp(nn.Module):
         self.act = activation if isinstance(activation, (ActivationFunctionEnum, ClampedGlu)) else ActivationFunctionEnum(activation)
         self._rows = FusedRows()
 
+    def lay_out_for_serving(self) -> None:
+        """Lays gate and up side by side for serving steps of a few rows, as the attention layer does with its projections."""
+        mods = (self.gate_proj, self.up_proj)
+        if all(type(m) is Linear and m.bias is None and m.weight.is_cuda and m.weight.dtype == torch.bfloat16 for m in mods):
+            self._rows.get([m.weight for m in mods])
+
     def _inner(self, x: torch.Tensor, build: bool = True) -> torch.Tensor:
         """The gated activation of packed rows; gate and up are one product when serving (no biases)."""
         mods = (self.gate_proj, self.up_proj)
@@ -193,8 +199,9 @@ class LlamaMlp(nn.Module):
         if self.tp is not None and self.tp.size > 1:
             x = self.tp.copy_to_region(x)
         if x.dim() == 2 and x.shape[0] <= DECODE_ROWS and not torch.is_grad_enabled() and x.dtype == self.gate_proj.weight.dtype == torch.bfloat16:
-            h = self._inner(x, build=x.shape[0] <= 128)  # decode steps; a prompt's rows are a multiple of 256
+            h = self._inner(x, build=False)
         else:
+            self._rows.hold([m.weight for m in (self.gate_proj, self.up_proj) if type(m) is Linear])
             h = gated_activation(*linear_many(x, self.gate_proj, self.up_proj), self.act)
         if self.tp is not None and self.tp.size > 1:
             out = self.tp.row_linear(h, self.down_proj)
@@ -296,6 +303,9 @@ class LlamaTransformer(nn.Module):
         return self.norm(x), new
 
     def initial_cache(self, max_pages: int, page_size: int, *, dtype=torch.bfloat16, device=None):
+        for l in self.layers:
+            if isinstance(l.mlp, LlamaMlp):
+                l.mlp.lay_out_for_serving()
         return [l.self_attn.empty_page_cache(max_pages, page_size, dtype=dtype, device=device) for l in self.layers]
 
 

@@ -14,6 +14,7 @@ Class names matter: the default weight-decay mask excludes parameters whose clas
 from __future__ import annotations
 
 import math
+import threading
 from typing import Optional, Sequence, Tuple
 
 import torch
@@ -77,40 +78,64 @@ class Linear(nn.Module):
 
 class FusedRows:
     """One matrix (or vector) whose row slices are the given parameters: projections that read the same rows become one product when
-    a model serves, and nothing is stored twice.  :meth:`get` returns it, building it first when the parameters are not (or, after
-    a move or a conversion, no longer) its slices (None there with ``build`` off); None for parameters in training, which belong to the gradient engine's own
-    flat buffers.  ``pad``: zero rows at the end."""
+    a model serves, and nothing is stored twice.  :meth:`get` returns it; None for parameters in training, which belong to the gradient engine's own
+    flat buffers.  Parameters that are not (or, after a move or a conversion, no longer) its slices are copied there and re-pointed first, unless
+    ``build`` is off or a CUDA graph has recorded where they lie (:meth:`hold`): its replays would go on reading the storage that was left.
+    ``pad``: zero rows at the end."""
 
     def __init__(self, pad: int = 0):
         self.pad = pad
-        self._fused: Optional[torch.Tensor] = None
+        self._held: set = set()  # addresses of parameters that a graph reads one by one
+
+    def _whole(self, params: Sequence[torch.Tensor]) -> Optional[torch.Tensor]:
+        """The matrix when its storage consists of the parameters in their order and the padding, and of nothing else."""
+        first = params[0]
+        storage = first.untyped_storage()
+        base = at = storage.data_ptr()
+        rows = self.pad
+        for p in params:
+            if p.data_ptr() != at or p.dtype != first.dtype or not p.is_contiguous() or p.untyped_storage().data_ptr() != base:
+                return None
+            at += p.numel() * p.element_size()
+            rows += p.shape[0]
+        width = first.stride(0)
+        if storage.nbytes() != rows * width * first.element_size():
+            return None
+        return first.detach().as_strided((rows, *first.shape[1:]), first.stride(), 0)
+
+    def hold(self, params: Sequence[torch.Tensor]) -> None:
+        """Called where the parameters are read one by one; while a graph is captured they stay where they are from then on."""
+        if params and params[0].is_cuda and torch.cuda.is_current_stream_capturing():
+            self._held.update(p.data_ptr() for p in params)
 
     def get(self, params: Sequence[torch.Tensor], build: bool = True) -> Optional[torch.Tensor]:
         if any(getattr(p, "main_grad", None) is not None or getattr(p, "grad_sink", None) is not None for p in params):
             return None
-        fused = self._fused
-        if fused is not None:
-            at = fused.data_ptr()
-            for p in params:
-                if p.data_ptr() != at or p.dtype != fused.dtype:
-                    fused = None
-                    break
-                at += p.numel() * p.element_size()
-        if fused is None:
-            if not build:
-                return None
-            if params[0].is_cuda and torch.cuda.is_current_stream_capturing():
-                return None  # the copy would be recorded and not made, and what follows would read the new rows
-            rows = [p.detach() for p in params]
-            if self.pad:
-                rows.append(rows[0].new_zeros(self.pad, *rows[0].shape[1:]))
-            fused = torch.cat(rows)
+        whole = self._whole(params)
+        if whole is not None:
+            return whole
+        self.hold(params)  # (under capture the copy would be recorded and not made)
+        if not build or any(p.is_inference() or p.data_ptr() in self._held for p in params):
+            return None
+        with _LAYING_OUT:
+            whole = self._whole(params)  # another thread may have come first
+            if whole is not None:
+                return whole
+            with torch.inference_mode(False), torch.no_grad():
+                rows = list(params)
+                if self.pad:
+                    rows.append(rows[0].new_zeros(self.pad, *rows[0].shape[1:]))
+                whole = torch.cat(rows)
             at = 0
             for p in params:
-                p.data = fused[at:at + p.shape[0]]
+                if p.is_cuda:  # the copy reads it on this stream, whatever stream it was made on
+                    p.data.record_stream(torch.cuda.current_stream(p.device))
+                p.data = whole[at:at + p.shape[0]]
                 at += p.shape[0]
-            self._fused = fused
-        return fused
+        return whole
+
+
+_LAYING_OUT = threading.Lock()
 
 
 class Embedding(nn.Module):

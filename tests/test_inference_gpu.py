@@ -277,3 +277,82 @@ def test_plain_serving_step_prepares_rows_in_one_pass(heads, kv, hidden, bias, t
     lib.check_status()
     assert (pages - pages_r).abs().max() <= 2 ** -7 * pages_r.abs().max()
     assert (out - out_r).norm() <= 2 ** -7 * out_r.norm()
+
+
+def _small_llama(layers=2):
+    from levanter_b200.models.llama import LlamaConfig
+
+    torch.manual_seed(0)
+    return LlamaConfig(seq_len=512, hidden_dim=256, intermediate_dim=512, num_layers=layers, num_heads=4, num_kv_heads=2, gradient_checkpointing=False) \
+        .build(512, device="cuda", dtype=torch.bfloat16).eval()
+
+
+def _decode_step(model, seqs, make_cache=True):
+    """Logits of one new token for each of ``seqs`` sequences of 5 tokens."""
+    from levanter_b200.inference.page_table import PageTable
+
+    table = PageTable.init(seqs, seqs, 16, 1)
+    for s in range(seqs):
+        table, _ = table.assign_seq_id_to_seq(s)
+    table, _ = table.allocate_for_seq(np.repeat(np.arange(seqs, dtype=np.int32), 4), np.tile(np.arange(4, dtype=np.int32), seqs))
+    table, info = table.allocate_for_seq(np.arange(seqs, dtype=np.int32), np.full(seqs, 4, np.int32))
+    cache = model.initial_cache(table, dtype=torch.bfloat16)
+    for i, c in enumerate(cache):
+        c.kv_pages.normal_(0.0, 0.5, generator=torch.Generator(device="cuda").manual_seed(i))
+    tokens = torch.arange(seqs, dtype=torch.int32, device="cuda") % 512
+    with torch.no_grad():
+        return model.decode(tokens, cache, info.to("cuda"), torch.full((seqs,), 4, dtype=torch.int32, device="cuda"))[0]
+
+
+def test_weights_lie_where_the_cache_was_made_and_steps_do_not_depend_on_earlier_ones():
+    """Steps of 3 to 256 rows read the joint matrices whether or not a smaller step ran before, and none of them moves a weight."""
+    got = {}
+    for order in ((200, 3, 256), (3, 256, 200)):
+        model = _small_llama()
+        model.initial_cache(4, 16)
+        state = model.state_dict()
+        where = {n: p.data_ptr() for n, p in model.named_parameters()}
+        for seqs in order:
+            logits = _decode_step(model, seqs)
+            if seqs in got:
+                assert torch.equal(got[seqs], logits)
+            got[seqs] = logits
+        assert where == {n: p.data_ptr() for n, p in model.named_parameters()} == {n: state[n].data_ptr() for n in where}
+        for layer in model.transformer.layers:
+            a, m = layer.self_attn, layer.mlp
+            assert a._fused_projection() is not None and m._rows.get([m.gate_proj.weight, m.up_proj.weight], build=False) is not None
+            assert torch.equal(a._fused_projection()[0], torch.cat([p.weight for p in (a.q_proj, a.k_proj, a.v_proj)]))
+    # separate products give the same numbers up to the rounding of bf16 sums in another order
+    for layer in model.transformer.layers:
+        for m in (layer.self_attn.q_proj, layer.self_attn.k_proj, layer.self_attn.v_proj, layer.mlp.gate_proj, layer.mlp.up_proj):
+            m.weight._keep_apart = m.weight.data = m.weight.data.clone()
+            layer.self_attn._rows._held.add(m.weight.data_ptr())
+            layer.mlp._rows._held.add(m.weight.data_ptr())
+    for seqs, logits in got.items():
+        apart = _decode_step(model, seqs)
+        assert layer.self_attn._fused_projection() is None
+        assert (apart.float() - logits.float()).norm() / logits.float().norm() < 2 ** -7
+
+
+def test_weights_that_a_graph_reads_are_not_moved():
+    """A graph captured on the separate weights, before any cache is made: its replays still read the weights that the model has."""
+    model = _small_llama()
+    ids = torch.randint(0, 512, (1, 300), device="cuda")
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        with torch.cuda.stream(side):
+            model(ids, None)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = model(ids, None)
+    where = {n: p.data_ptr() for n, p in model.named_parameters()}
+    _decode_step(model, 3)
+    assert where == {n: p.data_ptr() for n, p in model.named_parameters()}
+    with torch.no_grad():
+        for p in model.parameters():
+            p.mul_(1.25)
+        want = model(ids, None)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
