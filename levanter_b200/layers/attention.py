@@ -375,7 +375,7 @@ def dot_product_attention_with_sink(q, k, v, sink: torch.Tensor, mask=None, bias
 
 
 # --------------------------------------------------------------------------------------------- module
-from ..nn import FusedRows, Linear, RmsNorm, linear_many  # noqa: E402  (after function definitions to keep the file readable)
+from ..nn import FusedRows, Linear, RmsNorm, linear_many, plain  # noqa: E402  (after function definitions to keep the file readable)
 
 
 @dataclass(frozen=True)
@@ -507,6 +507,8 @@ class Attention(nn.Module):
         if self.q_norm is not None:
             q = self.q_norm(q)
             k = self.k_norm(k)
+        if not rotate and not all(plain(m, type(m)) for m in (self.q_proj, self.k_proj, self.q_norm, self.k_norm) if m is not None):
+            q, k = q.clone(), k.clone()  # the caller rotates in place, and a hook may have kept the rows
         if self.rot is not None and rotate:
             from ..ops import rope as rope_op
 
@@ -667,7 +669,8 @@ class Attention(nn.Module):
 
         D = self.config.head_size
         nq, nk = self.local_heads * D, self.local_kv * D
-        fused = self._fused_projection() if x.shape[0] <= DECODE_ROWS and self.q_norm is None and not self.training else None
+        fused = self._fused_projection() if (x.shape[0] <= DECODE_ROWS and self.q_norm is None and not self.training
+                                             and all(plain(m, Linear) for m in self._projections())) else None
         if fused is not None:
             y = project(x, fused[0], bias=fused[1])
             q, k, v = y[:, :nq].unflatten(1, (-1, D)), y[:, nq:nq + nk].unflatten(1, (-1, D)), y[:, nq + nk:nq + 2 * nk].unflatten(1, (-1, D))
@@ -705,7 +708,8 @@ class Attention(nn.Module):
         c = self.config
         T, D, Dv = x.shape[0], c.head_size, c.v_head_size
         nq, nk, nv = c.maps * self.local_heads * D, c.maps * self.local_kv * D, self.local_kv * Dv
-        fused = self._fused_projection(build=True) if (x.is_cuda and not torch.is_grad_enabled() and self.q_norm is None and not self.training) else None
+        fused = self._fused_projection(build=True) if (x.is_cuda and not torch.is_grad_enabled() and self.q_norm is None and not self.training
+                                                       and all(plain(m, Linear) for m in self._projections())) else None
         gate = None
         if fused is not None:
             y = project(x, fused[0], bias=fused[1])

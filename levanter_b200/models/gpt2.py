@@ -14,7 +14,7 @@ from torch.utils.checkpoint import checkpoint
 
 from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
 from ..layers.attention import AttentionBackend, AttentionMask, default_flash, dot_product_attention
-from ..nn import Dropout, Embedding, LayerNorm, Linear, fork_norm, trunc_normal_
+from ..nn import Dropout, Embedding, LayerNorm, Linear, fork_norm, plain, trunc_normal_
 from ..ops.flash_attention import flash_attention_joint
 from ..ops.gemm import linear_residual
 from ..utils.activation import ActivationFunctionEnum
@@ -153,8 +153,8 @@ class Gpt2Block(nn.Module):
 
     def forward(self, x, mask):
         h, x = fork_norm(self.ln_1, x)
-        if (self.resid_dropout.p == 0.0 or not self.training) and all(type(m) is Linear and not m._forward_hooks and not m._forward_pre_hooks
-                                                                      for m in (self.attn.c_proj, self.mlp.c_proj)):
+        if (self.resid_dropout.p == 0.0 or not self.training) and plain(self.resid_dropout, Dropout) and plain(self.attn, Gpt2Attention) \
+                and plain(self.mlp, Gpt2Mlp) and plain(self.attn.c_proj, Linear) and plain(self.mlp.c_proj, Linear):
             x = self.attn(h, mask, self.layer_idx, residual=x)  # added in the projections' epilogues
             h, x = fork_norm(self.ln_2, x)
             return self.mlp(h, residual=x)

@@ -21,7 +21,7 @@ from ..compat.hf_checkpoints import HFCheckpointConverter, HFCompatConfig
 from ..layers.attention import DECODE_ROWS, Attention, AttentionBackend, AttentionConfig, AttentionMask, KvPageCache
 from ..layers.normalization import LayerNormConfigBase, RmsNormConfig
 from ..layers.rotary import rope_config_from_hf, rope_to_hf_dict, DefaultRotaryEmbeddingsConfig, RotaryEmbeddingsConfig
-from ..nn import Embedding, FusedRows, Linear, fork_norm, linear_many
+from ..nn import Embedding, FusedRows, Linear, fork_norm, linear_many, plain
 from ..ops.gemm import linear_residual
 from ..ops.glu import ClampedGlu, GatedActivation, gated_activation
 from ..ops.residual_stream import add_linear, glu_of_rows, project
@@ -174,7 +174,7 @@ class LlamaMlp(nn.Module):
         """The gated activation of packed rows; gate and up are one product when serving (no biases)."""
         mods = (self.gate_proj, self.up_proj)
         w = None
-        if all(type(m) is Linear and m.bias is None for m in mods) and x.is_cuda and not self.training and not torch.is_grad_enabled():
+        if all(plain(m, Linear) and m.bias is None for m in mods) and x.is_cuda and not self.training and not torch.is_grad_enabled():
             w = self._rows.get([m.weight for m in mods], build)
         if w is not None:
             return glu_of_rows(project(x, w), self.gate_proj.weight.shape[0], self.act)

@@ -256,17 +256,24 @@ class LayerNorm(nn.Module):
         return norm_and_input(x, self.weight, self.bias, self.eps, layer_norm=True) if fork else layer_norm(x, self.weight, self.bias, self.eps)
 
 
+def plain(m: nn.Module, *kinds: type) -> bool:
+    """Whether ``m`` is one of these classes itself and a call of it is its ``forward`` and nothing else: no hook of any kind that would have to see the
+    call, its gradients or its result, and no ``forward`` of the instance.  Only then may a layer do the module's work in another way."""
+    return (type(m) in kinds and not m._forward_hooks and not m._forward_pre_hooks and not m._backward_hooks and not m._backward_pre_hooks
+            and "forward" not in m.__dict__ and not torch.nn.modules.module._has_any_global_hook())
+
+
 def fork_norm(norm: nn.Module, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
     """``(norm(x), x)`` of any norm module; this module's own add the two gradients of ``x`` in the norm's backward pass."""
-    return norm(x, fork=True) if type(norm) in (RmsNorm, LayerNorm) else (norm(x), x)
+    return norm(x, fork=True) if plain(norm, RmsNorm, LayerNorm) else (norm(x), x)
 
 
 def linear_many(x: torch.Tensor, *projections: nn.Module):
     """The projections of the same rows, one by one; in training their input gradients are summed in the epilogues of their products."""
     from .ops.gemm import linear_many as many
 
-    if x.requires_grad and torch.is_grad_enabled() and all(type(m) is Linear and m.bias is None and not m._forward_hooks and not m._forward_pre_hooks
-                                                          and getattr(m.weight, "grad_sink", None) is None for m in projections):
+    if x.requires_grad and torch.is_grad_enabled() and all(plain(m, Linear) and m.bias is None and getattr(m.weight, "grad_sink", None) is None
+                                                          for m in projections):
         got = many(x, [m.weight for m in projections])
         if got is not None:
             return got
