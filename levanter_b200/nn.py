@@ -92,16 +92,14 @@ class FusedRows:
         first = params[0]
         storage = first.untyped_storage()
         base = at = storage.data_ptr()
-        rows = self.pad
-        for p in params:
-            if p.data_ptr() != at or p.dtype != first.dtype or not p.is_contiguous() or p.untyped_storage().data_ptr() != base:
+        for p in params:  # a tensor inside the live storage is a slice of it
+            if p.data_ptr() != at or p.dtype != first.dtype or not p.is_contiguous():
                 return None
-            at += p.numel() * p.element_size()
-            rows += p.shape[0]
+            at += p.nbytes
         width = first.stride(0)
-        if storage.nbytes() != rows * width * first.element_size():
+        if storage.nbytes() != at - base + self.pad * width * first.itemsize:
             return None
-        return first.detach().as_strided((rows, *first.shape[1:]), first.stride(), 0)
+        return first.detach().as_strided((storage.nbytes() // (width * first.itemsize), *first.shape[1:]), first.stride(), 0)
 
     def hold(self, params: Sequence[torch.Tensor]) -> None:
         """Called where the parameters are read one by one; while a graph is captured they stay where they are from then on."""
