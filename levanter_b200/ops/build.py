@@ -28,9 +28,9 @@ SERVING_SOURCES = ("attention_any", "depth_stream", "elementwise", "flash_attn_f
                    "linear_attention", "linear_attention_umma", "moe_experts", "page_table", "paged_attention", "paged_latent", "qkv_prep",
                    "residual_stream", "sampler")
 
-# Kernels whose results are 32-bit throughout (norms of an fp32 stream, router scores, rotary angles, recurrences, fp32 attention): no
-# fast-math exponentials, divisions or square roots.
-ACCURATE_SOURCES = ("attention_any", "delta_chunks", "depth_stream", "gated_scan", "linear_attention", "linear_attention_umma", "moe_experts", "qkv_prep",
+# Kernels whose results are 32-bit throughout (norms of an fp32 stream, router scores, rotary angles, recurrences, fp32 attention, the
+# loss): no fast-math exponentials, divisions or square roots.
+ACCURATE_SOURCES = ("attention_any", "cross_entropy", "delta_chunks", "depth_stream", "gated_scan", "linear_attention", "linear_attention_umma", "moe_experts", "qkv_prep",
                     "residual_stream")
 
 NVCC_FLAGS = [

@@ -5,9 +5,12 @@ running maximum and sum of exponentials of its column tile, so that a logit is n
 to the log-sum-exp and the loss.  Backward: the same product again, whose epilogue writes the logits' gradient in bf16 for a chunk of
 tokens, and two more products with it, dX (K = vocabulary, split over CTA pairs) and dW.
 
-A vocabulary that is no multiple of 8 (GPT-2's 50257) used to take library products in fp32.  There the gradient keeps fp32's precision as
-two bf16 parts, the rounded number and what the rounding lost, side by side in the row: 16 bits of mantissa, and both products run over
-both parts in one accumulation.  A training step of four GPT-2 layers over 8192 tokens (768 wide) went from 43.1 to
+A vocabulary that is no multiple of 8 (GPT-2's 50257) used to take library products in fp32.  There the gradient is held as two bf16 parts side by
+side in the row, the rounded number and what the rounding lost: 16 bits of mantissa; up to ``THREE_PARTS`` tokens as three, 24 bits.  Both products run
+over all parts in one accumulation, the lowest first.  What is left is the tensor cores' accumulator, which cuts off what it cannot hold: against 64
+bits dW in an fp32 buffer is off by 4e-7 for 300 tokens, 1.3e-6 for 999 and 4.9e-6 for 8192 (two parts with the rounded numbers first: 1.4e-6,
+3.1e-6, 1.2e-5; fp32 library products 3e-7 to 6e-7), where a bf16 gradient is off by 1.65e-3 either way.  The loss is off by 0.7 to 1.1e-7, an fp32
+unit in the last place, for the library's 4 to 5e-8.  A training step of four GPT-2 layers over 8192 tokens (768 wide) went from 43.1 to
 9.9 ms with it; the products of the head took 30.7 ms of that in fp32, the passes over logits 8 more.
 
 While a copy-job provider is set (fully sharded training: plain GEMMs carry the next layer's weight gather) and for vocabularies up to 128 the
@@ -70,12 +73,15 @@ def _head(name):
         _f[name] = lib.fn(name, {
             "lvb_head_ce_stats": [P] * 5 + [i] * 5 + [f, P, P],
             "lvb_ce_combine": [P, i] + [P] * 4 + [i, i, f, P, P],
-            "lvb_head_ce_grad": [P] * 7 + [ll, i, ll] + [i] * 5 + [f, P, P],
-            "lvb_head_ce_product": [P] * 3 + [i] * 3 + [ll, i, ll] + [i] * 5 + [P] * 3}[name])
+            "lvb_head_ce_grad": [P] * 7 + [ll] + [i] * 7 + [f, P, P],
+            "lvb_head_ce_product": [P] * 3 + [i] * 3 + [ll] + [i] * 7 + [P] * 3}[name])
     return _f[name]
 
 
 GRAD_BYTES = 3 << 29  # of the logits' gradient at once
+# Tokens up to which a gradient in parts has a third one.  dW sums over the tokens, and from about a thousand on the accumulator hides what the third part
+# adds (300 tokens: 1.02e-6 without it, 4.2e-7 with it; 999: 1.254e-6, 1.253e-6), while it makes both products half as long again (8192 tokens: 1 ms).
+THREE_PARTS = 1024
 
 
 def _grad_chunk(T: int, row_bytes: int) -> int:
@@ -106,10 +112,10 @@ def _plain_gradients(x, weight, targets, cap, z, dloss, wanted):
 
 
 class _HeadCE(torch.autograd.Function):
-    """See the module docstring.  ``low``: the gradient in two bf16 parts."""
+    """See the module docstring.  ``parts``: of the gradient, 1 to 3."""
 
     @staticmethod
-    def forward(ctx, x, weight, targets, soft_cap, z_weight, chunk_rows, low):
+    def forward(ctx, x, weight, targets, soft_cap, z_weight, chunk_rows, parts):
         T, E = x.shape
         V = weight.shape[0]
         tg = targets.to(torch.int32).contiguous()
@@ -123,7 +129,7 @@ class _HeadCE(torch.autograd.Function):
         lib.check_rc(_head("lvb_ce_combine")(part.data_ptr(), tiles, tg.data_ptr(), tl.data_ptr(), lse.data_ptr(), loss.data_ptr(), T, V, z, st, stream),
                      "lvb_ce_combine")
         ctx.save_for_backward(x, weight, tg, lse)
-        ctx.args = (cap, z, chunk_rows, low)
+        ctx.args = (cap, z, chunk_rows, parts)
         ctx.weight_ref = weight
         ctx.mark_non_differentiable(lse)
         return loss, lse
@@ -131,18 +137,17 @@ class _HeadCE(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss, _dlse):
         x, weight, tg, lse = ctx.saved_tensors
-        cap, z, chunk_rows, low = ctx.args
-        if low and torch.is_grad_enabled():  # create_graph: these vocabularies have had second derivatives, from library products
+        cap, z, chunk_rows, parts = ctx.args
+        if parts > 1 and torch.is_grad_enabled():  # create_graph: these vocabularies have had second derivatives, from library products
             return _plain_gradients(x, weight, tg, cap, z, dloss, ctx.needs_input_grad) + (None,) * 5
         T, E = x.shape
         V = weight.shape[0]
         g_loss = dloss.float().contiguous()
         g_logz = (g_loss * (2.0 * z) * lse).contiguous() if z != 0.0 else None
         cols = -(-V // 64) * 64
-        ldd = 2 * cols if low else cols
+        ldd = parts * cols
         chunk = chunk_rows or _grad_chunk(T, 2 * ldd)
         d = torch.empty(min(chunk, T), ldd, dtype=torch.bfloat16, device=x.device)
-        off = cols if low else 0
         dx = torch.empty(T, E, dtype=x.dtype, device=x.device) if ctx.needs_input_grad[0] else None
         dw = acc = None
         flags = 0
@@ -158,15 +163,15 @@ class _HeadCE(torch.autograd.Function):
             n = min(chunk, T - r0)
             xs, out = x[r0:r0 + n], None if dx is None else dx[r0:r0 + n]
             lib.check_rc(_head("lvb_head_ce_grad")(xs.data_ptr(), weight.data_ptr(), tg[r0:].data_ptr(), lse[r0:].data_ptr(), g_loss[r0:].data_ptr(),
-                                                   0 if g_logz is None else g_logz[r0:].data_ptr(), d.data_ptr(), ldd, cols, off, n, V, E, x.stride(0),
+                                                   0 if g_logz is None else g_logz[r0:].data_ptr(), d.data_ptr(), ldd, cols, parts, n, V, E, x.stride(0),
                                                    weight.stride(0), cap, st, stream), "lvb_head_ce_grad")
             if out is not None:
-                splits = _dx_splits(-(-n // 256) * -(-E // 256), (2 if low else 1) * cols // 64)
+                splits = _dx_splits(-(-n // 256) * -(-E // 256), parts * cols // 64)
                 ws = torch.empty(splits * n * E, dtype=torch.float32, device=x.device) if splits > 1 else None
-                lib.check_rc(_head("lvb_head_ce_product")(d.data_ptr(), weight.data_ptr(), out.data_ptr(), n, V, E, ldd, cols, off, weight.stride(0), E, 0, 0,
+                lib.check_rc(_head("lvb_head_ce_product")(d.data_ptr(), weight.data_ptr(), out.data_ptr(), n, V, E, ldd, cols, parts, weight.stride(0), E, 0, 0,
                                                           splits, lib.ptr(ws), st, stream), "lvb_head_ce_product")
             if acc is not None:
-                lib.check_rc(_head("lvb_head_ce_product")(d.data_ptr(), xs.data_ptr(), acc.data_ptr(), n, V, E, ldd, cols, off, x.stride(0), acc.stride(0), 1,
+                lib.check_rc(_head("lvb_head_ce_product")(d.data_ptr(), xs.data_ptr(), acc.data_ptr(), n, V, E, ldd, cols, parts, x.stride(0), acc.stride(0), 1,
                                                           flags, 1, 0, st, stream), "lvb_head_ce_product")
                 flags |= _gemm.F_ACCUMULATE
         if dw is not None:
@@ -249,7 +254,7 @@ def fused_linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: t
         # the tensor maps want rows of 16-byte aligned, unit-stride numbers
         x, weight = (t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
                      for t in (x, weight))
-        return _HeadCE.apply(x, weight, targets, soft_cap, z_weight, chunk_rows, V % 8 != 0)
+        return _HeadCE.apply(x, weight, targets, soft_cap, z_weight, chunk_rows, 1 if V % 8 == 0 else 3 if x.shape[0] <= THREE_PARTS else 2)
     return _FusedLinearCE.apply(x, weight, targets, soft_cap, z_weight, chunk_rows)
 
 

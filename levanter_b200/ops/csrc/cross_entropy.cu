@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restric
     for (int t = w; t < tiles; t += 8) {
       const float2 v = part[static_cast<size_t>(t) * rows + row];
       const float nm = fmaxf(m, v.x);
-      s = (m == -INFINITY ? s : s * __expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * __expf(v.x - nm));
+      s = (m == -INFINITY ? s : s * expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * expf(v.x - nm));
       m = nm;
     }
   }
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restric
   for (int i = 1; i < 8; ++i) {
     const float2 v = share[i][lane];
     const float nm = fmaxf(m, v.x);
-    s = (m == -INFINITY ? s : s * __expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * __expf(v.x - nm));
+    s = (m == -INFINITY ? s : s * expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * expf(v.x - nm));
     m = nm;
   }
   const float lse = m + logf(s);

@@ -76,10 +76,12 @@ struct Params {
   int cj_u0, cj_u1;
   const uint8_t* cj_src[kMaxPeers];
   uint8_t* cj_dst;
-  // ---- operands that wrap (kPlain): K block kb >= k_wrap > 0 reads B's block kb - k_wrap again and A's with its x coordinate
-  // moved by a_wrap_x.  A matrix held as two bf16 parts (high and low, side by side) is then multiplied in one accumulation.
+  // ---- operands that wrap (kPlain, k_wrap > 0): A is a matrix held as `parts` bf16 parts, a_part_ld columns apart.  The K blocks come in groups of
+  // parts x k_wrap: k_wrap blocks of the lowest part, the same of the next one, and so on, each against the same blocks of B, in one accumulation.
+  // The accumulator cuts off what it cannot hold of every addend, so the small ones go in while it is small.  A group per split of K.
+  // (Without parts: k_wrap 0, parts 1.)
   int k_wrap = 0;
-  int a_wrap_x = 0;
+  int parts = 1, a_part_ld = 0;
   // ---- cross-entropy epilogues (kCeStats, kCeGrad): C is never stored, it is the logits
   const int* ce_targets = nullptr;
   float2* ce_part = nullptr;        // kCeStats: (max, sum of exponentials) of every (column tile, row)
@@ -88,15 +90,15 @@ struct Params {
   const float* ce_g_loss = nullptr;
   const float* ce_g_logz = nullptr; // may be null
   float ce_cap = 0.f;               // tanh soft cap of the logits, 0: none
-  int ce_cols = 0;                  // kCeGrad: columns of C to write; those from N on get zeros
-  long long ce_low = 0;             // kCeGrad: offset of the low parts (0: C holds one bf16 number per logit)
+  int ce_cols = 0;                  // kCeGrad: columns of C to write per part, one part beside the other; those from N on get zeros
 };
 
 constexpr int kPlain = 0;
 constexpr int kScatter = 1;
 constexpr int kCopyJob = 2;
 constexpr int kCeStats = 3;
-constexpr int kCeGrad = 4;
+constexpr int kCeGrad = 4;  // + 0, 1, 2: the gradient in one, two or three bf16 parts
+__host__ __device__ constexpr bool ce_grad(int mode) { return mode >= kCeGrad; }
 constexpr int kCopyUnit = 16384;                  // bytes per bulk copy of a copy job
 constexpr int kCopyExtra = 256 + 2 * kCopyUnit;  // extra dynamic shared memory of the copy-job kernel
 constexpr int kCopyThreads = kNumThreads + 32;
@@ -203,7 +205,7 @@ struct CeRow {
   template <int MODE>
   __device__ __forceinline__ void begin(const Params& p, int row) {
     target = __ldg(p.ce_targets + row);
-    if constexpr (MODE == kCeGrad) {
+    if constexpr (ce_grad(MODE)) {
       lse = __ldg(p.ce_lse + row);
       gl = __ldg(p.ce_g_loss + row);
       gp = gl + (p.ce_g_logz != nullptr ? __ldg(p.ce_g_logz + row) : 0.f);
@@ -243,10 +245,11 @@ struct CeRow {
     }
   }
   // d(cap)/d(raw) * ((g_loss + g_logz) * probability - g_loss * [column == target])
+  template <int PARTS>
   __device__ __forceinline__ void grad(const Params& p, int row, int col0, const uint32_t (&r)[32]) {
     if (col0 >= p.ce_cols) return;
     const int at = target - col0;
-    uint32_t hi[16], lo[16];
+    uint32_t part[PARTS][16];
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
       float g[2];
@@ -262,19 +265,22 @@ struct CeRow {
         if (j + e == at) x -= gl;
         g[e] = col0 + j + e < p.N ? x * slope : 0.f;
       }
-      const __nv_bfloat162 h = __floats2bfloat162_rn(g[0], g[1]);
-      hi[j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-      const float2 back = __bfloat1622float2(h);
-      lo[j >> 1] = pack_bf16x2(g[0] - back.x, g[1] - back.y);
+#pragma unroll
+      for (int k = 0; k < PARTS; ++k) {  // the rounded number, what the rounding lost, and what that rounding lost: 8 bits each
+        const __nv_bfloat162 h = __floats2bfloat162_rn(g[0], g[1]);
+        part[k][j >> 1] = *reinterpret_cast<const uint32_t*>(&h);
+        const float2 back = __bfloat1622float2(h);
+        g[0] -= back.x;
+        g[1] -= back.y;
+      }
     }
     // rows are multiples of 64 columns long and 16-byte aligned; a piece lies inside or outside them as a whole
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.C) + static_cast<size_t>(row) * p.ldc + col0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(out)[q] = make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
-    if (p.ce_low > 0) {
+    for (int k = 0; k < PARTS; ++k)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) reinterpret_cast<uint4*>(out + p.ce_low)[q] = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
-    }
+      for (int q = 0; q < 4; ++q)
+        reinterpret_cast<uint4*>(out + k * p.ce_cols)[q] = make_uint4(part[k][4 * q], part[k][4 * q + 1], part[k][4 * q + 2], part[k][4 * q + 3]);
   }
 };
 
@@ -360,17 +366,23 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
         const int n0 = nb * BN + static_cast<int>(cta) * BNH;   // this CTA's columns of the B tile
         const int kb0 = (t % splits) * kbps;
         const int kb1 = min(k_blocks, kb0 + kbps);
+        // k_wrap > 0: blocks left of this run of a part, and what takes kb to the block of B and of the part's columns
+        int left = p.k_wrap, back = kb0 - kb0 / p.parts, ax = (p.parts - 1) * p.a_part_ld;
         for (int kb = kb0; kb < kb1; ++kb) {
           ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.status, 100, stage);
           if (!ok) break;
           uint8_t* sa = smem + stage * L::kStageBytes;
           uint8_t* sb = sa + L::kABytes;
           if (cta == 0) mbar_expect_tx(&full_bar[stage], 2 * L::kStageBytes);  // both CTAs' loads of this stage
-          int k0 = kb * BK, ax = 0;
+          int k0 = kb * BK;
           if constexpr (MODE == kPlain) {
-            if (p.k_wrap > 0 && kb >= p.k_wrap) {
-              k0 -= p.k_wrap * BK;
-              ax = p.a_wrap_x;
+            if (p.k_wrap > 0) {
+              if (left-- == 0) {  // the next part, over the same blocks of B
+                left = p.k_wrap - 1;
+                back += p.k_wrap;
+                ax -= p.a_part_ld;
+              }
+              k0 -= back * BK;
             }
           }
           if constexpr (!A_MN) {
@@ -456,7 +468,7 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
         c_dst_row0 = reinterpret_cast<float*>(p.c_peer[c_dest]) + static_cast<size_t>(row0w - c_dest * p.c_rows_per_rank) * p.ldc;
       }
       CeRow ce;
-      if constexpr (MODE == kCeStats || MODE == kCeGrad) {
+      if constexpr (MODE == kCeStats || ce_grad(MODE)) {
         if (row < p.M) ce.begin<MODE>(p, row);
       }
 #pragma unroll 1
@@ -465,10 +477,10 @@ __device__ __forceinline__ void gemm_pair_body(const CUtensorMap& tmA, const CUt
         tmem_ld_32x32(taddr + c, r);
         tmem_ld_wait();
         const int col0 = n0 + c;
-        if constexpr (MODE == kCeStats || MODE == kCeGrad) {
+        if constexpr (MODE == kCeStats || ce_grad(MODE)) {
           if (row < p.M) {
             if constexpr (MODE == kCeStats) ce.stats(p, row, col0, r);
-            else ce.grad(p, row, col0, r);
+            else ce.grad<MODE - kCeGrad + 1>(p, row, col0, r);
           }
           continue;
         }
@@ -943,15 +955,15 @@ extern "C" int lvb_head_ce_stats(const void* x, const void* w, const int* target
   return launch_ce<kCeStats>(x, w, p, ldx, ldw, reinterpret_cast<cudaStream_t>(stream));
 }
 
-// The gradient of the logits, bf16 [T, ldd] with columns [V, cols) zero (cols a multiple of 64, at least V); with low > 0 what the
-// rounding lost is stored as a second bf16 number `low` columns further on.
+// The gradient of the logits, bf16 [T, ldd] with columns [V, cols) zero (cols a multiple of 64, at least V), in `parts` (1 to 3) numbers per logit,
+// cols columns apart: the rounded number, what the rounding lost, and what that rounding lost.
 extern "C" int lvb_head_ce_grad(const void* x, const void* w, const int* targets, const float* lse, const float* g_loss, const float* g_logz,
-                                void* dlogits, long long ldd, int cols, long long low, int T, int V, int E, int ldx, int ldw, float soft_cap,
+                                void* dlogits, long long ldd, int cols, int parts, int T, int V, int E, int ldx, int ldw, float soft_cap,
                                 int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::gemm2;
-  if (T <= 0 || V <= 128 || E <= 0 || (ldx & 7) || (ldw & 7) || (ldd & 7) || (low & 7) || (cols & 63) || cols < V || ldd > 0x7fffffff ||
-      ldd < low + cols || (low > 0 && low < cols))
+  if (T <= 0 || V <= 128 || E <= 0 || (ldx & 7) || (ldw & 7) || (ldd & 7) || (cols & 63) || cols < V || parts < 1 || parts > 3 ||
+      ldd > 0x7fffffff || ldd < static_cast<long long>(parts) * cols)
     return kErrBadArg;
   Params p{};
   p.splits = 1;
@@ -966,18 +978,21 @@ extern "C" int lvb_head_ce_grad(const void* x, const void* w, const int* targets
   p.ce_g_logz = g_logz;
   p.ce_cap = soft_cap;
   p.ce_cols = cols;
-  p.ce_low = low;
-  return launch_ce<kCeGrad>(x, w, p, ldx, ldw, reinterpret_cast<cudaStream_t>(stream));
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return parts == 1   ? launch_ce<kCeGrad>(x, w, p, ldx, ldw, s)
+         : parts == 2 ? launch_ce<kCeGrad + 1>(x, w, p, ldx, ldw, s)
+                      : launch_ce<kCeGrad + 2>(x, w, p, ldx, ldw, s);
 }
 
-// Products with the gradient d [T, ldd] that lvb_head_ce_grad made (low > 0: high and low parts, both multiplied in one accumulation):
+// Products with the gradient d [T, ldd] that lvb_head_ce_grad made (all of its parts multiplied in one accumulation):
 //   a_mn = 0: C[T, E] = d * w[V, E]      (K = V, split over CTA pairs where T x E has few tiles; workspace as lvb_gemm_bf16_pair_splitk)
 //   a_mn = 1: C[V, E] = d^T * x[T, E]    (K = T)
-extern "C" int lvb_head_ce_product(const void* d, const void* b, void* C, int T, int V, int E, long long ldd, int cols, long long low, int ldb,
+extern "C" int lvb_head_ce_product(const void* d, const void* b, void* C, int T, int V, int E, long long ldd, int cols, int parts, int ldb,
                                    int ldc, int a_mn, int flags, int splits, void* workspace, int* status, void* stream) {
   using namespace lvb;
   using namespace lvb::gemm2;
-  if (T <= 0 || V <= 0 || E <= 0 || (ldb & 7) || (ldd & 7) || ldd > 0x7fffffff || splits < 1 || splits > 8) return kErrBadArg;
+  if (T <= 0 || V <= 0 || E <= 0 || (ldb & 7) || (ldd & 7) || parts < 1 || parts > 3 || ldd > 0x7fffffff ||
+      ldd < static_cast<long long>(parts) * cols || splits < 1 || splits > 8) return kErrBadArg;
   Params p{};
   p.C = C;
   p.ldc = ldc;
@@ -988,12 +1003,13 @@ extern "C" int lvb_head_ce_product(const void* d, const void* b, void* C, int T,
   p.N = E;
   const int depth = a_mn ? T : cols;  // of one part
   const int blocks = (depth + BK - 1) / BK;
-  p.K = low > 0 ? 2 * blocks * BK : depth;
-  p.k_wrap = low > 0 ? blocks : 0;
-  p.a_wrap_x = static_cast<int>(low);
   p.splits = a_mn ? 1 : splits;
+  p.k_wrap = parts > 1 ? (blocks + p.splits - 1) / p.splits : 0;  // (blocks past the end: B's rows there are zeros)
+  p.K = parts > 1 ? parts * p.splits * p.k_wrap * BK : depth;
+  p.parts = parts;
+  p.a_part_ld = cols;
   p.ws = reinterpret_cast<float*>(workspace);
-  const int wide = low > 0 ? static_cast<int>(low) + cols : cols;  // columns of d
+  const int wide = parts * cols;  // columns of d
   CUtensorMap tmA, tmB;
   int rc = a_mn ? make_tmap_2d_bf16(&tmA, d, T, wide, static_cast<int>(ldd), BK, 64) : make_tmap_2d_bf16(&tmA, d, T, wide, static_cast<int>(ldd), BMC, BK);
   if (rc != kErrOk) return rc;

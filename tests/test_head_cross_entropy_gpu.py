@@ -22,10 +22,11 @@ def _rel(a, b):
     return float((a.double() - b).norm() / b.norm())
 
 
-# vocabularies around 128 (the old path), a tile of 256 and K blocks of 64; multiples of 8 (one part) and others (two); rows around a tile
+# vocabularies around 128 (the old path), a tile of 256 and K blocks of 64; multiples of 8 (one part) and others (two, or three up to 1024 tokens); rows around a tile
 @pytest.mark.parametrize("T,V,E,cap,z,chunk", [
     (1, 129, 8, None, None, None), (255, 136, 72, None, None, None), (256, 256, 64, 5.0, None, None), (257, 257, 64, None, 1e-3, None),
-    (700, 1000, 768, None, None, 256), (300, 4093, 264, 7.0, 1e-3, 256), (513, 50257, 768, None, None, None), (1000, 8191, 128, None, None, 512)])
+    (700, 1000, 768, None, None, 256), (300, 4093, 264, 7.0, 1e-3, 256), (513, 50257, 768, None, None, None), (1000, 8191, 128, None, None, 512),
+    (1300, 4093, 264, 7.0, 1e-3, 256)])
 def test_head_cross_entropy(T, V, E, cap, z, chunk):
     from levanter_b200.ops import cross_entropy as CE
 
@@ -46,12 +47,15 @@ def test_head_cross_entropy(T, V, E, cap, z, chunk):
     assert _rel(w.grad, dw) < limit
 
 
-def test_two_parts_hold_fp32_sums():
-    """With an fp32 accumulator for dW nothing is rounded to bf16: two parts leave 2^-17 of a logit's gradient, one part 2^-9."""
+@pytest.mark.parametrize("T,limit", [(300, 1e-6), (1024, 4e-6), (1025, 4e-6), (4100, 1.6e-5)])
+def test_gradients_in_parts_over_an_fp32_accumulator(T, limit):
+    """With an fp32 buffer for dW nothing is rounded to bf16.  Three parts (up to 1024 tokens) hold all of an fp32 number, two 16 bits, whose rounding
+    averages out over the tokens; the lowest part is added first.  What shows is the accumulator, which cuts every addend off below its own last bit: at
+    most 2^-24 of the sum for each of the T / 16 steps, 3.8e-9 per token, and a few 2^-24 of the probabilities."""
     from levanter_b200.ops import cross_entropy as CE
 
     torch.manual_seed(1)
-    T, V, E = 300, 1003, 128
+    V, E = 1003, 128
     x = torch.randn(T, E, device="cuda").bfloat16()
     w = (torch.randn(V, E, device="cuda") * 0.2).bfloat16().requires_grad_()
     w.main_grad = torch.zeros(V, E, device="cuda")
@@ -60,7 +64,7 @@ def test_two_parts_hold_fp32_sums():
     loss, _ = CE.fused_linear_cross_entropy(x, w, tgt)
     (loss * gl).sum().backward()
     assert w.grad is None
-    assert _rel(w.main_grad, _plain(x, w, tgt, None, None, gl)[2]) < 2e-5
+    assert _rel(w.main_grad, _plain(x, w, tgt, None, None, gl)[2]) < limit
 
 
 def test_odd_vocabulary_in_the_loss_takes_what_it_took():
