@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restric
     for (int t = w; t < tiles; t += 8) {
       const float2 v = part[static_cast<size_t>(t) * rows + row];
       const float nm = fmaxf(m, v.x);
-      s = (m == -INFINITY ? s : s * expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * expf(v.x - nm));
+      s = (m == nm ? s : s * expf(m - nm)) + (v.x == nm ? v.y : v.y * expf(v.x - nm));  // (equal infinities as well)
       m = nm;
     }
   }
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restric
   for (int i = 1; i < 8; ++i) {
     const float2 v = share[i][lane];
     const float nm = fmaxf(m, v.x);
-    s = (m == -INFINITY ? s : s * expf(m - nm)) + (v.x == -INFINITY ? v.y : v.y * expf(v.x - nm));
+    s = (m == nm ? s : s * expf(m - nm)) + (v.x == nm ? v.y : v.y * expf(v.x - nm));  // (equal infinities as well)
     m = nm;
   }
   const float lse = m + logf(s);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(256) ce_combine_kernel(const float2* __restric
   if (t >= vocab) record_status(status, kBoundsCheck, 500, t);
   // targets outside the vocabulary (padding, ignored ids) contribute no target logit; their loss weight is expected to be zero
   lse_out[row] = lse;
-  loss_out[row] = lse - (t >= 0 && t < vocab ? target_logit[row] : 0.f) + z_weight * lse * lse;
+  loss_out[row] = lse - (t >= 0 && t < vocab ? target_logit[row] : 0.f) + (z_weight != 0.f ? z_weight * lse * lse : 0.f);
 }
 
 }  // namespace ce

@@ -230,8 +230,9 @@ struct CeRow {
     }
     if (m != -INFINITY) {
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      const float base = m == INFINITY ? 0.f : m;  // a logit of +inf makes the sum inf, and not inf - inf
 #pragma unroll
-      for (int j = 0; j < 32; ++j) sum[j & 3] += __expf(v[j] - m);
+      for (int j = 0; j < 32; ++j) sum[j & 3] += __expf(v[j] - base);
       s += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     } else {  // nothing but -inf so far, or NaN, which has to show
 #pragma unroll

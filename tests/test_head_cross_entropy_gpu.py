@@ -67,6 +67,29 @@ def test_gradients_in_parts_over_an_fp32_accumulator(T, limit):
     assert _rel(w.main_grad, _plain(x, w, tgt, None, None, gl)[2]) < limit
 
 
+@pytest.mark.parametrize("V", [256, 257, 1003])
+def test_infinite_logits(V):
+    """+inf and -inf as in torch.logsumexp: a +inf anywhere makes the log-sum-exp +inf, columns of -inf are as if they were not there, NaN shows."""
+    from levanter_b200.ops import cross_entropy as CE
+
+    torch.manual_seed(3)
+    inf = float("inf")
+    base = (torch.randn(V, 64) * 0.2).bfloat16()
+    x = torch.ones(4, 64, device="cuda").bfloat16()
+    x[1] = -1.0
+    for rows, value in (([5], inf), ([V - 1], inf), ([5, V - 1], inf), ([7, 40, V - 2], -inf), (range(V - 1), -inf), ([9], float("nan"))):
+        w = base.clone()
+        w[list(rows)] = 0.0
+        w[list(rows), 0] = value  # one infinite product per logit: x[0] sees `value`, x[1] its opposite
+        w = w.cuda()
+        tgt = torch.tensor([0, 1, 2, V - 3], device="cuda")
+        loss, lse = CE.fused_linear_cross_entropy(x, w, tgt)
+        logits = x.double() @ w.double().t()
+        want = torch.logsumexp(logits, -1)
+        assert torch.allclose(lse.double(), want, rtol=1e-5, equal_nan=True), (lse, want)
+        assert torch.allclose(loss.double(), want - logits.gather(1, tgt[:, None])[:, 0], rtol=1e-5, atol=1e-5, equal_nan=True)
+
+
 def test_odd_vocabulary_in_the_loss_takes_what_it_took():
     """Targets out of range, strided operands and second derivatives, which the library products of these vocabularies allowed."""
     from levanter_b200.models.loss import maybe_fused_next_token_loss
