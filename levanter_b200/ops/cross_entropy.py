@@ -111,6 +111,12 @@ def _plain_gradients(x, weight, targets, cap, z, dloss, wanted):
     return tuple(next(got) if w else None for w in wanted[:2])
 
 
+def _tma_rows(t: torch.Tensor) -> torch.Tensor:
+    """``t [rows, cols]`` as the tensor maps can describe it: rows of unit stride that do not overlap, at 16-byte aligned strides."""
+    ok = t.stride(1) == 1 and t.stride(0) >= t.shape[1] and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.clone(memory_format=torch.contiguous_format)
+
+
 class _HeadCE(torch.autograd.Function):
     """See the module docstring.  ``parts``: of the gradient, 1 to 3."""
 
@@ -118,6 +124,9 @@ class _HeadCE(torch.autograd.Function):
     def forward(ctx, x, weight, targets, soft_cap, z_weight, chunk_rows, parts):
         T, E = x.shape
         V = weight.shape[0]
+        given = (x, weight)
+        ctx.weight_ref = weight
+        x, weight = _tma_rows(x), _tma_rows(weight)
         tg = targets.to(torch.int32).contiguous()
         tiles = -(-V // 256)
         part = torch.empty(tiles, T, 2, dtype=torch.float32, device=x.device)
@@ -128,9 +137,8 @@ class _HeadCE(torch.autograd.Function):
                                                 weight.stride(0), cap, st, stream), "lvb_head_ce_stats")
         lib.check_rc(_head("lvb_ce_combine")(part.data_ptr(), tiles, tg.data_ptr(), tl.data_ptr(), lse.data_ptr(), loss.data_ptr(), T, V, z, st, stream),
                      "lvb_ce_combine")
-        ctx.save_for_backward(x, weight, tg, lse)
+        ctx.save_for_backward(*given, tg, lse)
         ctx.args = (cap, z, chunk_rows, parts)
-        ctx.weight_ref = weight
         ctx.mark_non_differentiable(lse)
         return loss, lse
 
@@ -142,6 +150,7 @@ class _HeadCE(torch.autograd.Function):
             return _plain_gradients(x, weight, tg, cap, z, dloss, ctx.needs_input_grad) + (None,) * 5
         T, E = x.shape
         V = weight.shape[0]
+        x, weight = _tma_rows(x), _tma_rows(weight)
         g_loss = dloss.float().contiguous()
         g_logz = (g_loss * (2.0 * z) * lse).contiguous() if z != 0.0 else None
         cols = -(-V // 64) * 64
@@ -154,7 +163,9 @@ class _HeadCE(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             main_grad = getattr(ctx.weight_ref, "main_grad", None)
             if main_grad is not None:
-                acc, flags = main_grad, _gemm.F_OUT_F32 | _gemm.F_ACCUMULATE
+                if main_grad.shape != (V, E) or main_grad.stride(1) != 1 or main_grad.dtype not in (torch.float32, torch.bfloat16):
+                    raise ValueError("main_grad has to be a row-major fp32 or bf16 buffer of the weight's shape")
+                acc, flags = main_grad, _gemm.F_ACCUMULATE | (_gemm.F_OUT_F32 if main_grad.dtype == torch.float32 else 0)
             else:  # fp32 sums over several chunks, rounded once; the products of a single chunk are rounded as they are made
                 dw = acc = torch.empty(V, E, dtype=weight.dtype if chunk >= T else torch.float32, device=x.device)
                 flags = 0 if chunk >= T else _gemm.F_OUT_F32
@@ -251,9 +262,6 @@ def fused_linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, targets: t
     """Per-token ``(loss, logsumexp)`` of ``softmax(x @ weight.T)`` against ``targets``; ``x[T,E]`` bf16, ``weight[V,E]`` bf16."""
     V = weight.shape[0]
     if V > 128 and x.shape[0] > 0 and _gemm._copy_job_provider is None:
-        # the tensor maps want rows of 16-byte aligned, unit-stride numbers
-        x, weight = (t if t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
-                     for t in (x, weight))
         return _HeadCE.apply(x, weight, targets, soft_cap, z_weight, chunk_rows, 1 if V % 8 == 0 else 3 if x.shape[0] <= THREE_PARTS else 2)
     return _FusedLinearCE.apply(x, weight, targets, soft_cap, z_weight, chunk_rows)
 

@@ -90,6 +90,32 @@ def test_infinite_logits(V):
         assert torch.allclose(loss.double(), want - logits.gather(1, tgt[:, None])[:, 0], rtol=1e-5, atol=1e-5, equal_nan=True)
 
 
+@pytest.mark.parametrize("V", [264, 331])
+def test_rows_and_accumulators_of_other_layouts(V):
+    """Rows that overlap or repeat and a weight of other strides are copied for the tensor maps, and the parameter itself keeps its accumulator; a bf16
+    accumulator gets bf16 sums (2^-8), one of another shape is refused."""
+    from levanter_b200.ops import cross_entropy as CE
+
+    torch.manual_seed(4)
+    T, E = 40, 64
+    rows = torch.randn(E + 8 * T, device="cuda").bfloat16()
+    tgt = torch.randint(0, V, (T,), device="cuda")
+    gl = torch.rand(T, device="cuda") + 0.1
+    for x in (rows.as_strided((T, E), (8, 1)), rows[:E].expand(T, E), torch.randn(T * E + 1, device="cuda").bfloat16()[1:].view(T, E)):
+        for dtype in (torch.float32, torch.bfloat16):
+            w = (torch.randn(E, V, device="cuda") * 0.2).bfloat16().t().requires_grad_()  # columns in a row
+            w.main_grad = torch.full((V, E), 0.5, device="cuda", dtype=dtype)
+            loss, _ = CE.fused_linear_cross_entropy(x, w, tgt)
+            (loss * gl).sum().backward()
+            ref, _, dw = _plain(x, w, tgt, None, None, gl)
+            assert float((loss.detach().double() - ref).abs().max()) < 2e-5 * max(1.0, float(ref.abs().max()))
+            assert w.grad is None
+            assert _rel(w.main_grad, dw + 0.5) < (2e-3 if dtype == torch.float32 and V % 8 == 0 else 1e-5 if dtype == torch.float32 else 2 ** -8)
+    w.main_grad = torch.zeros(V, E + 8, device="cuda")
+    with pytest.raises(ValueError):
+        CE.fused_linear_cross_entropy(x, w, tgt)[0].sum().backward()
+
+
 def test_odd_vocabulary_in_the_loss_takes_what_it_took():
     """Targets out of range, strided operands and second derivatives, which the library products of these vocabularies allowed."""
     from levanter_b200.models.loss import maybe_fused_next_token_loss
