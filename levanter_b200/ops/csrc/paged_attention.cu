@@ -498,8 +498,8 @@ __global__ void __launch_bounds__(kThreads) paged_attention_staged_kernel(Params
 // shared memory so that ldmatrix reads are conflict-free) with one bulk copy per key (kExact; cp.async otherwise), double-buffered, and needs no CTA-wide barrier
 // inside the loop.  Scores S = Q K^T come from ldmatrix'd K rows, the online softmax runs on the accumulator fragments,
 // P is re-packed in registers as the A operand of O += P V (V rows through ldmatrix.trans), and the four warps' (max, sum,
-// O) are merged through shared memory at the end.  kSplitP: the probabilities enter O += P V as two bf16 parts, for a size whose scalar kernel
-// kept them in fp32 (heads of 64: 24 us there for one sequence of 300 tokens, 5.5 here).
+// O) are merged through shared memory at the end.  kSplitP: the probabilities enter O += P V as three bf16 parts, all 24 bits of them, for a size
+// whose scalar kernel kept them in fp32 (heads of 64: 24 us there for one sequence of 300 tokens, 5.5 here).  The lowest part goes first.
 constexpr int kMmaStageKeys = 16;
 constexpr int kMmaBufs = 2;  // stages of a warp.  Three leave room for two CTAs on an SM instead of three: 20 to 30 % slower, the warps are needed
 // A staged row: K, V (each rounded up to 16 columns) and 16 bytes of padding, which makes the stride an odd multiple of 16 bytes, so
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
     const float a_lo = (m_lo == -INFINITY) ? 0.f : exp2f(m_lo - mn_lo);
     const float a_hi = (m_hi == -INFINITY) ? 0.f : exp2f(m_hi - mn_hi);
     float sum_lo = 0.f, sum_hi = 0.f;
-    uint32_t pa[4], pl[4];
+    uint32_t pa[4], pl[2][4];
     {
       float pv[2][4];
 #pragma unroll
@@ -717,11 +717,18 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       pa[1] = pack_bf16x2(pv[0][2], pv[0][3]);  // (row_hi, keys 0-7 tile)
       pa[2] = pack_bf16x2(pv[1][0], pv[1][1]);  // (row_lo, keys 8-15 tile)
       pa[3] = pack_bf16x2(pv[1][2], pv[1][3]);  // (row_hi, keys 8-15 tile)
-      if constexpr (kSplitP) {  // what the rounding lost
+      if constexpr (kSplitP) {  // what the rounding lost, and what that rounding lost
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pa[i]));
-          pl[i] = pack_bf16x2(pv[i >> 1][2 * (i & 1)] - hi.x, pv[i >> 1][2 * (i & 1) + 1] - hi.y);
+          float r0 = pv[i >> 1][2 * (i & 1)], r1 = pv[i >> 1][2 * (i & 1) + 1];
+          uint32_t w = pa[i];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            const float2 up = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+            r0 -= up.x;
+            r1 -= up.y;
+            w = pl[k][i] = pack_bf16x2(r0, r1);
+          }
         }
       }
     }
@@ -746,12 +753,15 @@ __global__ void __launch_bounds__(kThreads) paged_attention_mma_kernel(Params p)
       float* ob = o[2 * np + 1];
       oa[0] *= a_lo; oa[1] *= a_lo; oa[2] *= a_hi; oa[3] *= a_hi;
       ob[0] *= a_lo; ob[1] *= a_lo; ob[2] *= a_hi; ob[3] *= a_hi;
+      if constexpr (kSplitP) {
+#pragma unroll
+        for (int k = 1; k >= 0; --k) {
+          mma_16816(o[2 * np], pl[k], b0, b1);
+          mma_16816(o[2 * np + 1], pl[k], b2, b3);
+        }
+      }
       mma_16816(o[2 * np], pa, b0, b1);
       mma_16816(o[2 * np + 1], pa, b2, b3);
-      if constexpr (kSplitP) {
-        mma_16816(o[2 * np], pl, b0, b1);
-        mma_16816(o[2 * np + 1], pl, b2, b3);
-      }
     }
     __syncwarp();  // every lane is done with this buffer before the copy of stage st + kMmaBufs overwrites it
   }
