@@ -681,7 +681,8 @@ extern "C" int lvb_norm_bwd(const void* dy, const void* x, const void* w, int w_
   const int vpt = ((dim >> 3) + TX - 1) / TX;
   auto go = [&](auto kern, int ring) {
     const int smem = base + ring * (dres_in != nullptr ? 3 : 2) * vpt_room(vpt) * TX * TY * 16;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return kErrCuda;
+    // the same limit from every call (four vectors, three kinds, two rows are 192 KB): another thread may be about to launch a wider row
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return kErrCuda;
     kern<<<nparts, block, smem, s>>>(DY, X, w, w_is_f32, rstd, mean, DR, DX, dw_part, db_part, rows, dim, w_offset);
     return kErrOk;
   };

@@ -986,12 +986,10 @@ template <int DKC, int DVC, bool kExact, bool kSplitP = false>
 int launch_mma(const Params& p, cudaStream_t s) {
   const int smem = kExact ? mma_smem(DKC, DVC, p.part) : mma_smem((p.dk + 15) & ~15, (p.dv + 15) & ~15, p.part);
   auto kern = paged_attention_mma_kernel<DKC, DVC, kExact, kSplitP>;
-  static int most = 0;  // 4096 keys per partition are those of contexts of a million tokens
-  if (smem > most) {
-    const int room = smem > mma_smem(DKC, DVC, 4096) ? smem : mma_smem(DKC, DVC, 4096);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, room) != cudaSuccess) return kErrCuda;
-    most = room;
-  }
+  constexpr int kRoom = 226 * 1024;  // what a CTA may have, set once: the partitions of other threads' calls may be longer
+  static const bool room = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom) == cudaSuccess;
+  if (!room) return kErrCuda;
+  if (smem > kRoom) return kErrTooLarge;
   return launch_chained(kern, dim3(p.T, p.KV, p.parts), kThreads, smem, s, p) == cudaSuccess ? kErrOk : kErrCuda;
 }
 

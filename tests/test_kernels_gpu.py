@@ -233,3 +233,33 @@ def test_projections_of_the_same_rows_and_a_norm_that_forks(rows):
         assert (a - b).norm() <= 2 ** -7 * b.norm()
     h, r = fork_norm(ln, x.detach())
     assert torch.equal(h, ln(x.detach())) and torch.equal(r, x.detach())
+
+
+def test_norm_backward_from_two_threads():
+    """Rows of 64 and of 4096 with a residual's gradient go through the same kernel with 8 and 96 KB of shared memory: neither thread may take the
+    other's room away between its request and its launch."""
+    import threading
+
+    from levanter_b200.ops import norm as N
+
+    failed = []
+
+    def work(dim, seed):
+        try:
+            g = torch.Generator(device="cuda").manual_seed(seed)
+            x = torch.randn(64, dim, device="cuda", generator=g).bfloat16().requires_grad_()
+            w = torch.ones(dim, device="cuda").bfloat16().requires_grad_()
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(200):
+                    y, h = N.norm_and_input(x, w, None, 1e-6, layer_norm=False)
+                    torch.autograd.grad((y.float() + h.float()).sum(), (x, w))
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(dim, i)) for i, dim in enumerate((4096, 64, 4096, 64))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
