@@ -427,6 +427,7 @@ class _LinearManyFn(torch.autograd.Function):
         ctx.save_for_backward(x.reshape(-1, x.shape[-1]), *weights)
         ctx.x_shape = x.shape
         ctx.refs = weights
+        ctx.set_materialize_grads(False)  # a product that nothing uses has no gradient, and its weight none
         return tuple(_linear_rows(x, w, None, None) for w in weights)
 
     @staticmethod
@@ -434,6 +435,9 @@ class _LinearManyFn(torch.autograd.Function):
         x2, *weights = ctx.saved_tensors
         dx, dws = None, []
         for i, (dy, w, ref) in enumerate(zip(dys, weights, ctx.refs)):
+            if dy is None:
+                dws.append(None)
+                continue
             dy2 = dy.reshape(-1, dy.shape[-1])
             if dy2.dtype != torch.bfloat16:
                 dy2 = dy2.to(torch.bfloat16)

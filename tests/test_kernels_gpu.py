@@ -263,3 +263,17 @@ def test_norm_backward_from_two_threads():
         t.join()
     torch.cuda.synchronize()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("used", [(0,), (1,), (0, 2)])
+def test_joint_projections_that_nothing_uses_have_no_gradient(used):
+    from levanter_b200.nn import Linear, linear_many
+
+    torch.manual_seed(0)
+    mods = [Linear(64, n).cuda().bfloat16() for n in (64, 128, 32)]
+    x = torch.randn(48, 64, device="cuda").bfloat16().requires_grad_()
+    ys = linear_many(x, *mods)
+    sum(ys[i].float().sum() for i in used).backward()
+    assert [m.weight.grad is not None for m in mods] == [i in used for i in range(3)]
+    want = sum(torch.ones(48, mods[i].out_features, device="cuda", dtype=torch.double) @ mods[i].weight.double() for i in used)
+    assert (x.grad.double() - want).norm() / want.norm() < 2 ** -7
