@@ -91,10 +91,15 @@ def _grad_chunk(T: int, row_bytes: int) -> int:
     return -(-(-(-T // n)) // 256) * 256
 
 
-def _dx_splits(tiles: int, k_blocks: int) -> int:
-    """CTA pairs per 256 x 256 tile of dX.  K is the whole vocabulary there and a narrow model has few tiles (4096 x 768: 48 on 74
-    pairs), so the cost is the number of waves times K per split; at least 16 K blocks each, ties to fewer splits."""
-    return min(range(1, max(1, min(8, k_blocks // 16)) + 1), key=lambda s: (-(-tiles * s // 74) / s, s))
+def _dx_splits(tiles: int, k_blocks: int, pairs: int, out_bytes: int) -> int:
+    """CTA pairs per 256 x 256 tile of dX.  K is the whole vocabulary there and a narrow model has few tiles (4096 x 768: 48 on 74 pairs), so a
+    product takes its waves times K per split, 0.44 us for a block of 64 (of K) and a tile at the tensor cores' rate; every split also writes its sums in
+    fp32 (``out_bytes`` each) and they are read again, at 5 TB/s and 3 us more.  At least 16 K blocks each, and sums of at most ``GRAD_BYTES`` in all."""
+    def cost(s):
+        return -(-tiles * s // pairs) * -(-k_blocks // s) * 0.44 + (3.0 + 2 * s * out_bytes / 5e6 if s > 1 else 0.0)
+
+    most = max(1, min(8, k_blocks // 16, GRAD_BYTES // max(1, out_bytes)))
+    return min(range(1, most + 1), key=lambda s: (cost(s), s))
 
 
 def _plain_gradients(x, weight, targets, cap, z, dloss, wanted):
@@ -170,6 +175,7 @@ class _HeadCE(torch.autograd.Function):
                 dw = acc = torch.empty(V, E, dtype=weight.dtype if chunk >= T else torch.float32, device=x.device)
                 flags = 0 if chunk >= T else _gemm.F_OUT_F32
         st, stream = lib.status_buffer().data_ptr(), lib.stream_ptr()
+        pairs = torch.cuda.get_device_properties(x.device).multi_processor_count // 2
         for r0 in range(0, T, chunk):
             n = min(chunk, T - r0)
             xs, out = x[r0:r0 + n], None if dx is None else dx[r0:r0 + n]
@@ -177,7 +183,7 @@ class _HeadCE(torch.autograd.Function):
                                                    0 if g_logz is None else g_logz[r0:].data_ptr(), d.data_ptr(), ldd, cols, parts, n, V, E, x.stride(0),
                                                    weight.stride(0), cap, st, stream), "lvb_head_ce_grad")
             if out is not None:
-                splits = _dx_splits(-(-n // 256) * -(-E // 256), parts * cols // 64)
+                splits = _dx_splits(-(-n // 256) * -(-E // 256), parts * cols // 64, pairs, 4 * n * E)
                 ws = torch.empty(splits * n * E, dtype=torch.float32, device=x.device) if splits > 1 else None
                 lib.check_rc(_head("lvb_head_ce_product")(d.data_ptr(), weight.data_ptr(), out.data_ptr(), n, V, E, ldd, cols, parts, weight.stride(0), E, 0, 0,
                                                           splits, lib.ptr(ws), st, stream), "lvb_head_ce_product")
