@@ -94,7 +94,7 @@ def attention(tb: Table, T=8192, n_seq=4, H=32, KV=8, S=64, ctx=4096):
         flops = 2.0 * H * (dk + dv) * keys
         d = 64 if max(dk, dv) <= 64 else 128
         ql, kl, vl = (_randn(1, T, h, d) for h in (H, KV, KV))
-        m = AttentionMask.causal().with_segment_ids(seg[None], sorted=True)
+        m = AttentionMask.causal().with_segment_ids(seg[None])
         tb.pair(f"prefill attention {dk}/{dv}, chunk {chunk or 'none'}, gated",
                 lambda: FA.flash_attention_packed(q, k, v, pos, scaling_factor=dk ** -0.5, chunk=chunk, gate=gate), f"Llama prefill attention {d}",
                 lambda: dot_product_attention(ql, kl, vl, m), flops=flops, nbytes=2.0 * (y.numel() + T * H * dv),

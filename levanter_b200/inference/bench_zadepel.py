@@ -20,7 +20,7 @@ def attention(tb: Table, T=8192, n_seq=4, H=32, KV=8, S=64, ctx=4096):
     L = T // n_seq
     pos = (torch.arange(T, device="cuda") % L).int()
     seg = (torch.arange(T, device="cuda") // L).int()
-    m = AttentionMask.causal().with_segment_ids(seg[None], sorted=True)
+    m = AttentionMask.causal().with_segment_ids(seg[None])
     for what, hk, dk, dv, window in (("attention", KV, 128, 128, None), ("attention", KV, 128, 64, None), ("latent", H, 192, 128, None),
                                      ("latent", H, 192, 128, 1024), ("latent", H, 128, 128, 1024), ("latent", H, 96, 64, 256)):
         y = _randn(T, H * dk + hk * (dk + dv))

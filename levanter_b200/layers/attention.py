@@ -81,7 +81,7 @@ class AttentionMask:
     sliding_window: Optional[int] = None
     segments_sorted: bool = False
     """the segment ids are non-decreasing along the sequence with negative ids (padding) only at the end, as in packed
-    batches: kernels may then skip every key block that lies before a query block's first sequence"""
+    batches.  A statement that callers may make; the kernels skip blocks of other segments by the ids themselves, in any order, and do not need it"""
     chunk_size: Optional[int] = None
     """positions are cut into chunks of this size, counted from the start of the sequence (of the segment, with segment ids), and a
     query sees the keys of its own chunk only; queries and keys must be the same positions"""
@@ -619,7 +619,7 @@ class Attention(nn.Module):
         if seg is not None and x.is_cuda:
             # pure prefill: nothing to read from the cache, so this is causal attention over the packed tokens with one segment
             # per sequence (the flash kernel), instead of the decode kernel walking pages
-            m = AttentionMask.causal(sliding_window=c.sliding_window).with_segment_ids(seg.unsqueeze(0), sorted=True)
+            m = AttentionMask.causal(sliding_window=c.sliding_window).with_segment_ids(seg.unsqueeze(0))
             out = dot_product_attention(q.unsqueeze(0), k.unsqueeze(0), v.unsqueeze(0), m, attn_backend=c.attn_backend,
                                         logits_soft_cap=c.logits_soft_cap, scaling_factor=c.scaling_factor, inference=True).squeeze(0)
         elif prepared:

@@ -37,11 +37,6 @@ def _fwd2_hd():
     return _f["f2h"]
 
 
-def _fwd2():
-    """The form that most layers take: causal, head size 128, no sink."""
-    return _fwd2_hd()
-
-
 def _bwd_hd():
     if "bh" not in _f:
         c = lib
@@ -138,9 +133,8 @@ def _attend(q, k, v, q_seg, k_seg, scale, soft_cap, window, causal, sink):
     lse2 = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
     tail = (float(scale), float(soft_cap or 0.0), int(window or 0), lib.status_buffer().data_ptr(), lib.stream_ptr())
     if not _FORCE_ONE_TILE:
-        fwd = _fwd2() if D == 128 and causal and sink is None else _fwd2_hd()
-        rc = fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), _strides(q, k, v), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg),
-                 lib.ptr(ranges), lib.ptr(sink), B, S, Sk, Hq, Hkv, D, int(bool(causal)), *tail)
+        rc = _fwd2_hd()(q.data_ptr(), k.data_ptr(), v.data_ptr(), _strides(q, k, v), o.data_ptr(), lse2.data_ptr(), lib.ptr(q_seg), lib.ptr(k_seg),
+                        lib.ptr(ranges), lib.ptr(sink), B, S, Sk, Hq, Hkv, D, int(bool(causal)), *tail)
     else:
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
         if D != 128 or not causal or sink is not None:
@@ -227,7 +221,7 @@ def _mask_parts(mask, B: int, S: int, Sk: int, device):
         return None, None, 0, False
     if mask.chunk_size is not None:
         if mask.segment_ids is None:
-            mask = mask.with_segment_ids(torch.zeros(B, S, dtype=torch.int32, device=device), sorted=True)
+            mask = mask.with_segment_ids(torch.zeros(B, S, dtype=torch.int32, device=device))
         mask = mask.chunks_as_segments()  # a chunk is a segment of its own
     q_seg = k_seg = None
     if mask.segment_ids is not None:

@@ -460,8 +460,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 }  // namespace fab2
 }  // namespace lvb
 
-// Backward of lvb_flash_attn_fwd, pipelined form (arguments of lvb_flash_attn_bwd, whose ranges come from lvb_segment_ranges).  dq32: fp32 [B,S,Hq,128], must be
-// zero on entry.  delta: fp32 [B,Hq,S] scratch.  strides: (sequence, row) in elements of q, k, v, and of dk and dv.  Any S.
+// Backward of causal attention with heads of 128, pipelined form (arguments as lvb_flash_attn_bwd_hd).  dq32: fp32 [B,S,Hq,128], must be zero on
+// entry.  delta: fp32 [B,Hq,S] scratch.  strides: (sequence, row) in elements of q, k, v, and of dk and dv.  Any S.
 extern "C" int lvb_flash_attn_bwd2(const void* q, const void* k, const void* v, const long long* strides, const void* o, const void* d_o, const float* lse2,
                                    float* delta, float* dq32, void* dk, void* dv, const int* q_seg, const int* k_seg, const void* ranges, int B, int S,
                                    int Hq, int Hkv, float scale, float soft_cap, int window, int* status, void* stream) {

@@ -12,7 +12,7 @@ def test_keep_attention_checkpointing_same_gradients_fewer_launches(monkeypatch)
     from levanter_b200.ops import _flash_impl, lib
 
     calls = {"fwd": 0}
-    real_fwd2, real_fwd = _flash_impl._fwd2, _flash_impl._fwd
+    real_fwd2, real_fwd = _flash_impl._fwd2_hd, _flash_impl._fwd
 
     def counting(getter):
         def get():
@@ -26,7 +26,7 @@ def test_keep_attention_checkpointing_same_gradients_fewer_launches(monkeypatch)
 
         return get
 
-    monkeypatch.setattr(_flash_impl, "_fwd2", counting(real_fwd2))
+    monkeypatch.setattr(_flash_impl, "_fwd2_hd", counting(real_fwd2))
     monkeypatch.setattr(_flash_impl, "_fwd", counting(real_fwd))
     out = {}
     for gc in ("full", True):
