@@ -316,11 +316,13 @@ _few_dw = None
 
 
 def few_outputs_dw(dy: torch.Tensor, x: torch.Tensor, out_dtype: torch.dtype) -> Optional[torch.Tensor]:
-    """``dy^T x`` of rows ``dy [rows, outputs]`` and ``x [rows, cols]`` with few outputs and many rows, or None where the GEMM is the better form: from
-    1024 rows on and up to 32 outputs its one or two tiles leave the SMs idle."""
+    """``dy^T x`` of rows ``dy [rows, outputs]`` and ``x [rows, cols]`` with few outputs and many rows, or None where the GEMM is the better form.  Its
+    few tiles walk all rows, 5 us and 5.1 more per 1024 rows whatever the columns (16384 rows: 88); the lanes' time goes with rows x outputs x columns.
+    us, lanes / GEMM: 8 x 1024 over 1024 rows 7.1 / 9.9, over 16384 15 / 88; 16 x 1024 8.4 / 9.9, 26 / 88; 32 x 1024 11.7 / 9.8, over 2048 13.9 / 15.1, over
+    16384 46 / 88; 8 x 4096 11.7 / 10.0, 13.9 / 15.2, 72 / 100; 16 x 4096 over 2048 21.9 / 15.2, over 16384 134 / 97."""
     global _few_dw
     (rows, outputs), cols = dy.shape, x.shape[1]
-    if not (outputs <= 32 and rows >= 1024 and x.is_cuda and lib.available() and outputs % 8 == 0 and cols % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32)
+    if not (0 < outputs <= 32 and rows >= 1024 and outputs * cols <= min(16 * rows, 32768) and x.is_cuda and lib.available() and outputs % 8 == 0 and cols % 8 == 0 and out_dtype in (torch.bfloat16, torch.float32)
             and dy.dtype == x.dtype == torch.bfloat16 and all(t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0 for t in (dy, x))):
         return None
     if _few_dw is None:
@@ -452,8 +454,9 @@ MANY_ROWS = 2048
 
 def linear_many(x: torch.Tensor, weights):
     """``[x W^T for W in weights]`` on the tcgen05 GEMM, or None where :func:`linear` would not take it for all of them, and for more rows than the
-    launches bound: an epilogue that reads back what it adds to costs a large product more than a pass of its own (Gated DeltaNet, two layers:
-    1500 rows 5.40 -> 4.95 ms, 16384 rows 22.96 -> 23.71)."""
+    host's part bounds.  What one function saves is autograd's work per projection; on the device an epilogue that reads back what it adds to costs as much
+    as a pass of its own or more (input gradients of six projections 1024 wide: 1500 rows 88 us, 70 with added passes; 16384 rows 284, 236; of two
+    2048 wide 81, 76 and 555, 555).  Gated DeltaNet, two layers: 1500 rows 5.40 -> 4.95 ms, 16384 rows 22.96 -> 23.71."""
     if not (x.numel() <= MANY_ROWS * x.shape[-1] and x.is_cuda and lib.available() and x.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 and _tma_shapes_ok(w) for w in weights)):
         return None
     return _LinearManyFn.apply(x, *weights)

@@ -277,3 +277,12 @@ def test_joint_projections_that_nothing_uses_have_no_gradient(used):
     assert [m.weight.grad is not None for m in mods] == [i in used for i in range(3)]
     want = sum(torch.ones(48, mods[i].out_features, device="cuda", dtype=torch.double) @ mods[i].weight.double() for i in used)
     assert (x.grad.double() - want).norm() / want.norm() < 2 ** -7
+
+
+@pytest.mark.parametrize("rows,outputs,cols,lanes", [(1024, 16, 1024, True), (1024, 8, 4096, False), (2047, 32, 1024, False), (2048, 32, 1024, True), (2048, 8, 4096, True),
+                                                     (16384, 16, 4096, False)])
+def test_few_outputs_dw_where_it_is_the_faster_form(rows, outputs, cols, lanes):
+    from levanter_b200.ops.gemm import few_outputs_dw
+
+    dy, x = (torch.zeros(rows, n, device="cuda").bfloat16() for n in (outputs, cols))
+    assert (few_outputs_dw(dy, x, torch.bfloat16) is not None) == lanes
