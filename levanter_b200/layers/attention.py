@@ -765,7 +765,9 @@ class Attention(nn.Module):
 
 # Rows up to which a serving step's projections that read the same rows are one product over their weights laid out side by side.  Such products
 # stream their weights, and each of them costs about 7 us beside that: 8 rows of a Llama 3 8B layer, three products 33 us and three sums of their
-# parts 7, one product 15 and 2 (a round of four such layers 827 -> 726 us).  Larger steps are bound by the tensor cores.
+# parts 7, one product 15 and 2 (a round of four such layers 827 -> 726 us).  Weights out of the cache, us separate / joint, q, k, v and gate with up:
+# 128 rows 36 / 18 and 53 / 50, 256 rows 48 / 26 and 63 / 58, 512 rows 55 / 29 and 104 / 101.  The joint form is the faster one beyond the line as well;
+# 256 is the largest step that was measured as a whole round.
 DECODE_ROWS = 256
 
 
